@@ -383,7 +383,7 @@ int32_t run_stage(const BmndStageParams& sp, const float* noisy, const float* pi
                                   sp.match_threshold, w.sel, w.count, w.accepted, stream, thr_dev,
                                   sp.match_noise_ssd, sp.ssd_gamma, allow_alloc, null_moments,
                                   sp.null_max_count, sp.ssd_poisson_bias != 0, w.aux, w.aux_floats, w.ssd,
-                                  w.ssd_bytes);
+                                  w.ssd_bytes, w.agg_base, w.agg_base ? w.agg.bytes : 0);
     if (rc) return rc;
     if (det) {
         rc = launch_entry_index(sp, w.sel, w.count, n_refs, w.agg_base, w.agg, stream);

@@ -217,7 +217,8 @@ int32_t launch_blockmatch_volume(const BmndMatchParams& mp, const float* volume,
                                  float gamma = 0.0f, bool allow_alloc = true,
                                  const double* null_moments = nullptr, int null_max = 0,
                                  bool poisson_bias = false, float* aux_ws = nullptr, int64_t aux_ws_floats = 0,
-                                 char* ssd_ws = nullptr, uint64_t ssd_ws_bytes = 0);
+                                 char* ssd_ws = nullptr, uint64_t ssd_ws_bytes = 0, char* box_ws = nullptr,
+                                 uint64_t box_ws_bytes = 0);
 // squared norm of a patch centred on mu, from its sum of squares s2 and sum s1:
 // s2 - 2 mu s1 + P mu^2 (float32, clamped at zero); the screening and the
 // selection evaluate it with the same operations
