@@ -36,6 +36,7 @@ namespace bmnd {
 namespace {
 
 constexpr int kThreads = 256;      // threads per group (CTA)
+constexpr int kMiscWild = 13;      // misc word: the group holds a value of 1e30 or more, an infinity or NaN
 
 // Shared-memory plan.  A fixed part holds the group matrix, the transform
 // tables, positions and small per-group arrays.  The union region first holds
@@ -47,8 +48,9 @@ constexpr int kThreads = 256;      // threads per group (CTA)
 // shrinkage, so they get a region of their own after the group buffers.
 struct Layout {
     // byte offsets into dynamic shared memory
-    int64_t g, gt, fw, fi, fit, dir, win, mdiag, pos, shf, shl, sg, ex, part, lag, uni, s, x, r, v, grid, lval,
+    int64_t g, gt2, fw, fi, fit, dir, win, mdiag, voff, kron, pos, org0, shf, shl, sg, ex, part, lag, uni, s, x, r, v, grid, lval,
         lstart, lent, scan, plane, wts, misc, risk, total;
+    int32_t part_over;  // the exact phase's partial sums overwrite its lists
 };
 
 struct FilterArgs {
@@ -79,6 +81,10 @@ struct FilterArgs {
     AggStore store;      // deterministic aggregation: rows of the entry store, or store.store == null
 };
 
+__host__ __device__ inline bool kron_in_smem(const BmndStageParams& sp, int P, int kmax) {
+    return kron_jr(P) == 2 && kmax > 0 && sp.noise_model == BMND_NOISE_POISSON;
+}
+
 __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax, int64_t ucells, bool sigma) {
     Layout L{};
     int64_t off = 0;
@@ -92,7 +98,7 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     const bool wiener = sp.filter == BMND_FILTER_WIENER;
     const int kpad = (kmax + 3) / 4 * 4;
     L.g = take(4 * nmax * nmax);
-    L.gt = take(4 * nmax * (kpad > 0 ? kpad : 4));
+    L.gt2 = take(8 * nmax * (kpad > 0 ? kpad : 4));  // exact planes' G entries in pairs (g, g) for packed products
     L.fw = take(4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE);
     L.fi = take(4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE);
     // group-mass conservation: transposed inverse spatial matrices, and the
@@ -101,8 +107,13 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.fit = take(mass ? 4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE : 16);
     L.dir = take(mass ? 4 * (BMND_MAX_STACK + BMND_MAX_DIMS * BMND_MAX_EDGE) : 16);
     L.win = take(4 * P);
-    L.mdiag = take(8 * P);
+    L.mdiag = take(sp.windowed_synthesis ? 8 * P : 16);
+    L.voff = take(4 * P);
+    // S^T of patches of 33-64 voxels (16 KB): the exact phase reads it with
+    // 32-bit addresses and no L1 tags
+    L.kron = take(kron_in_smem(sp, P, kmax) ? 4 * static_cast<int64_t>(P) * kron_stride(P) : 16);
     L.pos = take(4 * nmax * BMND_MAX_DIMS);
+    L.org0 = take(4 * nmax);
     L.shf = take(4 * nmax * BMND_MAX_DIMS);
     L.shl = take(4 * nmax);
     // hard thresholding with a sigma map keeps each coefficient's sigma until the scatter
@@ -131,24 +142,39 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     const bool keep = sp.exact_risk_weights != 0;
     const int kl = (gauss && !keep) ? 0 : kmax;
     const int64_t umax = kl > 0 ? (np < ucells ? np : ucells) : 0;
+    // member masks per union coordinate of every axis: a union box of at most
+    // ucells cells has at most ucells / prod(other patch edges) along an axis
+    int64_t axis_masks = 0;
+    for (int d = 0; d < sp.ndim; ++d) {
+        const int64_t most = ucells * sp.block[d] / P;
+        axis_masks += most < sp.shape[d] ? most : sp.shape[d];
+    }
     L.grid = keep ? L.uni + group_bytes : L.uni;
-    L.lval = L.grid + round16(kl > 0 ? 4 * ucells : 0);
+    L.lval = L.grid + round16(kl > 0 ? 4 * axis_masks : 0);
     L.lstart = L.lval + round16(4 * umax);
     L.lent = L.lstart + round16(4 * (umax + 1));
-    const int64_t list_end = L.lent + round16(kl > 0 ? 4 * np : 0);
+    const int64_t list_end = L.lent + round16(kl > 0 ? 4 * (np + 2) : 0);
     off = keep ? list_end : L.uni + (group_bytes > list_end - L.uni ? group_bytes : list_end - L.uni);
     // exact variance: per-warp partial sums of one tile of 4 planes x 32 JR
-    // coefficients (64 for the half-warp form), added in warp order afterwards;
-    // they take the occupancy grid's place (free once the lists are built) when
-    // it is large enough
+    // coefficients (64 for the half-warp form), added in warp order afterwards.
+    // With a single tile (k <= 4 and P <= its width: the default profiles) the
+    // lists are done with by then and give their place.
     const int tile_w = kron_jr(P) == 2 ? 64 : 32 * kron_jr(P);
     const int64_t part_bytes = 4 * (kThreads / 32) * 4 * static_cast<int64_t>(tile_w);
+    L.part_over = !keep && kmax <= 4 && P <= tile_w;
     if (gauss || kmax <= 0) L.part = L.grid;
-    else if (4 * ucells >= part_bytes) L.part = L.grid;
-    else L.part = take(part_bytes);
+    else if (L.part_over) {
+        L.part = L.grid;
+        if (off < L.part + part_bytes) off = L.part + part_bytes;
+    } else L.part = take(part_bytes);
     L.total = off;
     return L;
 }
+
+template <bool V>
+struct BoolTag {
+    static constexpr bool value = V;
+};
 
 template <typename T>
 __device__ __forceinline__ T* sm(unsigned char* base, int64_t off) {
@@ -261,6 +287,96 @@ __device__ void group_axis_inplace(float* buf, int P, const float* G) {
     }
 }
 
+// Haar group axis of a power-of-two size N as the matrix product above without
+// its zero entries: row 0 and row 1 are dense, the 2^(l-1) rows of level l reach
+// N / 2^(l-1) columns each, so a column takes log2(N) + 1 multiply-adds per
+// output instead of N.  Leaving out fma(0, x, acc) = acc keeps every result's
+// bits for finite x (the caller checks).  C is the chunk of 8 outputs a warp
+// takes; entry values come from the matrix, so their rounding is its own.
+template <int N, int KIND, int C>
+__device__ __forceinline__ void haar_chunk(const float* buf, int P, int p, const float* G,
+                                           float (&acc)[N >= 16 ? 8 : N]) {
+    constexpr int IC = N >= 16 ? 8 : N;
+    constexpr int i0 = C * IC;
+    {
+        if constexpr (KIND == 1) {
+            // out[g] = sum over rows k whose support holds g, ascending
+            constexpr int LV = N >= 32 ? 5 : (N >= 16 ? 4 : (N >= 8 ? 3 : (N >= 4 ? 2 : 1)));
+            const float x0 = buf[p], m0 = G[0];
+#pragma unroll
+            for (int ii = 0; ii < IC; ++ii) acc[ii] = fmaf(m0, x0, 0.0f);
+#pragma unroll
+            for (int l = 0; l < LV; ++l) {
+                const int w = N >> l;  // support width of the 2^l rows of this level
+#pragma unroll
+                for (int j = 0; j < (1 << l); ++j) {
+                    const int k = (1 << l) + j, b = j * w;
+                    if (b < i0 + IC && b + w > i0) {
+                        const float x = buf[k * P + p], m = G[k * N + b];
+#pragma unroll
+                        for (int ii = 0; ii < IC; ++ii) {
+                            const int g = i0 + ii;
+                            if (g >= b && g < b + w) acc[ii] = fmaf(g < b + w / 2 ? m : -m, x, acc[ii]);
+                        }
+                    }
+                }
+            }
+        } else {
+            float x[N];  // the columns this chunk's rows reach
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                bool used = false;
+#pragma unroll
+                for (int ii = 0; ii < IC; ++ii) {
+                    const int i = i0 + ii;
+                    const int top = i == 0 ? 1 : (i < 2 ? 1 : (i < 4 ? 2 : (i < 8 ? 4 : (i < 16 ? 8 : 16))));
+                    const int w = N / top, b = i == 0 ? 0 : (i - top) * w;
+                    used = used || (k >= b && k < b + w);
+                }
+                if (used) x[k] = buf[k * P + p];
+            }
+#pragma unroll
+            for (int ii = 0; ii < IC; ++ii) {
+                const int i = i0 + ii;
+                const int top = i < 2 ? 1 : (i < 4 ? 2 : (i < 8 ? 4 : (i < 16 ? 8 : 16)));
+                const int w = N / top, b = i == 0 ? 0 : (i - top) * w;
+                float m = G[i * N + b];
+                if (KIND == 2) m = mul_rn(m, m);
+                float t = 0.0f;
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    if (k >= b && k < b + w) t = fmaf(KIND == 2 || i == 0 || k < b + w / 2 ? m : -m, x[k], t);
+                acc[ii] = t;
+            }
+        }
+    }
+}
+
+template <int N, int KIND>
+__device__ void haar_product(float* buf, int P, const float* G) {
+    constexpr int IC = N >= 16 ? 8 : N;
+    constexpr int CH = N / IC;
+    const int cols = static_cast<int>(blockDim.x) / CH;
+    const int chunk = static_cast<int>(threadIdx.x) / cols;  // the same for a whole warp
+    for (int c0 = 0; c0 < P; c0 += cols) {
+        const int p = c0 + static_cast<int>(threadIdx.x) % cols;
+        const bool act = static_cast<int>(threadIdx.x) < cols * CH && p < P;
+        float acc[IC];
+        if (act) {
+            if (CH == 1 || chunk == 0) haar_chunk<N, KIND, 0>(buf, P, p, G, acc);
+            else if (CH == 2 || chunk == 1) haar_chunk<N, KIND, (CH > 1 ? 1 : 0)>(buf, P, p, G, acc);
+            else if (chunk == 2) haar_chunk<N, KIND, (CH > 2 ? 2 : 0)>(buf, P, p, G, acc);
+            else haar_chunk<N, KIND, (CH > 3 ? 3 : 0)>(buf, P, p, G, acc);
+        }
+        __syncthreads();
+        if (act) {
+#pragma unroll
+            for (int ii = 0; ii < IC; ++ii) buf[(chunk * IC + ii) * P + p] = acc[ii];
+        }
+        __syncthreads();
+    }
+}
+
 // Haar group axis by its sum pyramid (one thread per column, O(N) operations):
 // row (l, j) of the orthonormal Haar matrix, block width w = N / 2^(l-1), is
 // (first-half sum - second-half sum) / sqrt(w); its elementwise square gives the
@@ -312,7 +428,7 @@ __device__ __forceinline__ void haar_column(float* buf, int p, int P) {
 
 template <int N, int KIND>
 __device__ void haar_axis_fast(float* buf, int P) {
-    for (int p = threadIdx.x; p < P; p += blockDim.x) haar_column<N, KIND>(buf, p, P);
+    for (int p = static_cast<int>(threadIdx.x); p < P; p += blockDim.x) haar_column<N, KIND>(buf, p, P);
     __syncthreads();
 }
 
@@ -320,7 +436,7 @@ __device__ void haar_axis_fast(float* buf, int P) {
 // 2), x and r (kind 0; r may be null)
 template <int N>
 __device__ void haar_axis_fast3(float* s, float* x, float* r, int P) {
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
+    for (int p = static_cast<int>(threadIdx.x); p < P; p += blockDim.x) {
         haar_column<N, 2>(s, p, P);
         haar_column<N, 0>(x, p, P);
         if (r) haar_column<N, 0>(r, p, P);
@@ -354,7 +470,7 @@ __device__ bool haar_axis_any(float* buf, int n, int P) {
 // runtime group size (not a power of two): one thread per column
 template <int KIND>
 __device__ void group_axis_generic(float* buf, int n, int P, const float* G) {
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
+    for (int p = static_cast<int>(threadIdx.x); p < P; p += blockDim.x) {
         float x[BMND_MAX_STACK];
         for (int k = 0; k < n; ++k) x[k] = buf[k * P + p];
         for (int i = 0; i < n; ++i) {
@@ -366,8 +482,19 @@ __device__ void group_axis_generic(float* buf, int n, int P, const float* G) {
     __syncthreads();
 }
 
+// `sparse`: G is the Haar matrix and every value is finite
 template <int KIND>
-__device__ void group_axis_any(float* buf, int n, int P, const float* G) {
+__device__ void group_axis_any(float* buf, int n, int P, const float* G, bool sparse) {
+    if (sparse) {
+        switch (n) {
+            case 2: haar_product<2, KIND>(buf, P, G); return;
+            case 4: haar_product<4, KIND>(buf, P, G); return;
+            case 8: haar_product<8, KIND>(buf, P, G); return;
+            case 16: haar_product<16, KIND>(buf, P, G); return;
+            case 32: haar_product<32, KIND>(buf, P, G); return;
+            default: break;
+        }
+    }
     switch (n) {
         case 1: group_axis_inplace<1, KIND>(buf, P, G); break;
         case 2: group_axis_inplace<2, KIND>(buf, P, G); break;
@@ -405,7 +532,7 @@ __device__ void space_axis_reg(float* buf, int total, const float* Msrc, bool sq
         m[q] = square ? mul_rn(v, v) : v;
     }
     const int lines = total / B;
-    for (int line = threadIdx.x; line < lines; line += blockDim.x) {
+    for (int line = static_cast<int>(threadIdx.x); line < lines; line += blockDim.x) {
         const int o = line / INNER;
         const int t = line - o * INNER;
         space_line<B, INNER>(buf, o * B * INNER + t, m);
@@ -425,7 +552,7 @@ __device__ void space_axis_reg3(float* s, float* x, float* r, int total, const f
         m2[q] = mul_rn(v, v);
     }
     const int lines = total / B;
-    for (int line = threadIdx.x; line < lines; line += blockDim.x) {
+    for (int line = static_cast<int>(threadIdx.x); line < lines; line += blockDim.x) {
         const int o = line / INNER;
         const int t = line - o * INNER;
         const int base = o * B * INNER + t;
@@ -442,7 +569,7 @@ __device__ void space_axis_generic(const GM& geo, int d, float* buf, int n, cons
     const int m = geo.b(d);
     const int inner = geo.inner(d);
     const int lines = n * geo.P() / m;
-    for (int line = threadIdx.x; line < lines; line += blockDim.x) {
+    for (int line = static_cast<int>(threadIdx.x); line < lines; line += blockDim.x) {
         const int o = line / inner;
         const int t = line - o * inner;
         const int base = o * m * inner + t;
@@ -491,9 +618,11 @@ __device__ void transform_group(const GM& geo, const FilterArgs& a, unsigned cha
     if (!fast_haar && a.sp.group_transform != BMND_GROUP_NONE) {
         // kind 3 (transposed inverse): the group transforms are orthonormal, so
         // the transposed inverse of the group axis is the forward transform
-        if (kind == 0 || kind == 3) group_axis_any<0>(buf, n, geo.P(), G);
-        else if (kind == 1) group_axis_any<1>(buf, n, geo.P(), G);
-        else group_axis_any<2>(buf, n, geo.P(), G);
+        const bool sparse = a.sp.group_transform == BMND_GROUP_HAAR && kind != 3 && !a.den_ro &&
+                            sm<int>(smem, a.L.misc)[kMiscWild] == 0;
+        if (kind == 0 || kind == 3) group_axis_any<0>(buf, n, geo.P(), G, sparse);
+        else if (kind == 1) group_axis_any<1>(buf, n, geo.P(), G, sparse);
+        else group_axis_any<2>(buf, n, geo.P(), G, sparse);
     }
     const bool square = kind == 2;
     if constexpr (ND > 0) {
@@ -626,6 +755,11 @@ struct KronVec<4> {
 template <int NQ>
 struct PlaneVec {
     float v[NQ];
+    // from the paired table (g, g)
+    __device__ __forceinline__ void load_pairs(const unsigned char* p) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) v[q] = reinterpret_cast<const float2*>(p)[q].x;
+    }
     __device__ __forceinline__ void load(const float* p) {
         if constexpr (NQ == 4) {
             const float4 t = *reinterpret_cast<const float4*>(p);
@@ -653,8 +787,9 @@ struct PlaneVec {
 template <int RL, int NQ>
 __device__ __forceinline__ void exact_stream(const float* __restrict__ lval, const int* __restrict__ lstart,
                                              const uint32_t* __restrict__ lent, int u_lo, int u_hi,
-                                             const float* __restrict__ gt0, int kpad,
+                                             const unsigned char* smem, uint32_t plane_byte, uint32_t stride,
                                              const float* __restrict__ stl, float (&var)[RL][NQ]) {
+    const unsigned char* gb = smem + plane_byte;
 #pragma unroll
     for (int r = 0; r < RL; ++r)
 #pragma unroll
@@ -673,15 +808,15 @@ __device__ __forceinline__ void exact_stream(const float* __restrict__ lval, con
     uint32_t ent1 = lent[e];
     PlaneVec<NQ> g0;
     KronVec<RL> s0;
-    g0.load(gt0 + (ent1 & 0xffu) * kpad);
-    s0.load(stl + (ent1 >> 8));
+    g0.load_pairs(gb + (ent1 & 0xffffu));
+    s0.load(stl + (ent1 >> 16) * stride);
     ent1 = lent[e + 1 < e_end ? e + 1 : e];
     for (; e < e_end; ++e) {
         // loads of entry e + 1 (harmless repeats of the last entry at the end)
         PlaneVec<NQ> g1;
         KronVec<RL> s1;
-        g1.load(gt0 + (ent1 & 0xffu) * kpad);
-        s1.load(stl + (ent1 >> 8));
+        g1.load_pairs(gb + (ent1 & 0xffffu));
+        s1.load(stl + (ent1 >> 16) * stride);
         const uint32_t ent2 = lent[e + 2 < e_end ? e + 2 : e_end - 1];
         if (e == next_start) {
 #pragma unroll
@@ -710,64 +845,272 @@ __device__ __forceinline__ void exact_stream(const float* __restrict__ lval, con
         for (int q = 0; q < NQ; ++q) var[r][q] = fmaf(mul_rn(v, c[r][q]), c[r][q], var[r][q]);
 }
 
-// one tile of NQ planes x 32 JR coefficients over the warp's voxels
-template <int JR, int NQ>
-__device__ void exact_tile(const float* __restrict__ lval, const int* __restrict__ lstart,
-                           const uint32_t* __restrict__ lent, int u_lo, int u_hi,
-                           const float* __restrict__ GT, int kpad, int i0,
-                           const float* __restrict__ st, int j0, float (&var)[JR][NQ]) {
-    const int lane = threadIdx.x & 31;
-    exact_stream<JR, NQ>(lval, lstart, lent, u_lo, u_hi, GT + i0, kpad, st + j0 + JR * lane, var);
+// The same stream for four coefficients per lane in packed pairs (two
+// multiply-adds per instruction, each rounded as its scalar form).  It is bound
+// by instruction issue, so addresses are kept in 32-bit shared-memory form (the
+// generic 64-bit pointers cost more integer instructions than the products):
+// an entry word holds the shared-memory byte offset of the member's paired G
+// entries and the patch element; two words past the last one are readable.  A
+// voxel's first entry starts its sums with a product.
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void lds_pairs(float2& a, float2& b, uint32_t addr) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(b.x), "=f"(b.y)
+                 : "r"(addr));
 }
 
-// Patches of 33-64 voxels (JR = 2): the two half-warps take the two halves of
-// the warp's voxels and each lane holds 4 coefficients, j = 4 (lane % 16) + r,
-// so an entry costs the same three loads for 4 NQ fused multiply-adds instead
-// of 2 NQ.  The halves' sums are added at the end (lanes l and l + 16 hold the
-// same coefficients).
+// G pairs of an entry's member (planes from `plane`, a shared-memory address)
 template <int NQ>
-__device__ void exact_tile_hw(const float* __restrict__ lval, const int* __restrict__ lstart,
-                              const uint32_t* __restrict__ lent, int u_lo, int u_hi,
-                              const float* __restrict__ GT, int kpad, int i0,
-                              const float* __restrict__ st, float (&var)[4][NQ]) {
-    const int lane = threadIdx.x & 31;
-    const int half = lane >> 4;
-    // split at the first voxel whose entries start in the second half of the entries
-    const int e_mid = (lstart[u_lo] + lstart[u_hi]) >> 1;
-    int lo = u_lo, hi = u_hi;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (lstart[mid] < e_mid) lo = mid + 1;
-        else hi = mid;
+__device__ __forceinline__ void load_pairs(float2 (&g)[NQ], uint32_t plane, uint32_t ent) {
+    const uint32_t at = plane + (ent & 0xffffu);
+    if constexpr (NQ == 4) {
+        lds_pairs(g[0], g[1], at);
+        lds_pairs(g[2], g[3], at + 16);
+    } else if constexpr (NQ == 2) {
+        lds_pairs(g[0], g[1], at);
+    } else {
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(g[0].x), "=f"(g[0].y) : "r"(at));
     }
-    const int u_mid = lo;
-    exact_stream<4, NQ>(lval, lstart, lent, half ? u_mid : u_lo, half ? u_hi : u_mid, GT + i0, kpad,
-                        st + 4 * (lane & 15), var);
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) var[r][q] = add_rn(var[r][q], __shfl_xor_sync(0xffffffffu, var[r][q], 16));
 }
 
-// all tiles of (NQ planes) x (TW coefficients); EX[i * P + j] receives the
+// the lane's four coefficients of the entry's row of S^T
+__device__ __forceinline__ void load_row(float2 (&sv)[2], const char* row0, uint32_t ent, uint32_t stride_b) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(row0 + static_cast<uint64_t>(ent >> 16) * stride_b));
+    sv[0] = make_float2(t.x, t.y);
+    sv[1] = make_float2(t.z, t.w);
+}
+
+template <int NQ>
+__device__ __forceinline__ void exact_pairs(const unsigned char* smem, const float* lval, const int* lstart,
+                                            const uint32_t* lent, int u_lo, int u_hi, uint32_t plane_byte,
+                                            const float* __restrict__ st, uint32_t stride_b,
+                                            float2 (&var)[2][NQ]) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) var[0][q] = var[1][q] = make_float2(0.0f, 0.0f);
+    if (u_lo >= u_hi) return;
+    const uint32_t plane = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + plane_byte;
+    const uint32_t ents = static_cast<uint32_t>(__cvta_generic_to_shared(lent));
+    uint32_t ls = static_cast<uint32_t>(__cvta_generic_to_shared(lstart + u_lo));
+    const uint32_t lv = static_cast<uint32_t>(__cvta_generic_to_shared(lval)) -
+                        static_cast<uint32_t>(__cvta_generic_to_shared(lstart));  // lval[u] at lv + &lstart[u]
+    const char* row0 = reinterpret_cast<const char*>(st);
+    uint32_t ep = ents + 4u * static_cast<uint32_t>(lstart[u_lo]);
+    const uint32_t end = ents + 4u * static_cast<uint32_t>(lstart[u_hi]);
+    uint32_t next = ep;
+    float v = 0.0f;  // before the first voxel: a fold of zeros
+    float2 c[2][NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) c[0][q] = c[1][q] = make_float2(0.0f, 0.0f);
+    float2 g0[NQ], s0[2], g1[NQ], s1[2];
+    uint32_t ent = lds32(ep);
+    load_pairs<NQ>(g0, plane, ent);
+    load_row(s0, row0, ent, stride_b);
+    ent = lds32(ep + 4);
+    auto fold = [&]() {
+        const float2 vv = make_float2(v, v);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            var[0][q] = __ffma2_rn(__fmul2_rn(vv, c[0][q]), c[0][q], var[0][q]);
+            var[1][q] = __ffma2_rn(__fmul2_rn(vv, c[1][q]), c[1][q], var[1][q]);
+        }
+    };
+    auto step = [&](const float2 (&g)[NQ], const float2 (&sv)[2]) {
+        if (ep == next) {
+            fold();
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                c[0][q] = __fmul2_rn(g[q], sv[0]);
+                c[1][q] = __fmul2_rn(g[q], sv[1]);
+            }
+            v = __uint_as_float(lds32(ls + lv));
+            ls += 4;
+            next = ents + 4u * lds32(ls);
+        } else {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                c[0][q] = __ffma2_rn(g[q], sv[0], c[0][q]);
+                c[1][q] = __ffma2_rn(g[q], sv[1], c[1][q]);
+            }
+        }
+        ep += 4;
+    };
+    while (true) {
+        // the loads of the next entry are issued before this one's products
+        load_pairs<NQ>(g1, plane, ent);
+        load_row(s1, row0, ent, stride_b);
+        ent = lds32(ep + 8);
+        step(g0, s0);
+        if (ep == end) break;
+        load_pairs<NQ>(g0, plane, ent);
+        load_row(s0, row0, ent, stride_b);
+        ent = lds32(ep + 8);
+        step(g1, s1);
+        if (ep == end) break;
+    }
+    fold();
+}
+
+// The stream for Haar groups, whose planes 0 .. 3 have one magnitude each: plane 0
+// is a everywhere, plane 1 is a on the first half of the members and -a on the
+// second, planes 2 and 3 are +-b on the quarters of one half and zero on the
+// other.  So an entry needs no G value, only its member's quarter, and three
+// products instead of four: ch collects the half-plane of the current half and
+// is folded into its variance where the (ascending) members cross the middle.
+// Skipped terms are exact zeros, so every sum keeps its bits.  A voxel with one
+// entry (a third of 3-D entries' voxels, more in 2-D) is folded at once.
+//
+// An entry word is the byte offset of its row of S^T, with the quarter in the
+// two lowest bits.  RP pairs of coefficients per lane: 2 for P > 64 (S^T in
+// global memory, through L1), 1 for P in 33-64 (S^T in shared memory).
+template <int RP, int NQ>
+__device__ __forceinline__ void exact_haar(const float* lval, const int* lstart, const uint32_t* lent, int u_lo,
+                                           int u_hi, float a0, float b0, const float* __restrict__ st_lane,
+                                           uint32_t kron_lane, float2 (&var)[RP][NQ]) {
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+#pragma unroll
+        for (int r = 0; r < RP; ++r) var[r][q] = make_float2(0.0f, 0.0f);
+    if (u_lo >= u_hi) return;
+    const uint32_t ents = static_cast<uint32_t>(__cvta_generic_to_shared(lent));
+    uint32_t ls = static_cast<uint32_t>(__cvta_generic_to_shared(lstart + u_lo));
+    const uint32_t lv = static_cast<uint32_t>(__cvta_generic_to_shared(lval)) -
+                        static_cast<uint32_t>(__cvta_generic_to_shared(lstart));  // lval[u] at lv + &lstart[u]
+    uint32_t ep = ents + 4u * static_cast<uint32_t>(lstart[u_lo]);
+    const uint32_t end = ents + 4u * static_cast<uint32_t>(lstart[u_hi]);
+    const float2 A = make_float2(a0, a0), nA = make_float2(-a0, -a0), B = make_float2(b0, b0),
+                 nB = make_float2(-b0, -b0);
+    auto row = [&](float2 (&sv)[RP], uint32_t ent) {
+        if constexpr (RP == 2) {
+            const float4 t = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const char*>(st_lane) + (ent & ~3u)));
+            sv[0] = make_float2(t.x, t.y);
+            sv[RP - 1] = make_float2(t.z, t.w);
+        } else {
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+                         : "=f"(sv[0].x), "=f"(sv[0].y)
+                         : "r"(kron_lane + (ent & ~3u)));
+        }
+    };
+    uint32_t ent = lds32(ep);
+    uint32_t nx = lds32(ls + 4);
+    while (true) {
+        const uint32_t next = ents + 4u * nx;
+        const float v = __uint_as_float(lds32(ls + lv));
+        ls += 4;
+        nx = lds32(ls + 4);  // (one word past the last voxel's is readable)
+        const float2 vv = make_float2(v, v);
+        float2 sv[RP];
+        row(sv, ent);
+        uint32_t q = ent;
+        ep += 4;
+        ent = lds32(ep);
+        if (ep == next) {
+#pragma unroll
+            for (int r = 0; r < RP; ++r) {
+                const float2 c = __fmul2_rn(A, sv[r]), x = __fmul2_rn(vv, c);
+                var[r][0] = __ffma2_rn(x, c, var[r][0]);
+                if constexpr (NQ > 1) var[r][1] = __ffma2_rn(x, c, var[r][1]);
+            }
+            if constexpr (NQ > 2) {
+                float2 y[RP], d[RP];
+#pragma unroll
+                for (int r = 0; r < RP; ++r) {
+                    d[r] = __fmul2_rn(B, sv[r]);
+                    y[r] = __fmul2_rn(vv, d[r]);
+                }
+                if (q & 2u) {
+#pragma unroll
+                    for (int r = 0; r < RP; ++r) var[r][NQ - 1] = __ffma2_rn(y[r], d[r], var[r][NQ - 1]);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < RP; ++r) var[r][NQ - 2] = __ffma2_rn(y[r], d[r], var[r][NQ - 2]);
+                }
+            }
+        } else {
+            float2 c0[RP], c1[RP], ch[RP];
+            uint32_t half = q & 2u;
+            float2 m1 = half ? nA : A, mb = (q & 1u) ? nB : B;
+#pragma unroll
+            for (int r = 0; r < RP; ++r) {
+                c0[r] = __fmul2_rn(A, sv[r]);
+                if constexpr (NQ > 1) c1[r] = __fmul2_rn(m1, sv[r]);
+                if constexpr (NQ > 2) ch[r] = __fmul2_rn(mb, sv[r]);
+            }
+            do {
+                row(sv, ent);
+                q = ent;
+                ep += 4;
+                ent = lds32(ep);
+                mb = (q & 1u) ? nB : B;
+                if ((q & 2u) != half) {  // into the second half: plane 2 is complete
+                    half = 2u;
+                    m1 = nA;
+                    if constexpr (NQ > 2) {
+#pragma unroll
+                        for (int r = 0; r < RP; ++r) {
+                            var[r][NQ - 2] = __ffma2_rn(__fmul2_rn(vv, ch[r]), ch[r], var[r][NQ - 2]);
+                            ch[r] = __fmul2_rn(mb, sv[r]);
+                        }
+                    }
+                } else if constexpr (NQ > 2) {
+#pragma unroll
+                    for (int r = 0; r < RP; ++r) ch[r] = __ffma2_rn(mb, sv[r], ch[r]);
+                }
+#pragma unroll
+                for (int r = 0; r < RP; ++r) {
+                    c0[r] = __ffma2_rn(A, sv[r], c0[r]);
+                    if constexpr (NQ > 1) c1[r] = __ffma2_rn(m1, sv[r], c1[r]);
+                }
+            } while (ep != next);
+#pragma unroll
+            for (int r = 0; r < RP; ++r) {
+                var[r][0] = __ffma2_rn(__fmul2_rn(vv, c0[r]), c0[r], var[r][0]);
+                if constexpr (NQ > 1) var[r][1] = __ffma2_rn(__fmul2_rn(vv, c1[r]), c1[r], var[r][1]);
+            }
+            if constexpr (NQ > 2) {
+                if (half) {
+#pragma unroll
+                    for (int r = 0; r < RP; ++r)
+                        var[r][NQ - 1] = __ffma2_rn(__fmul2_rn(vv, ch[r]), ch[r], var[r][NQ - 1]);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < RP; ++r)
+                        var[r][NQ - 2] = __ffma2_rn(__fmul2_rn(vv, ch[r]), ch[r], var[r][NQ - 2]);
+                }
+            }
+        }
+        if (ep == end) break;
+    }
+}
+
+// all tiles of (NQ planes) x (32 JR coefficients); EX[i * P + j] receives the
 // standard deviation sqrt(max(var, 0)) of planes i < kk.  NQ = 4 in general;
 // groups with fewer exact planes (k < 4, or fewer members) use NQ = kk.  Each
 // warp leaves its partial sums in `part`; after one barrier every thread adds
 // the warps' partials of its (plane, coefficient) pairs in warp order.
-template <int JR, int NQ>
-__device__ void exact_planes(const float* __restrict__ lval, const int* __restrict__ lstart,
-                             const uint32_t* __restrict__ lent, int U, const float* __restrict__ GT,
-                             int kpad, int kk, const float* __restrict__ st, int P,
-                             float* __restrict__ EX, float* __restrict__ part) {
-    constexpr bool kHalf = JR == 2;
-    constexpr int RL = kHalf ? 4 : JR;       // coefficients per lane
-    constexpr int TW = kHalf ? 64 : 32 * JR;  // coefficients per tile
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+//
+// Patches of 33-64 voxels (JR = 2): the two half-warps take the two halves of
+// the warp's voxels and each lane holds 4 coefficients, j = 4 (lane % 16) + r,
+// so an entry costs the same loads for 4 NQ multiply-adds instead of 2 NQ; the
+// halves' sums are added at the end.  (A whole warp per half, without the
+// divergence where only one half ends a voxel, took 14 % more instructions.)
+template <int JR, int NQ, bool HAAR>
+__device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint32_t kron_byte, const float* __restrict__ lval,
+                             const int* __restrict__ lstart, const uint32_t* __restrict__ lent, int U,
+                             int kk, const float* __restrict__ st, int P,
+                             float* __restrict__ EX, float* __restrict__ part, bool part_over) {
+    constexpr bool kHalf = JR == 2 && !HAAR;
+    constexpr int RL = kHalf ? 4 : JR;  // coefficients per lane
+    constexpr int TW = 32 * JR;         // coefficients per tile
+    const uint32_t stride = static_cast<uint32_t>(kron_stride(P));
+    const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
     const int nw = blockDim.x >> 5;
     // voxel range of this warp: voxels whose first entry lies in its entry share
     const int E = lstart[U];
-    auto first_voxel = [&](int e) {
-        int lo = 0, hi = U;  // first u in [0, U] with lstart[u] >= e
+    auto first_voxel = [&](int e, int lo, int hi) {  // first u in [lo, hi] with lstart[u] >= e
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
             if (lstart[mid] < e) lo = mid + 1;
@@ -775,23 +1118,71 @@ __device__ void exact_planes(const float* __restrict__ lval, const int* __restri
         }
         return lo;
     };
-    const int u_lo = first_voxel(static_cast<int>(static_cast<int64_t>(E) * warp / nw));
-    const int u_hi = warp == nw - 1 ? U : first_voxel(static_cast<int>(static_cast<int64_t>(E) * (warp + 1) / nw));
+    const int u_lo = first_voxel(static_cast<int>(static_cast<int64_t>(E) * warp / nw), 0, U);
+    const int u_hi = warp == nw - 1 ? U : first_voxel(static_cast<int>(static_cast<int64_t>(E) * (warp + 1) / nw), 0, U);
     const int jl = kHalf ? 4 * (lane & 15) : JR * lane;
-    const bool writer = !kHalf || lane < 16;
     for (int i0 = 0; i0 < kk; i0 += NQ) {
         for (int j0 = 0; j0 < P; j0 += TW) {
-            float var[RL][NQ];
-            if constexpr (kHalf) exact_tile_hw<NQ>(lval, lstart, lent, u_lo, u_hi, GT, kpad, i0, st, var);
-            else exact_tile<JR, NQ>(lval, lstart, lent, u_lo, u_hi, GT, kpad, i0, st, j0, var);
-            if (writer) {
+            float out[RL][NQ];
+            if constexpr (HAAR && JR > 1) {
+                // JR == 2: the halves of the warp's voxels one after the other (their
+                // sums are added as in the generic form below)
+                constexpr int RP = JR / 2;
+                const int u_mid = JR == 2 ? first_voxel((lstart[u_lo] + lstart[u_hi]) >> 1, u_lo, u_hi) : u_hi;
+                const uint32_t kron_lane = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + kron_byte + 8u * lane;
+                float2 var[RP][NQ];
+                exact_haar<RP, NQ>(lval, lstart, lent, u_lo, u_mid, a0, b0, st + JR * lane, kron_lane, var);
 #pragma unroll
                 for (int q = 0; q < NQ; ++q)
 #pragma unroll
-                    for (int r = 0; r < RL; ++r) part[(warp * NQ + q) * TW + jl + r] = var[r][q];
+                    for (int r = 0; r < RP; ++r) {
+                        out[2 * r][q] = var[r][q].x;
+                        out[2 * r + 1][q] = var[r][q].y;
+                    }
+                if constexpr (JR == 2) {
+                    exact_haar<RP, NQ>(lval, lstart, lent, u_mid, u_hi, a0, b0, st + JR * lane, kron_lane, var);
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) {
+                        out[0][q] = add_rn(out[0][q], var[0][q].x);
+                        out[1][q] = add_rn(out[1][q], var[0][q].y);
+                    }
+                }
+            } else if constexpr (JR == 1) {
+                exact_stream<1, NQ>(lval, lstart, lent, u_lo, u_hi, smem, 8u * i0, stride, st + j0 + lane, out);
+            } else {
+                float2 var[2][NQ];
+                int lo = u_lo, hi = u_hi;
+                if (kHalf) {
+                    // split at the first voxel whose entries start in the second half of the entries
+                    const int u_mid = first_voxel((lstart[u_lo] + lstart[u_hi]) >> 1, u_lo, u_hi);
+                    if (lane >> 4) lo = u_mid;
+                    else hi = u_mid;
+                }
+                exact_pairs<NQ>(smem, lval, lstart, lent, lo, hi, 8u * i0, st + j0 + jl, 4u * stride, var);
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        out[2 * r][q] = var[r][q].x;
+                        out[2 * r + 1][q] = var[r][q].y;
+                    }
+                if (kHalf) {
+#pragma unroll
+                    for (int r = 0; r < RL; ++r)
+#pragma unroll
+                        for (int q = 0; q < NQ; ++q)
+                            out[r][q] = add_rn(out[r][q], __shfl_xor_sync(0xffffffffu, out[r][q], 16));
+                }
+            }
+            if (part_over) __syncthreads();  // every warp is done with the lists
+            if (!kHalf || lane < 16) {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+#pragma unroll
+                    for (int r = 0; r < RL; ++r) part[(warp * NQ + q) * TW + jl + r] = out[r][q];
             }
             __syncthreads();
-            for (int t = threadIdx.x; t < NQ * TW; t += blockDim.x) {
+            for (int t = static_cast<int>(threadIdx.x); t < NQ * TW; t += blockDim.x) {
                 const int q = t / TW, jj = t - q * TW;
                 const int i = i0 + q, j = j0 + jj;
                 if (i < kk && j < P) {
@@ -806,13 +1197,18 @@ __device__ void exact_planes(const float* __restrict__ lval, const int* __restri
 }
 
 template <int JR>
-__device__ void exact_planes_any(const float* __restrict__ lval, const int* __restrict__ lstart,
-                                 const uint32_t* __restrict__ lent, int U, const float* __restrict__ GT,
-                                 int kpad, int kk, const float* __restrict__ st, int P,
-                                 float* __restrict__ EX, float* __restrict__ part) {
-    if (kk == 1) exact_planes<JR, 1>(lval, lstart, lent, U, GT, kpad, kk, st, P, EX, part);
-    else if (kk == 2) exact_planes<JR, 2>(lval, lstart, lent, U, GT, kpad, kk, st, P, EX, part);
-    else exact_planes<JR, 4>(lval, lstart, lent, U, GT, kpad, kk, st, P, EX, part);
+__device__ void exact_planes_any(const unsigned char* smem, bool haar, float a0, float b0, uint32_t kron_byte,
+                                 const float* __restrict__ lval, const int* __restrict__ lstart,
+                                 const uint32_t* __restrict__ lent, int U, int kk, const float* __restrict__ st, int P,
+                                 float* __restrict__ EX, float* __restrict__ part, bool part_over) {
+    auto run = [&](auto h) {
+        constexpr bool H = decltype(h)::value;
+        if (kk == 1) exact_planes<JR, 1, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        else if (kk == 2) exact_planes<JR, 2, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        else exact_planes<JR, 4, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+    };
+    if (JR > 1 && haar) run(BoolTag<JR != 1>{});
+    else run(BoolTag<false>{});
 }
 
 // Exact noise risk of the first kk planes (wiener.py:638-711, :505-535; the
@@ -824,12 +1220,12 @@ __device__ void exact_planes_any(const float* __restrict__ lval, const int* __re
 // one tile); (f SM)[j] = sum_p f[p] SM[p][j] takes f[p] from its lane by a
 // shuffle.  The voxel terms are float32, their sum over voxels float64.
 template <int JR, int NQ>
-__device__ double exact_risk_tile(const float* __restrict__ lval, const int* __restrict__ lstart,
+__device__ double exact_risk_tile(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
                                   const uint32_t* __restrict__ lent, int u_lo, int u_hi,
-                                  const float* __restrict__ GT, int kpad, int i0, int kk,
+                                  int i0, int kk,
                                   const float* __restrict__ st, const float* __restrict__ smt,
                                   const float* __restrict__ att, int P) {
-    const int lane = threadIdx.x & 31;
+    const int lane = static_cast<int>(threadIdx.x) & 31;
     const int stride = kron_stride(P);
     const float* stl = st + JR * lane;
     float gq[JR][NQ];
@@ -840,7 +1236,6 @@ __device__ double exact_risk_tile(const float* __restrict__ lval, const int* __r
             const int j = JR * lane + r, i = i0 + q;
             gq[r][q] = (j < P && i < kk) ? att[i * P + j] : 0.0f;
         }
-    const float* gt0 = GT + i0;
     double acc = 0.0;
     for (int u = u_lo; u < u_hi; ++u) {
         int e = lstart[u];
@@ -849,9 +1244,9 @@ __device__ double exact_risk_tile(const float* __restrict__ lval, const int* __r
         {
             const uint32_t ent = lent[e];
             PlaneVec<NQ> gv;
-            gv.load(gt0 + (ent & 0xffu) * kpad);
+            gv.load_pairs(smem + 8 * i0 + (ent & 0xffffu));
             KronVec<JR> sv;
-            sv.load(stl + (ent >> 8));
+            sv.load(stl + (ent >> 16) * static_cast<uint32_t>(stride));
 #pragma unroll
             for (int r = 0; r < JR; ++r)
 #pragma unroll
@@ -860,9 +1255,9 @@ __device__ double exact_risk_tile(const float* __restrict__ lval, const int* __r
         for (++e; e < e1; ++e) {
             const uint32_t ent = lent[e];
             PlaneVec<NQ> gv;
-            gv.load(gt0 + (ent & 0xffu) * kpad);
+            gv.load_pairs(smem + 8 * i0 + (ent & 0xffffu));
             KronVec<JR> sv;
-            sv.load(stl + (ent >> 8));
+            sv.load(stl + (ent >> 16) * static_cast<uint32_t>(stride));
 #pragma unroll
             for (int r = 0; r < JR; ++r)
 #pragma unroll
@@ -907,11 +1302,10 @@ __device__ double exact_risk_tile(const float* __restrict__ lval, const int* __r
 // warp w takes the voxels whose entry lists start in its share of all entries
 // (the exact variance's split); lanes, then warps, add in a fixed order
 template <int JR, int NQ>
-__device__ void exact_risk(const float* __restrict__ lval, const int* __restrict__ lstart,
-                           const uint32_t* __restrict__ lent, int U, const float* __restrict__ GT, int kpad,
-                           int kk, const float* __restrict__ st, const float* __restrict__ smt,
+__device__ void exact_risk(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
+                           const uint32_t* __restrict__ lent, int U, int kk, const float* __restrict__ st, const float* __restrict__ smt,
                            const float* __restrict__ att, int P, double* __restrict__ part) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
     const int nw = blockDim.x >> 5;
     const int E = lstart[U];
     auto first_voxel = [&](int e) {
@@ -927,12 +1321,12 @@ __device__ void exact_risk(const float* __restrict__ lval, const int* __restrict
     const int u_hi = warp == nw - 1 ? U : first_voxel(static_cast<int>(static_cast<int64_t>(E) * (warp + 1) / nw));
     double acc = 0.0;
     for (int i0 = 0; i0 < kk; i0 += NQ)
-        acc += exact_risk_tile<JR, NQ>(lval, lstart, lent, u_lo, u_hi, GT, kpad, i0, kk, st, smt, att, P);
+        acc += exact_risk_tile<JR, NQ>(smem, lval, lstart, lent, u_lo, u_hi, i0, kk, st, smt, att, P);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) part[warp] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (static_cast<int>(threadIdx.x) == 0) {
         double t = 0.0;
         for (int w = 0; w < nw; ++w) t += part[w];
         part[nw] = t;
@@ -941,23 +1335,30 @@ __device__ void exact_risk(const float* __restrict__ lval, const int* __restrict
 }
 
 template <int JR>
-__device__ void exact_risk_any(const float* __restrict__ lval, const int* __restrict__ lstart,
-                               const uint32_t* __restrict__ lent, int U, const float* __restrict__ GT, int kpad,
+__device__ void exact_risk_any(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
+                               const uint32_t* __restrict__ lent, int U,
                                int kk, const float* __restrict__ st, const float* __restrict__ smt,
                                const float* __restrict__ att, int P, double* __restrict__ part) {
-    if (kk == 1) exact_risk<JR, 1>(lval, lstart, lent, U, GT, kpad, kk, st, smt, att, P, part);
-    else if (kk == 2) exact_risk<JR, 2>(lval, lstart, lent, U, GT, kpad, kk, st, smt, att, P, part);
-    else exact_risk<JR, 4>(lval, lstart, lent, U, GT, kpad, kk, st, smt, att, P, part);
+    if (kk == 1) exact_risk<JR, 1>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
+    else if (kk == 2) exact_risk<JR, 2>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
+    else exact_risk<JR, 4>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
 }
 
-template <int ND, int B0, int B1, int B2, int NT>
-__global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) group_filter_kernel(FilterArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
+// f(member, patch element, index) over an n x P group: a warp takes whole rows
+template <typename F>
+__device__ __forceinline__ void for_members(int n, int P, F f) {
+    const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31, nw = blockDim.x >> 5;
+    for (int g = warp; g < n; g += nw)
+        for (int p = lane; p < P; p += 32) f(g, p, g * P + p);
+}
+
+// One group, by a whole CTA.
+template <int ND, int B0, int B1, int B2>
+__device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char* smem, int64_t gid) {
     using GM = Geom<ND, B0, B1, B2>;
     const BmndStageParams& sp = a.sp;
     const GM geo(sp);
-    const int64_t gid = blockIdx.x;
-    const int tid = threadIdx.x;
+    const int tid = static_cast<int>(threadIdx.x);
     const int P = geo.P();
     const int n = a.count[gid];
     if (n <= 0) return;
@@ -966,15 +1367,17 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
         return;
     }
     const bool wiener = sp.filter == BMND_FILTER_WIENER;
+    const int kmax = a.kmax;
 
     float* G = sm<float>(smem, a.L.g);
-    float* GT = sm<float>(smem, a.L.gt);
+    float2* GT2 = sm<float2>(smem, a.L.gt2);
     float* Fw = sm<float>(smem, a.L.fw);
-    float* Fi = sm<float>(smem, a.L.fi);
     float* win = sm<float>(smem, a.L.win);
     double* mdiag = sm<double>(smem, a.L.mdiag);
+    int* voff = sm<int>(smem, a.L.voff);
     int* pos = sm<int>(smem, a.L.pos);
     int* shf = sm<int>(smem, a.L.shf);
+    int* org0 = sm<int>(smem, a.L.org0);
     float* S = sm<float>(smem, a.L.s);
     float* EX = sm<float>(smem, a.L.ex);
     float* X = sm<float>(smem, a.L.x);
@@ -993,7 +1396,60 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
     const int kk = k < n ? k : n;
     const int kpad = (a.kmax + 3) / 4 * 4;
 
-    // ---- setup: positions, matrices, window ----
+    // ---- setup: constants of the launch, positions, group matrix ----
+    {
+        float* Fi = sm<float>(smem, a.L.fi);
+        if (ND > 0 && !sp.exact_risk_weights) {
+            // from the tables spatial_kron_kernel left after S^T: the parameters
+            // live in the constant bank, where lanes reading different addresses
+            // take turns
+            const float* tab = a.st + static_cast<int64_t>(P) * kron_stride(P);
+            constexpr int EE = BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE;
+            for (int e = tid; e < EE; e += blockDim.x) {
+                Fw[e] = __ldg(tab + e);
+                Fi[e] = __ldg(tab + EE + e);
+            }
+            for (int e = tid; e < P; e += blockDim.x) win[e] = __ldg(tab + 2 * EE + e);
+        } else {
+            for (int d = 0; d < geo.nd(); ++d) {
+                const int bb = geo.b(d) * geo.b(d);
+                for (int q = tid; q < bb; q += blockDim.x) {
+                    Fw[d * BMND_MAX_EDGE * BMND_MAX_EDGE + q] = sp.spatial_fwd[d][q];
+                    Fi[d * BMND_MAX_EDGE * BMND_MAX_EDGE + q] = sp.spatial_inv[d][q];
+                }
+            }
+            for (int e = tid; e < P; e += blockDim.x) win[e] = sp.window[e];
+        }
+        for (int e = tid; e < P; e += blockDim.x) {
+            int p = e, off = 0;
+#pragma unroll
+            for (int d = BMND_MAX_DIMS - 1; d >= 0; --d) {
+                if (d < geo.nd()) {
+                    off += (p % geo.b(d)) * static_cast<int>(a.vstride[d]);
+                    p /= geo.b(d);
+                }
+            }
+            voff[e] = off;
+        }
+        if (sp.windowed_synthesis)  // the only reader of the metric diagonal
+            for (int e = tid; e < P; e += blockDim.x) mdiag[e] = sp.spatial_metric_diag[e];
+        if (kron_in_smem(sp, P, kmax)) {
+            float4* kron = sm<float4>(smem, a.L.kron);
+            const int words = P * kron_stride(P) / 4;
+            for (int e = tid; e < words; e += blockDim.x) kron[e] = __ldg(reinterpret_cast<const float4*>(a.st) + e);
+        }
+        if (a.den_ro) {
+            // matrices are stored densely, b x b row-major, per axis
+            float* Fit = sm<float>(smem, a.L.fit);
+            constexpr int EE = BMND_MAX_EDGE * BMND_MAX_EDGE;
+            for (int e = tid; e < BMND_MAX_DIMS * EE; e += blockDim.x) {
+                const int d = e / EE, q = e % EE;
+                const int b = d < geo.nd() ? geo.b(d) : 1;
+                const int i = q / b, k = q % b;
+                Fit[e] = q < b * b ? sp.spatial_inv[d][k * b + i] : 0.0f;
+            }
+        }
+    }
     // a member outside the patch grid skips the group (matching never makes one)
     bool bad_member = false;
     if (tid < n) {
@@ -1001,50 +1457,35 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
         bad_member = lin < 0 || lin >= a.n_lins;
         // lins fit in 31 bits (volumes are limited to 2^31 voxels): 32-bit division
         uint32_t rem = static_cast<uint32_t>(lin);
+        int origin = 0;
         for (int d = geo.nd() - 1; d >= 0 && !bad_member; --d) {
             const uint32_t c = static_cast<uint32_t>(a.counts[d]);
             const uint32_t q = rem / c;
             pos[tid * BMND_MAX_DIMS + d] = static_cast<int>(rem - q * c);
+            origin += static_cast<int>(rem - q * c) * static_cast<int>(a.vstride[d]);
             rem = q;
         }
+        org0[tid] = origin;
     }
     if (__syncthreads_or(bad_member)) {
         if (tid == 0 && a.err) atomicExch(a.err, 2);
         return;
     }
+    // the exact phase's entries carry quarters of the Haar group (exact_haar)
+    const bool quarters = ND > 0 && kron_jr(P) > 1 && sp.group_transform == BMND_GROUP_HAAR && is_pow2(n) &&
+                          sp.noise_model == BMND_NOISE_POISSON && k <= 4;
     {
         const float* gtab = a.st + 2 * static_cast<int64_t>(P) * kron_stride(P) + group_table_offset(n);
         for (int e = tid; e < n * n; e += blockDim.x) G[e] = __ldg(gtab + e);
-    }
-    // only the b x b entries of each axis are read; the parameters live in the
-    // constant bank, where lanes reading different addresses take turns
-    for (int d = 0; d < geo.nd(); ++d) {
-        const int bb = geo.b(d) * geo.b(d);
-        for (int q = tid; q < bb; q += blockDim.x) {
-            Fw[d * BMND_MAX_EDGE * BMND_MAX_EDGE + q] = sp.spatial_fwd[d][q];
-            Fi[d * BMND_MAX_EDGE * BMND_MAX_EDGE + q] = sp.spatial_inv[d][q];
+        // G^T restricted to the exact planes, padded to 4, each entry twice:
+        // GT2[g * kpad + i] = (G[i, g], G[i, g])
+        for (int e = tid; !quarters && e < n * kpad; e += blockDim.x) {
+            const int g = e / kpad, i = e % kpad;
+            const float v = i < kk ? __ldg(gtab + i * n + g) : 0.0f;
+            GT2[e] = make_float2(v, v);
         }
     }
-    for (int e = tid; e < P; e += blockDim.x) win[e] = sp.window[e];
-    if (sp.windowed_synthesis)  // the only reader of the metric diagonal
-        for (int e = tid; e < P; e += blockDim.x) mdiag[e] = sp.spatial_metric_diag[e];
-    if (a.den_ro) {
-        // matrices are stored densely, b x b row-major, per axis
-        float* Fit = sm<float>(smem, a.L.fit);
-        constexpr int EE = BMND_MAX_EDGE * BMND_MAX_EDGE;
-        for (int e = tid; e < BMND_MAX_DIMS * EE; e += blockDim.x) {
-            const int d = e / EE, q = e % EE;
-            const int b = d < geo.nd() ? geo.b(d) : 1;
-            const int i = q / b, k = q % b;
-            Fit[e] = q < b * b ? sp.spatial_inv[d][k * b + i] : 0.0f;
-        }
-    }
-    __syncthreads();
-    // G^T restricted to the exact planes, padded to 4: GT[g * kpad + i] = G[i, g]
-    for (int e = tid; e < n * kpad; e += blockDim.x) {
-        int g = e / kpad, i = e % kpad;
-        GT[e] = i < kk ? G[i * n + g] : 0.0f;
-    }
+    if (tid == 32) misc[kMiscWild] = 0;
     if (tid < 32) {
         // group origin (min over members), member shifts, union extent, and the
         // patch-linear offset of each shift: element p of member g lies in union
@@ -1161,99 +1602,118 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
             org[d] = misc[d];
             ucells *= ush[d];
         }
-        for (int c = tid; c < ucells; c += blockDim.x) grid[c] = 0u;
-        __syncthreads();
-        for (int e = tid; e < total; e += blockDim.x) {
-            const int g = e / P;
-            int p = e - g * P;
-            int cell = 0, mul = 1;
-#pragma unroll
-            for (int d = BMND_MAX_DIMS - 1; d >= 0; --d) {
-                if (d < geo.nd()) {
-                    cell += (shf[g * BMND_MAX_DIMS + d] + p % geo.b(d)) * mul;
-                    mul *= ush[d];
-                    p /= geo.b(d);
-                }
-            }
-            atomicOr(grid + cell, 1u << g);
+        // A union cell's members are those whose patch reaches its coordinate on
+        // every axis: one member mask per axis coordinate, ANDed per cell.
+        int aoff[BMND_MAX_DIMS] = {0, 0, 0}, masks = 0;
+        for (int d = 0; d < geo.nd(); ++d) {
+            aoff[d] = masks;
+            masks += ush[d];
         }
-        __syncthreads();
-        // compact occupied cells (ascending) and their entries (ascending
-        // member): warp w takes a contiguous 1/nw of the cells, 32 at a time,
-        // one cell per lane; voxel ranks come from ballots and entry offsets
-        // from a warp scan of the cells' member counts, after the warps'
-        // totals are added up in warp order.  The cell index is parked in lval
-        // until the variance pass below.
         {
             const int nw = blockDim.x >> 5, warp = tid >> 5, lane = tid & 31;
-            const int cpw = (ucells + nw - 1) / nw;
-            const int wc0 = min(ucells, warp * cpw), wc1 = min(ucells, wc0 + cpw);
-            int wv = 0, wsum = 0;
-            for (int base = wc0; base < wc1; base += 32) {
-                const int c = base + lane;
-                const uint32_t m = c < wc1 ? grid[c] : 0u;
-                wv += __popc(__ballot_sync(0xffffffffu, m != 0u));
-                wsum += __popc(m);
+            for (int q = warp; q < masks; q += nw) {
+                int d = 0;
+#pragma unroll
+                for (int t = 1; t < BMND_MAX_DIMS; ++t)
+                    if (t < geo.nd() && q >= aoff[t]) d = t;
+                const int c = q - aoff[d];
+                const int bd = geo.b(d);
+                const bool in = lane < n && static_cast<unsigned>(c - shf[lane * BMND_MAX_DIMS + d]) < static_cast<unsigned>(bd);
+                const uint32_t m = __ballot_sync(0xffffffffu, in);
+                if (lane == 0) grid[q] = m;
             }
+        }
+        __syncthreads();
+        // Occupied cells (ascending) and their entries (ascending member): thread t
+        // takes a contiguous 1/NT of the cells, counts its voxels and entries, gets
+        // its offsets from a block scan and writes them.  The voxel's offset in the
+        // volume is parked in lval until the variance pass below.
+        {
+            const int last = geo.nd() - 1;
+            const int cpt = (ucells + static_cast<int>(blockDim.x) - 1) / static_cast<int>(blockDim.x);
+            const int c0 = min(ucells, tid * cpt), c1 = min(ucells, c0 + cpt);
+            const uint32_t* xm = grid + aoff[last];
+            const int ux = ush[last];
+            // walk(f): f(mask, position) over this thread's occupied cells
+            auto walk = [&](auto f) {
+                int cc[BMND_MAX_DIMS] = {0, 0, 0};
+                int rem = c0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-            if (lane == 0) scan[warp] = make_int2(wv, wsum);
-            __syncthreads();
-            int vbase = 0, ebase = 0, vtot = 0, etot = 0;
-            for (int w = 0; w < nw; ++w) {
-                const int2 t = scan[w];
-                if (w < warp) {
-                    vbase += t.x;
-                    ebase += t.y;
+                for (int d = BMND_MAX_DIMS - 1; d >= 0; --d) {
+                    if (d < geo.nd()) {
+                        const int q = d > 0 ? small_div(rem, 1.0f / static_cast<float>(ush[d])) : 0;
+                        cc[d] = rem - q * ush[d];
+                        rem = q;
+                    }
                 }
-                vtot += t.x;
-                etot += t.y;
-            }
-            const int* shl = sm<int>(smem, a.L.shl);
-            const int kstride = kron_stride(P);
-            float inv_ush[BMND_MAX_DIMS];
+                int c = c0;
+                while (c < c1) {
+                    uint32_t outer = 0xffffffffu;
+                    int vox = 0, lin = 0;
 #pragma unroll
-            for (int d = 0; d < BMND_MAX_DIMS; ++d) inv_ush[d] = 1.0f / static_cast<float>(ush[d]);
-            const uint32_t below = (1u << lane) - 1u;
-            for (int base = wc0; base < wc1; base += 32) {
-                const int c = base + lane;
-                uint32_t m = c < wc1 ? grid[c] : 0u;
-                const uint32_t occ = __ballot_sync(0xffffffffu, m != 0u);
-                const int cnt = __popc(m);
-                int incl = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                if (m) {
-                    const int w = vbase + __popc(occ & below);
-                    int we = ebase + incl - cnt;
-                    // cell -> union-box coordinates -> patch-linear offset
-                    int rem = c, lin = 0, cc[BMND_MAX_DIMS] = {0, 0, 0};
-#pragma unroll
-                    for (int d = BMND_MAX_DIMS - 1; d >= 0; --d) {
-                        if (d < geo.nd()) {
-                            const int q = d > 0 ? small_div(rem, inv_ush[d]) : 0;
-                            cc[d] = rem - q * ush[d];
-                            rem = q;
+                    for (int d = 0; d < BMND_MAX_DIMS; ++d) {
+                        if (d < last) {
+                            outer &= grid[aoff[d] + cc[d]];
+                            vox += (cc[d] + org[d]) * static_cast<int>(a.vstride[d]);
+                            lin += cc[d] * geo.inner(d);
                         }
                     }
+                    const int x = cc[last];
+                    const int run = min(ux - x, c1 - c);
+                    if (outer) {
+                        for (int k = 0; k < run; ++k) {
+                            const uint32_t m = outer & xm[x + k];
+                            if (m) f(m, vox + x + k + org[last], lin + x + k);
+                        }
+                    }
+                    c += run;
+                    cc[last] = 0;
 #pragma unroll
-                    for (int d = 0; d < BMND_MAX_DIMS; ++d)
-                        if (d < geo.nd()) lin += cc[d] * geo.inner(d);
-                    reinterpret_cast<int*>(lval)[w] = c;
-                    lstart[w] = we;
-                    while (m) {
-                        const int g = __ffs(m) - 1;
-                        m &= m - 1;
-                        lent[we++] = static_cast<uint32_t>(g) | (static_cast<uint32_t>((lin - shl[g]) * kstride) << 8);
+                    for (int d = BMND_MAX_DIMS - 1; d >= 0; --d) {
+                        if (d < last) {
+                            if (++cc[d] < ush[d]) break;
+                            cc[d] = 0;
+                        }
                     }
                 }
-                vbase += __popc(occ);
-                ebase += __shfl_sync(0xffffffffu, incl, 31);
+            };
+            uint32_t mine = 0;  // voxels << 16 | entries (both below 2^15)
+            walk([&](uint32_t m, int, int) { mine += 0x10000u + static_cast<uint32_t>(__popc(m)); });
+            const int nw = blockDim.x >> 5, warp = tid >> 5, lane = tid & 31;
+            uint32_t incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
             }
-            if (tid == 0) scan[blockDim.x] = make_int2(vtot, etot);
+            if (lane == 31) scan[warp].x = static_cast<int>(incl);
+            __syncthreads();
+            uint32_t base = 0, all = 0;
+            for (int w = 0; w < nw; ++w) {
+                const uint32_t t = static_cast<uint32_t>(scan[w].x);
+                if (w < warp) base += t;
+                all += t;
+            }
+            base += incl - mine;
+            int w = static_cast<int>(base >> 16), we = static_cast<int>(base & 0xffffu);
+            const int* shl = sm<int>(smem, a.L.shl);
+            const uint32_t gt2_off = static_cast<uint32_t>(a.L.gt2), row_b = 4u * static_cast<uint32_t>(kron_stride(P));
+            const int lg = ilog2_floor(n);
+            walk([&](uint32_t m, int vox, int lin) {
+                reinterpret_cast<int*>(lval)[w] = vox;
+                lstart[w++] = we;
+                do {
+                    const int g = __ffs(m) - 1;
+                    m &= m - 1;
+                    const uint32_t pe = static_cast<uint32_t>(lin - shl[g]);
+                    lent[we++] = quarters ? pe * row_b + static_cast<uint32_t>((4 * g) >> lg)
+                                          : gt2_off + static_cast<uint32_t>(g * kpad * 8) + (pe << 16);
+                } while (m);
+            });
+            if (tid == 0) {
+                scan[blockDim.x] = make_int2(static_cast<int>(all >> 16), static_cast<int>(all & 0xffffu));
+                lent[all & 0xffffu] = lent[(all & 0xffffu) + 1] = quarters ? 0u : gt2_off;  // read ahead, never used
+            }
         }
         __syncthreads();
         U = scan[blockDim.x].x;
@@ -1265,30 +1725,22 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
                 lval[u] = sp.exact_source_variance;
                 continue;
             }
-            int rem = reinterpret_cast<const int*>(lval)[u];
-            int64_t vox = 0;
-#pragma unroll
-            for (int d = BMND_MAX_DIMS - 1; d >= 0; --d) {
-                if (d < geo.nd()) {
-                    const int q = d > 0 ? small_div(rem, 1.0f / static_cast<float>(ush[d])) : 0;
-                    vox += static_cast<int64_t>(rem - q * ush[d] + org[d]) * a.vstride[d];
-                    rem = q;
-                }
-            }
+            const int vox = reinterpret_cast<const int*>(lval)[u];
             lval[u] = variance_of(__ldg(varsrc + vox), scale_f, floor_f);
         }
         __syncthreads();
         if (gauss) {
             // sigma comes from the covariance maps
         } else if constexpr (ND > 0) {
-            exact_planes_any<kron_jr(B0 * B1 * B2)>(lval, lstart, lent, U, GT, kpad, kk, a.st, P, EX,
-                                                    sm<float>(smem, a.L.part));
+            exact_planes_any<kron_jr(B0 * B1 * B2)>(smem, quarters, G[0], kk > 2 ? G[2 * n] : 0.0f,
+                                                    static_cast<uint32_t>(a.L.kron), lval, lstart, lent, U, kk, a.st,
+                                                    P, EX, sm<float>(smem, a.L.part), a.L.part_over != 0);
         } else {
             const int jr = kron_jr(P);
             float* part = sm<float>(smem, a.L.part);
-            if (jr == 1) exact_planes_any<1>(lval, lstart, lent, U, GT, kpad, kk, a.st, P, EX, part);
-            else if (jr == 2) exact_planes_any<2>(lval, lstart, lent, U, GT, kpad, kk, a.st, P, EX, part);
-            else exact_planes_any<4>(lval, lstart, lent, U, GT, kpad, kk, a.st, P, EX, part);
+            if (jr == 1) exact_planes_any<1>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            else if (jr == 2) exact_planes_any<2>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            else exact_planes_any<4>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
         }
     }
 
@@ -1296,17 +1748,21 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
     // (after the exact phase: S shares the union region with its lists)
     // The observation (and the pilot) are gathered here too, so the volume the
     // variance comes from is read once (its lists are no longer needed).
-    bool gathered = false;
+    bool gathered = false, wild = false;
     bool fused = false;  // X and R already forward-transformed with S
     if (!gauss && need_approx) {
-        for (int e = tid; e < total; e += blockDim.x) {
-            const int g = e / P;
-            const int64_t off = geo.offset(pos + g * BMND_MAX_DIMS, e - g * P, a.vstride);
+        for_members(n, P, [&](int g, int p, int e) {
+            const int off = org0[g] + voff[p];
             const float vs = __ldg(varsrc + off);
-            S[e] = variance_of(vs, scale_f, floor_f);
-            X[e] = varsrc == a.noisy ? vs : __ldg(a.noisy + off);
-            if (wiener) R[e] = varsrc == a.pilot ? vs : __ldg(a.pilot + off);
-        }
+            const float vv = variance_of(vs, scale_f, floor_f);
+            const float xv = varsrc == a.noisy ? vs : __ldg(a.noisy + off);
+            const float rv = !wiener ? 0.0f : (varsrc == a.pilot ? vs : __ldg(a.pilot + off));
+            S[e] = vv;
+            X[e] = xv;
+            if (wiener) R[e] = rv;
+            wild |= !(vv < 1e30f && fabsf(xv) < 1e30f && fabsf(rv) < 1e30f);
+        });
+        if (wild) misc[kMiscWild] = 1;
         gathered = true;
         __syncthreads();
         fused = transform_forward3<ND, B0, B1, B2>(geo, a, smem, n, S, X, wiener ? R : nullptr);
@@ -1373,12 +1829,15 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
 
     // ---- gather and forward-transform the observation (and the pilot) ----
     if (!gathered) {
-        for (int e = tid; e < total; e += blockDim.x) {
-            const int g = e / P;
-            const int64_t off = geo.offset(pos + g * BMND_MAX_DIMS, e - g * P, a.vstride);
-            X[e] = __ldg(a.noisy + off);
-            if (wiener) R[e] = __ldg(a.pilot + off);
-        }
+        for_members(n, P, [&](int g, int p, int e) {
+            const int off = org0[g] + voff[p];
+            const float xv = __ldg(a.noisy + off);
+            const float rv = wiener ? __ldg(a.pilot + off) : 0.0f;
+            X[e] = xv;
+            if (wiener) R[e] = rv;
+            wild |= !(fabsf(xv) < 1e30f && fabsf(rv) < 1e30f);
+        });
+        if (wild) misc[kMiscWild] = 1;
         __syncthreads();
     }
     if (!fused) {
@@ -1472,9 +1931,9 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
         if (exact_risk) {
             const float* smt = a.st + static_cast<int64_t>(P) * kron_stride(P);
             const int jr = kron_jr(P);
-            if (jr == 1) exact_risk_any<1>(lval, lstart, lent, U, GT, kpad, kk, a.st, smt, V, P, riskp);
-            else if (jr == 2) exact_risk_any<2>(lval, lstart, lent, U, GT, kpad, kk, a.st, smt, V, P, riskp);
-            else exact_risk_any<4>(lval, lstart, lent, U, GT, kpad, kk, a.st, smt, V, P, riskp);
+            if (jr == 1) exact_risk_any<1>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
+            else if (jr == 2) exact_risk_any<2>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
+            else exact_risk_any<4>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
         }
     }
 
@@ -1672,11 +2131,9 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
             a.store.wstore[s] = wts[tid];
         }
         __syncthreads();
-        for (int e = tid; e < total; e += blockDim.x) {
-            const int g = e / P;
-            const int p = e - g * P;
+        for_members(n, P, [&](int g, int p, int e) {
             a.store.store[static_cast<int64_t>(slot[g]) * a.store.row + p] = mul_rn(X[e], mul_rn(wts[g], win[p]));
-        }
+        });
         return;
     }
     for (int e = tid; e < total; e += blockDim.x) {
@@ -1696,10 +2153,28 @@ __global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) gr
     }
 }
 
+// One CTA per group.  (Persistent CTAs walking the groups, which would set up the
+// constants once, spill: the compiler then keeps 1.9 KB of local memory a thread.)
+template <int ND, int B0, int B1, int B2, int NT>
+__global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) group_filter_kernel(FilterArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    filter_group<ND, B0, B1, B2>(a, smem, blockIdx.x);
+}
+
 // S^T[p * stride + j] = S[j, p] with S = kron(F_0, ..., F_{nd-1}) built axis by
 // axis in float32 (fl(fl(F0 * F1) * F2)), as the reference builds its spatial
 // matrix (variance.py:744-755); columns j >= P of the padded rows are zero
 __global__ void spatial_kron_kernel(BmndStageParams sp, int P, int stride, float* st) {
+    if (blockIdx.x == 0 && P >= 64 && !sp.exact_risk_weights) {
+        // the matrices and the window as a table after S^T (the place of the risk metric)
+        constexpr int E1 = BMND_MAX_EDGE * BMND_MAX_EDGE, EE = BMND_MAX_DIMS * E1;
+        float* tab = st + static_cast<int64_t>(P) * stride;
+        for (int e = threadIdx.x; e < EE; e += blockDim.x) {
+            tab[e] = sp.spatial_fwd[e / E1][e % E1];
+            tab[EE + e] = sp.spatial_inv[e / E1][e % E1];
+        }
+        for (int e = threadIdx.x; e < P; e += blockDim.x) tab[2 * EE + e] = sp.window[e];
+    }
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < P * stride; idx += gridDim.x * blockDim.x) {
         const int p = idx / stride, j = idx % stride;
         if (j >= P) {
