@@ -120,9 +120,9 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.sg = take(sigma && !wiener ? 4 * np : 16);
     L.ex = take(4 * static_cast<int64_t>(kmax) * P);
 
-    // Gaussian noise: lag index of every member pair (i >= j)
+    // Gaussian noise: covariance-map row of every member pair (i > j)
     const bool gauss = sp.noise_model == BMND_NOISE_GAUSSIAN;
-    L.lag = take(gauss && kmax > 0 ? 4 * static_cast<int64_t>(nmax) * (nmax + 1) / 2 : 16);
+    L.lag = take(gauss && kmax > 0 ? 4 * static_cast<int64_t>(nmax) * ((nmax + 3) / 4 * 4) : 16);
     L.scan = take(8 * (kThreads + 1));
     L.plane = take(8 * (nmax > 40 ? nmax : 40));  // also the mass phase's 8 warps x 5 sums
     L.wts = take(4 * nmax);
@@ -1352,6 +1352,72 @@ __device__ __forceinline__ void for_members(int n, int P, F f) {
         for (int p = lane; p < P; p += 32) f(g, p, g * P + p);
 }
 
+// Exact Gaussian variances of planes 0 .. 3 of a Haar group (kk of them): with
+// plane magnitudes a (planes 0, 1) and b (2, 3), every product of the pair sums
+//   sum_i w_i C(0) w_i + sum_{j < i} (w_i w_j) 2 C(lag_ij)
+// is +-a^2 or +-b^2 times 2 C, so planes 0 and 1 share one load and one product
+// per pair, and planes 2 and 3 take the pairs within one half of the members.
+// (One thread per plane and coefficient loaded every covariance four times, 528
+// rows per plane, and was bound by those loads.)  Half of the threads sum planes
+// 0 and 1, the other half 2 and 3; a thread's coefficient is its index.  The sums
+// keep the generic order (ascending i, then j), with up to 8 loads in flight.
+__device__ __forceinline__ void gauss_haar(const float* __restrict__ cm, const int* lag, int lrow, int n, int kk, int P,
+                                           const float* G, float* EX) {
+    const int half_threads = blockDim.x >> 1;
+    const bool outer = static_cast<int>(threadIdx.x) < half_threads;  // planes 0 and 1
+    const int c = outer ? threadIdx.x : threadIdx.x - half_threads;
+    if (c >= P || (!outer && kk <= 2)) return;
+    const float w = outer ? G[0] : G[2 * n];
+    const float pv = __ldg(cm + c), ww = mul_rn(w, w), diag = mul_rn(mul_rn(w, pv), w);
+    const float* cc = cm + c;
+    float v0 = 0.0f, v1 = 0.0f;
+    const int half = n >> 1, quarter = n >> 2;
+    // pairs (i, j0 <= j < j1), all of one sign in plane 1 (planes 2, 3: in v0)
+    auto run = [&](int i, int j0, int j1, bool minus) {
+        const int* row = lag + i * lrow;
+        for (int j = j0; j < j1; j += 8) {
+            float cv[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) cv[u] = j + u < j1 ? __ldg(cc + row[j + u]) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (j + u < j1) {
+                    const float t = mul_rn(ww, add_rn(cv[u], cv[u]));
+                    if (outer) {
+                        v0 = add_rn(v0, t);
+                        v1 = minus ? sub_rn(v1, t) : add_rn(v1, t);
+                    } else {
+                        v0 = minus ? sub_rn(v0, t) : add_rn(v0, t);
+                    }
+                }
+            }
+        }
+    };
+    if (outer) {
+        for (int i = 0; i < n; ++i) {
+            v0 = add_rn(v0, diag);
+            v1 = add_rn(v1, diag);
+            const int split = i >= half ? half : 0;  // second-half member: the first half counts negatively
+            run(i, 0, split, true);
+            run(i, split, i, false);
+        }
+        EX[c] = fmaxf(v0, 0.0f);
+        if (kk > 1) EX[P + c] = fmaxf(v1, 0.0f);
+    } else {
+        for (int h = 0; h < 2 && 2 + h < kk; ++h) {
+            v0 = 0.0f;
+            const int first = h * half;
+            for (int i = first; i < first + half; ++i) {
+                v0 = add_rn(v0, diag);
+                const int split = i >= first + quarter ? first + quarter : first;
+                run(i, first, split, true);
+                run(i, split, i, false);
+            }
+            EX[(2 + h) * P + c] = fmaxf(v0, 0.0f);
+        }
+    }
+}
+
 // One group, by a whole CTA.
 template <int ND, int B0, int B1, int B2>
 __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char* smem, int64_t gid) {
@@ -1532,14 +1598,12 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         // exact planes g < kk: sum_{i,j} G[g,i] G[g,j] C_c((x_i - x_j) mod domain),
         // C_c the covariance map of spatial coefficient c; the other planes
         // share what is left of n times the patch variance C_c(0)
-        int* lag = sm<int>(smem, a.L.lag);
-        const int npair = n * (n + 1) / 2;
+        int* lag = sm<int>(smem, a.L.lag);  // lag[i * lrow + j]: first element of the pair's map row
+        const int lrow = (n + 3) / 4 * 4;
         if (kk > 0) {
-            for (int q = tid; q < npair; q += blockDim.x) {
-                int i = static_cast<int>((sqrtf(8.0f * static_cast<float>(q) + 1.0f) - 1.0f) * 0.5f);
-                while (i * (i + 1) / 2 > q) --i;
-                while ((i + 1) * (i + 2) / 2 <= q) ++i;
-                const int j = q - i * (i + 1) / 2;
+            for (int q = tid; q < n * n; q += blockDim.x) {
+                const int i = q / n, j = q - i * n;
+                if (j >= i) continue;
                 int flat = 0;
                 for (int d = 0; d < geo.nd(); ++d) {
                     const int D = sp.cov_domain[d];
@@ -1547,32 +1611,36 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
                     if (l < 0) l += D;
                     flat = flat * D + l;
                 }
-                lag[q] = flat;
+                lag[i * lrow + j] = flat * P;
             }
             __syncthreads();
         }
         const float* cm = sp.cov_maps;
-        // one thread per (plane, coefficient): the planes' sums are independent
-        for (int t = tid; t < kk * P; t += blockDim.x) {
-            const int g = t / P, c = t - g * P;
-            const float pv = __ldg(cm + c);  // lag 0: the patch variance of coefficient c
-            const float* Gr = G + g * n;
-            float value = 0.0f;
-            for (int i = 0; i < n; ++i) {
-                const float wi = Gr[i];
-                if (wi == 0.0f) continue;
-                value = add_rn(value, mul_rn(mul_rn(wi, pv), wi));
-                const int* lrow = lag + i * (i + 1) / 2;
-                for (int j = 0; j < i; ++j) {
-                    const float wj = Gr[j];
-                    if (wj == 0.0f) continue;
-                    const float cv = __ldg(cm + static_cast<int64_t>(lrow[j]) * P + c);
-                    value = add_rn(value, mul_rn(mul_rn(wi, wj), add_rn(cv, cv)));
+        if (kk > 0 && sp.group_transform == BMND_GROUP_HAAR && is_pow2(n) && kk <= 4 && 2 * P <= static_cast<int>(blockDim.x)) {
+            gauss_haar(cm, lag, lrow, n, kk, P, G, EX);
+        } else {
+            // one thread per (plane, coefficient): the planes' sums are independent
+            for (int t = tid; t < kk * P; t += blockDim.x) {
+                const int g = t / P, c = t - g * P;
+                const float pv = __ldg(cm + c);  // lag 0: the patch variance of coefficient c
+                const float* Gr = G + g * n;
+                float value = 0.0f;
+                for (int i = 0; i < n; ++i) {
+                    const float wi = Gr[i];
+                    if (wi == 0.0f) continue;
+                    value = add_rn(value, mul_rn(mul_rn(wi, pv), wi));
+                    for (int j = 0; j < i; ++j) {
+                        const float wj = Gr[j];
+                        if (wj == 0.0f) continue;
+                        const float cv = __ldg(cm + lag[i * lrow + j] + c);
+                        value = add_rn(value, mul_rn(mul_rn(wi, wj), add_rn(cv, cv)));
+                    }
                 }
+                EX[g * P + c] = fmaxf(value, 0.0f);
             }
-            EX[g * P + c] = fmaxf(value, 0.0f);
         }
         __syncthreads();
+        // the other planes' standard deviation, parked in X (not gathered yet)
         for (int c = tid; c < P; c += blockDim.x) {
             const float pv = __ldg(cm + c);
             float ex_sum = 0.0f;
@@ -1582,11 +1650,10 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
                 rest = div_rn(sub_rn(mul_rn(static_cast<float>(n), pv), ex_sum), static_cast<float>(n - kk));
                 rest = fmaxf(rest, 0.0f);
             }
-            for (int g = 0; g < n; ++g) {
-                const float v = g < kk ? EX[g * P + c] : rest;
-                S[g * P + c] = sqrtf(fmaxf(v, 0.0f));
-            }
+            X[c] = sqrtf(fmaxf(rest, 0.0f));
         }
+        __syncthreads();
+        for_members(n, P, [&](int g, int c, int e) { S[e] = g < kk ? sqrtf(EX[e]) : X[c]; });
         __syncthreads();
     }
 
