@@ -21,12 +21,17 @@
 //   5. per-patch aggregation weights 1 / (sum_g Ginv[o,g]^2 plane_risk[g] +
 //      eps) (aggregationweights.py:213-259, :616-653), or one weight per group
 //      from its exact windowed-synthesis risk (wiener.py:638-822);
-//   6. inverse transform and weighted Kaiser-window scatter into float64
-//      numerator / denominator volumes (patchaggregation.py:170-199).
+//   6. inverse transform and weighted Kaiser-window scatter: to the members'
+//      store rows, summed in a fixed order afterwards, or by atomics into
+//      float64 numerator / denominator volumes (patchaggregation.py:170-199).
 //
-// The union of overlapping voxels is found with a per-group occupancy grid
-// holding one bit per group member (N <= 32), so each voxel's entries come out
-// in ascending group order and the float32 sums are deterministic.
+// The union of overlapping voxels comes from one member mask per axis and
+// coordinate (N <= 32): a cell's members are the AND of its coordinates' masks,
+// so each voxel's entries come out in ascending group order and the float32 sums
+// are deterministic.
+//
+// What bounds it: the instructions issued (78 % of the issue slots at 16 members
+// of 8x8), half of them in the exact variance's products; memory stays below 10 %.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -40,7 +45,7 @@ constexpr int kMiscWild = 13;      // misc word: the group holds a value of 1e30
 
 // Shared-memory plan.  A fixed part holds the group matrix, the transform
 // tables, positions and small per-group arrays.  The union region first holds
-// the exact-variance phase's occupancy grid and union-voxel lists; once that
+// the exact-variance phase's axis masks and union-voxel lists; once that
 // phase is done it holds the group buffers: S (noise sigma), X (noisy
 // coefficients) and R (pilot coefficients, Wiener) or V (attenuation, hard
 // thresholding).  Transforms run in place, so no scratch buffer is needed.
@@ -77,12 +82,27 @@ struct FilterArgs {
     // group probe: per-group intermediate arrays instead of the aggregation
     GroupProbe probe;
     int64_t n_lins;      // patch-grid positions: a member's lin lies in [0, n_lins)
-    int64_t ucells_cap;  // union-box cells the occupancy grid of the layout holds
+    int64_t ucells_cap;  // union-box cells the layout's lists hold
     AggStore store;      // deterministic aggregation: rows of the entry store, or store.store == null
 };
 
 __host__ __device__ inline bool kron_in_smem(const BmndStageParams& sp, int P, int kmax) {
     return kron_jr(P) == 2 && kmax > 0 && sp.noise_model == BMND_NOISE_POISSON;
+}
+
+// The group buffers (S, X, R, V, SG) of 8x8 patches keep one spare word after
+// every row: the lines of the last axis, 8 words apart, then fall into different
+// banks (8-way conflicts before; with the joint forward sweep below, a 17 K-group
+// final stage of 32 members went from 3.12 to 2.89 ms).  4x4x4 patches conflict
+// 4-way at most and measured the same with and without the padding (3.56 ms), so
+// they have none.  LB is the row length.
+template <int LB>
+__host__ __device__ __forceinline__ constexpr int padded(int p) {
+    return LB == 8 ? p + p / 8 : p;
+}
+__host__ inline int64_t padded_patch(const BmndStageParams& sp, int P) {
+    const int32_t* b = sp.block;
+    return sp.ndim == 2 && b[0] == 8 && b[1] == 8 && !sp.exact_risk_weights ? padded<8>(P) : P;
 }
 
 __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax, int64_t ucells, bool sigma) {
@@ -95,6 +115,7 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
         return o;
     };
     const int64_t np = static_cast<int64_t>(nmax) * P;
+    const int64_t npp = static_cast<int64_t>(nmax) * padded_patch(sp, P);
     const bool wiener = sp.filter == BMND_FILTER_WIENER;
     const int kpad = (kmax + 3) / 4 * 4;
     L.g = take(4 * nmax * nmax);
@@ -117,7 +138,7 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.shf = take(4 * nmax * BMND_MAX_DIMS);
     L.shl = take(4 * nmax);
     // hard thresholding with a sigma map keeps each coefficient's sigma until the scatter
-    L.sg = take(sigma && !wiener ? 4 * np : 16);
+    L.sg = take(sigma && !wiener ? 4 * npp : 16);
     L.ex = take(4 * static_cast<int64_t>(kmax) * P);
 
     // Gaussian noise: covariance-map row of every member pair (i > j)
@@ -130,7 +151,7 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.risk = take(8 * (kThreads / 32 + 1));  // exact risk: per-warp partial sums, then the total
     // union region
     L.uni = off;
-    const int64_t buf = round16(4 * np);
+    const int64_t buf = round16(4 * npp);
     L.s = L.uni;
     L.x = L.s + buf;
     L.r = L.x + buf;  // Wiener: pilot coefficients, then the attenuation
@@ -199,6 +220,18 @@ struct Geom {
         return b_[d];
     }
     __device__ __forceinline__ int P() const { return ND > 0 ? B0 * B1 * B2 : P_; }
+    // group buffers: words per member, and the word of patch element p
+    static constexpr int LB = ND == 0 ? 0 : (ND == 3 ? B2 : (ND == 2 ? B1 : B0));
+    __device__ __forceinline__ int PP() const { return ND > 0 ? padded<LB>(B0 * B1 * B2) : P_; }
+    __device__ __forceinline__ int at(int g, int p) const { return g * PP() + padded<LB>(p); }
+    // f(member, patch element, its word) over an n x P group
+    template <typename F>
+    __device__ __forceinline__ void each(int n, F f) const {
+        for (int e = threadIdx.x; e < n * P(); e += blockDim.x) {
+            const int g = e / P(), p = e - g * P();
+            f(g, p, at(g, p));
+        }
+    }
     // product of the patch extents after axis d
     __device__ __forceinline__ int inner(int d) const {
         int v = 1;
@@ -239,21 +272,23 @@ __device__ __forceinline__ float gmat(const float* G, int N, int i, int k) {
     return KIND == 2 ? mul_rn(m, m) : m;
 }
 
-template <int N, int KIND>
-__device__ void group_axis_inplace(float* buf, int P, const float* G) {
+// (C columns of S words per member, column p at padded<LB>(p))
+template <int N, int KIND, int LB>
+__device__ void group_axis_inplace(float* buf, int C, int S, const float* G) {
     constexpr int IC = N >= 16 ? 8 : N;  // outputs per thread
     constexpr int CH = N / IC;           // threads per column
     // a warp shares one output chunk over 32 consecutive columns: matrix reads
     // are broadcasts, column reads and writes hit consecutive banks
     const int cols = static_cast<int>(blockDim.x) / CH;
-    for (int c0 = 0; c0 < P; c0 += cols) {
-        const int p = c0 + static_cast<int>(threadIdx.x) % cols;
+    for (int c0 = 0; c0 < C; c0 += cols) {
+        const int col = c0 + static_cast<int>(threadIdx.x) % cols;
         const int i0 = (static_cast<int>(threadIdx.x) / cols) * IC;
-        const bool act = static_cast<int>(threadIdx.x) < cols * CH && p < P;
+        const bool act = static_cast<int>(threadIdx.x) < cols * CH && col < C;
+        const int p = padded<LB>(col);
         float x[N];
         if (act) {
 #pragma unroll
-            for (int k = 0; k < N; ++k) x[k] = buf[k * P + p];
+            for (int k = 0; k < N; ++k) x[k] = buf[k * S + p];
         }
         __syncthreads();
         if (act) {
@@ -280,7 +315,7 @@ __device__ void group_axis_inplace(float* buf, int P, const float* G) {
 #pragma unroll
                     for (int k = 0; k < N; ++k) acc = fmaf(gmat<KIND>(G, N, i, k), x[k], acc);
                 }
-                buf[i * P + p] = acc;
+                buf[i * S + p] = acc;
             }
         }
         __syncthreads();
@@ -353,28 +388,89 @@ __device__ __forceinline__ void haar_chunk(const float* buf, int P, int p, const
 }
 
 template <int N, int KIND>
-__device__ void haar_product(float* buf, int P, const float* G) {
+__device__ __forceinline__ void haar_chunk_any(int chunk, const float* buf, int S, int p, const float* G,
+                                               float (&acc)[N >= 16 ? 8 : N]) {
+    constexpr int CH = N / (N >= 16 ? 8 : N);
+    if (CH == 1 || chunk == 0) haar_chunk<N, KIND, 0>(buf, S, p, G, acc);
+    else if (CH == 2 || chunk == 1) haar_chunk<N, KIND, (CH > 1 ? 1 : 0)>(buf, S, p, G, acc);
+    else if (chunk == 2) haar_chunk<N, KIND, (CH > 2 ? 2 : 0)>(buf, S, p, G, acc);
+    else haar_chunk<N, KIND, (CH > 3 ? 3 : 0)>(buf, S, p, G, acc);
+}
+
+template <int N, int KIND, int LB>
+__device__ void haar_product(float* buf, int C, int S, const float* G) {
     constexpr int IC = N >= 16 ? 8 : N;
     constexpr int CH = N / IC;
     const int cols = static_cast<int>(blockDim.x) / CH;
     const int chunk = static_cast<int>(threadIdx.x) / cols;  // the same for a whole warp
-    for (int c0 = 0; c0 < P; c0 += cols) {
-        const int p = c0 + static_cast<int>(threadIdx.x) % cols;
-        const bool act = static_cast<int>(threadIdx.x) < cols * CH && p < P;
+    for (int c0 = 0; c0 < C; c0 += cols) {
+        const int col = c0 + static_cast<int>(threadIdx.x) % cols;
+        const bool act = static_cast<int>(threadIdx.x) < cols * CH && col < C;
+        const int p = padded<LB>(col);
+        float acc[IC];
+        if (act) haar_chunk_any<N, KIND>(chunk, buf, S, p, G, acc);
+        __syncthreads();
+        if (act) {
+#pragma unroll
+            for (int ii = 0; ii < IC; ++ii) buf[(chunk * IC + ii) * S + p] = acc[ii];
+        }
+    }
+    __syncthreads();  // (the columns of one round are not read by the next)
+}
+
+// The forward Haar axis of all the group's buffers in one sweep: s squared (kind
+// 2), x and, unless null, r (kind 0).  Two small buffers (hard thresholding of
+// at most 16 members and 64 columns) are taken by half of the threads each.
+template <int N, int LB>
+__device__ void haar_product_all(float* s, float* x, float* r, int C, int S, const float* G) {
+    constexpr int IC = N >= 16 ? 8 : N;
+    constexpr int CH = N / IC;
+    const int tid = threadIdx.x;
+    if (r == nullptr && CH <= 2 && C <= 64 && blockDim.x == 256) {
+        const bool second = tid >= 128;
+        const int t = tid & 127;
+        constexpr int cols = 128 / (CH <= 2 ? CH : 2);
+        const int chunk = t / cols, col = t % cols;
+        const bool act = col < C;
+        const int p = padded<LB>(col);
         float acc[IC];
         if (act) {
-            if (CH == 1 || chunk == 0) haar_chunk<N, KIND, 0>(buf, P, p, G, acc);
-            else if (CH == 2 || chunk == 1) haar_chunk<N, KIND, (CH > 1 ? 1 : 0)>(buf, P, p, G, acc);
-            else if (chunk == 2) haar_chunk<N, KIND, (CH > 2 ? 2 : 0)>(buf, P, p, G, acc);
-            else haar_chunk<N, KIND, (CH > 3 ? 3 : 0)>(buf, P, p, G, acc);
+            if (second) haar_chunk_any<N, 0>(chunk, x, S, p, G, acc);
+            else haar_chunk_any<N, 2>(chunk, s, S, p, G, acc);
+        }
+        __syncthreads();
+        if (act) {
+            float* buf = second ? x : s;
+#pragma unroll
+            for (int ii = 0; ii < IC; ++ii) buf[(chunk * IC + ii) * S + p] = acc[ii];
+        }
+        __syncthreads();
+        return;
+    }
+    const int cols = static_cast<int>(blockDim.x) / CH;
+    const int chunk = tid / cols;
+    for (int c0 = 0; c0 < C; c0 += cols) {
+        const int col = c0 + tid % cols;
+        const bool act = tid < cols * CH && col < C;
+        const int p = padded<LB>(col);
+        float as[IC], ax[IC], ar[IC];
+        if (act) {
+            haar_chunk_any<N, 2>(chunk, s, S, p, G, as);
+            haar_chunk_any<N, 0>(chunk, x, S, p, G, ax);
+            if (r) haar_chunk_any<N, 0>(chunk, r, S, p, G, ar);
         }
         __syncthreads();
         if (act) {
 #pragma unroll
-            for (int ii = 0; ii < IC; ++ii) buf[(chunk * IC + ii) * P + p] = acc[ii];
+            for (int ii = 0; ii < IC; ++ii) {
+                const int e = (chunk * IC + ii) * S + p;
+                s[e] = as[ii];
+                x[e] = ax[ii];
+                if (r) r[e] = ar[ii];
+            }
         }
-        __syncthreads();
     }
+    __syncthreads();
 }
 
 // Haar group axis by its sum pyramid (one thread per column, O(N) operations):
@@ -426,139 +522,200 @@ __device__ __forceinline__ void haar_column(float* buf, int p, int P) {
     }
 }
 
-template <int N, int KIND>
-__device__ void haar_axis_fast(float* buf, int P) {
-    for (int p = static_cast<int>(threadIdx.x); p < P; p += blockDim.x) haar_column<N, KIND>(buf, p, P);
+template <int N, int KIND, int LB>
+__device__ void haar_axis_fast(float* buf, int C, int S) {
+    for (int c = static_cast<int>(threadIdx.x); c < C; c += blockDim.x) haar_column<N, KIND>(buf, padded<LB>(c), S);
     __syncthreads();
 }
 
 // the forward Haar group axis of three groups in one sweep: s squared (kind
 // 2), x and r (kind 0; r may be null)
-template <int N>
-__device__ void haar_axis_fast3(float* s, float* x, float* r, int P) {
-    for (int p = static_cast<int>(threadIdx.x); p < P; p += blockDim.x) {
-        haar_column<N, 2>(s, p, P);
-        haar_column<N, 0>(x, p, P);
-        if (r) haar_column<N, 0>(r, p, P);
+template <int N, int LB>
+__device__ void haar_axis_fast3(float* s, float* x, float* r, int C, int S) {
+    for (int c = static_cast<int>(threadIdx.x); c < C; c += blockDim.x) {
+        const int p = padded<LB>(c);
+        haar_column<N, 2>(s, p, S);
+        haar_column<N, 0>(x, p, S);
+        if (r) haar_column<N, 0>(r, p, S);
     }
     __syncthreads();
 }
 
-__device__ bool haar_axis_any3(float* s, float* x, float* r, int n, int P) {
+template <int LB>
+__device__ bool haar_axis_any3(float* s, float* x, float* r, int n, int C, int S) {
     switch (n) {
-        case 2: haar_axis_fast3<2>(s, x, r, P); return true;
-        case 4: haar_axis_fast3<4>(s, x, r, P); return true;
-        case 8: haar_axis_fast3<8>(s, x, r, P); return true;
-        case 16: haar_axis_fast3<16>(s, x, r, P); return true;
-        case 32: haar_axis_fast3<32>(s, x, r, P); return true;
+        case 2: haar_axis_fast3<2, LB>(s, x, r, C, S); return true;
+        case 4: haar_axis_fast3<4, LB>(s, x, r, C, S); return true;
+        case 8: haar_axis_fast3<8, LB>(s, x, r, C, S); return true;
+        case 16: haar_axis_fast3<16, LB>(s, x, r, C, S); return true;
+        case 32: haar_axis_fast3<32, LB>(s, x, r, C, S); return true;
         default: return false;
     }
 }
 
-template <int KIND>
-__device__ bool haar_axis_any(float* buf, int n, int P) {
+template <int KIND, int LB>
+__device__ bool haar_axis_any(float* buf, int n, int C, int S) {
     switch (n) {
-        case 2: haar_axis_fast<2, KIND>(buf, P); return true;
-        case 4: haar_axis_fast<4, KIND>(buf, P); return true;
-        case 8: haar_axis_fast<8, KIND>(buf, P); return true;
-        case 16: haar_axis_fast<16, KIND>(buf, P); return true;
-        case 32: haar_axis_fast<32, KIND>(buf, P); return true;
+        case 2: haar_axis_fast<2, KIND, LB>(buf, C, S); return true;
+        case 4: haar_axis_fast<4, KIND, LB>(buf, C, S); return true;
+        case 8: haar_axis_fast<8, KIND, LB>(buf, C, S); return true;
+        case 16: haar_axis_fast<16, KIND, LB>(buf, C, S); return true;
+        case 32: haar_axis_fast<32, KIND, LB>(buf, C, S); return true;
         default: return false;
     }
 }
 
 // runtime group size (not a power of two): one thread per column
-template <int KIND>
-__device__ void group_axis_generic(float* buf, int n, int P, const float* G) {
-    for (int p = static_cast<int>(threadIdx.x); p < P; p += blockDim.x) {
+template <int KIND, int LB>
+__device__ void group_axis_generic(float* buf, int n, int C, int S, const float* G) {
+    for (int c = static_cast<int>(threadIdx.x); c < C; c += blockDim.x) {
+        const int p = padded<LB>(c);
         float x[BMND_MAX_STACK];
-        for (int k = 0; k < n; ++k) x[k] = buf[k * P + p];
+        for (int k = 0; k < n; ++k) x[k] = buf[k * S + p];
         for (int i = 0; i < n; ++i) {
             float acc = 0.0f;
             for (int k = 0; k < n; ++k) acc = fmaf(gmat<KIND>(G, n, i, k), x[k], acc);
-            buf[i * P + p] = acc;
+            buf[i * S + p] = acc;
         }
     }
     __syncthreads();
 }
 
 // `sparse`: G is the Haar matrix and every value is finite
-template <int KIND>
-__device__ void group_axis_any(float* buf, int n, int P, const float* G, bool sparse) {
+template <int KIND, int LB>
+__device__ void group_axis_any(float* buf, int n, int C, int S, const float* G, bool sparse) {
     if (sparse) {
         switch (n) {
-            case 2: haar_product<2, KIND>(buf, P, G); return;
-            case 4: haar_product<4, KIND>(buf, P, G); return;
-            case 8: haar_product<8, KIND>(buf, P, G); return;
-            case 16: haar_product<16, KIND>(buf, P, G); return;
-            case 32: haar_product<32, KIND>(buf, P, G); return;
+            case 2: haar_product<2, KIND, LB>(buf, C, S, G); return;
+            case 4: haar_product<4, KIND, LB>(buf, C, S, G); return;
+            case 8: haar_product<8, KIND, LB>(buf, C, S, G); return;
+            case 16: haar_product<16, KIND, LB>(buf, C, S, G); return;
+            case 32: haar_product<32, KIND, LB>(buf, C, S, G); return;
             default: break;
         }
     }
     switch (n) {
-        case 1: group_axis_inplace<1, KIND>(buf, P, G); break;
-        case 2: group_axis_inplace<2, KIND>(buf, P, G); break;
-        case 4: group_axis_inplace<4, KIND>(buf, P, G); break;
-        case 8: group_axis_inplace<8, KIND>(buf, P, G); break;
-        case 16: group_axis_inplace<16, KIND>(buf, P, G); break;
-        case 32: group_axis_inplace<32, KIND>(buf, P, G); break;
-        default: group_axis_generic<KIND>(buf, n, P, G); break;
+        case 1: group_axis_inplace<1, KIND, LB>(buf, C, S, G); break;
+        case 2: group_axis_inplace<2, KIND, LB>(buf, C, S, G); break;
+        case 4: group_axis_inplace<4, KIND, LB>(buf, C, S, G); break;
+        case 8: group_axis_inplace<8, KIND, LB>(buf, C, S, G); break;
+        case 16: group_axis_inplace<16, KIND, LB>(buf, C, S, G); break;
+        case 32: group_axis_inplace<32, KIND, LB>(buf, C, S, G); break;
+        default: group_axis_generic<KIND, LB>(buf, n, C, S, G); break;
     }
 }
 
-// patch axis d with compile-time edge B and stride INNER: each thread
+// patch axis d with compile-time edge B and INNER elements after it: each thread
 // transforms whole lines of B values (matrix in registers), so lines never
-// share a thread and the product overwrites its input
-template <int B, int INNER>
+// share a thread and the product overwrites its input.  line_base and kStep are
+// a line's first word and its element stride in the padded buffers.
+template <int B, int STEP>
 __device__ __forceinline__ void space_line(float* buf, int base, const float (&m)[B * B]) {
     float x[B];
 #pragma unroll
-    for (int k = 0; k < B; ++k) x[k] = buf[base + k * INNER];
+    for (int k = 0; k < B; ++k) x[k] = buf[base + k * STEP];
 #pragma unroll
     for (int i = 0; i < B; ++i) {
         float acc = 0.0f;
 #pragma unroll
         for (int k = 0; k < B; ++k) acc = fmaf(m[i * B + k], x[k], acc);
-        buf[base + i * INNER] = acc;
+        buf[base + i * STEP] = acc;
     }
 }
 
-template <int B, int INNER>
-__device__ void space_axis_reg(float* buf, int total, const float* Msrc, bool square) {
-    float m[B * B];
-#pragma unroll
-    for (int q = 0; q < B * B; ++q) {
-        const float v = Msrc[q];
-        m[q] = square ? mul_rn(v, v) : v;
-    }
-    const int lines = total / B;
-    for (int line = static_cast<int>(threadIdx.x); line < lines; line += blockDim.x) {
+template <int B, int INNER, int LB>
+struct Lines {
+    static constexpr int kStep = INNER == 1 ? 1 : padded<LB>(INNER);
+    __device__ static __forceinline__ int base(int line) {
         const int o = line / INNER;
         const int t = line - o * INNER;
-        space_line<B, INNER>(buf, o * B * INNER + t, m);
+        return INNER == 1 ? padded<LB>(o * B) : o * B * kStep + padded<LB>(t);
+    }
+};
+
+// Edge 8: two threads of a warp (lanes l and l + 16) share a line, four outputs
+// each, so that a half of the matrix, 32 registers instead of 64, stays in a
+// thread and 16 members keep all warps of the block busy.
+template <int INNER, int LB>
+__device__ __forceinline__ void space_axis_half(float* buf, int lines, const float (&m)[32]) {
+    using L = Lines<8, INNER, LB>;
+    const int lane = threadIdx.x & 31, h = lane >> 4;
+    for (int l0 = 0; l0 < lines; l0 += blockDim.x >> 1) {
+        const int line = l0 + (static_cast<int>(threadIdx.x) >> 5) * 16 + (lane & 15);
+        const int base = L::base(line);
+        float x[8];
+        if (line < lines) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = buf[base + k * L::kStep];
+        }
+        __syncwarp();
+        if (line < lines) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float acc = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) acc = fmaf(m[i * 8 + k], x[k], acc);
+                buf[base + (h * 4 + i) * L::kStep] = acc;
+            }
+        }
+    }
+}
+
+// one axis of one buffer (`square`: by the squared matrix) ...
+template <int B, int INNER, int LB>
+__device__ void space_axis_reg(float* buf, int lines, const float* Msrc, bool square) {
+    constexpr int kRows = B == 8 ? 4 : B;
+    const int row0 = B == 8 ? (threadIdx.x >> 4 & 1) * 4 : 0;
+    float m[kRows * B];
+#pragma unroll
+    for (int q = 0; q < kRows * B; ++q) {
+        const float v = Msrc[row0 * B + q];
+        m[q] = square ? mul_rn(v, v) : v;
+    }
+    if constexpr (B == 8) {
+        space_axis_half<INNER, LB>(buf, lines, m);
+    } else {
+        using L = Lines<B, INNER, LB>;
+        for (int line = threadIdx.x; line < lines; line += blockDim.x)
+            space_line<B, L::kStep>(buf, L::base(line), m);
     }
     __syncthreads();
 }
 
-// the same axis of three groups in one sweep: s with the squared matrix, x and
-// r (may be null) with the matrix itself
-template <int B, int INNER>
-__device__ void space_axis_reg3(float* s, float* x, float* r, int total, const float* Msrc) {
-    float m[B * B], m2[B * B];
+// ... and of all the group's buffers in one sweep: s by the squared matrix, x and
+// r (may be null) by the matrix itself; up to 128 lines of two buffers are taken
+// by half of the threads each
+template <int B, int INNER, int LB>
+__device__ void space_axis_reg_all(float* s, float* x, float* r, int lines, const float* Msrc) {
+    const int tid = threadIdx.x;
+    constexpr int kRows = B == 8 ? 4 : B;
+    const int row0 = B == 8 ? (tid >> 4 & 1) * 4 : 0;
+    float m[kRows * B];
 #pragma unroll
-    for (int q = 0; q < B * B; ++q) {
-        const float v = Msrc[q];
-        m[q] = v;
-        m2[q] = mul_rn(v, v);
-    }
-    const int lines = total / B;
-    for (int line = static_cast<int>(threadIdx.x); line < lines; line += blockDim.x) {
-        const int o = line / INNER;
-        const int t = line - o * INNER;
-        const int base = o * B * INNER + t;
-        space_line<B, INNER>(s, base, m2);
-        space_line<B, INNER>(x, base, m);
-        if (r) space_line<B, INNER>(r, base, m);
+    for (int q = 0; q < kRows * B; ++q) m[q] = Msrc[row0 * B + q];
+    if constexpr (B == 8) {
+        space_axis_half<INNER, LB>(x, lines, m);
+        if (r) space_axis_half<INNER, LB>(r, lines, m);
+#pragma unroll
+        for (int q = 0; q < kRows * B; ++q) m[q] = mul_rn(m[q], m[q]);
+        space_axis_half<INNER, LB>(s, lines, m);
+    } else {
+        using L = Lines<B, INNER, LB>;
+        const int half = blockDim.x >> 1;
+        const bool split = r == nullptr && lines <= half;
+        const int step = split ? half : static_cast<int>(blockDim.x);
+        if (!split || tid >= half) {
+            for (int line = split ? tid - half : tid; line < lines; line += step) {
+                const int base = L::base(line);
+                space_line<B, L::kStep>(x, base, m);
+                if (r) space_line<B, L::kStep>(r, base, m);
+            }
+        }
+        if (!split || tid < half) {
+#pragma unroll
+            for (int q = 0; q < B * B; ++q) m[q] = mul_rn(m[q], m[q]);
+            for (int line = tid; line < lines; line += step) space_line<B, L::kStep>(s, L::base(line), m);
+        }
     }
     __syncthreads();
 }
@@ -589,17 +746,22 @@ __device__ void space_axis_generic(const GM& geo, int d, float* buf, int n, cons
 }
 
 template <int ND, int B0, int B1, int B2, int D>
+struct Axis {
+    static constexpr int B = D == 0 ? B0 : (D == 1 ? B1 : B2);
+    static constexpr int INNER = D == 0 ? (ND > 1 ? B1 : 1) * (ND > 2 ? B2 : 1) : (D == 1 ? (ND > 2 ? B2 : 1) : 1);
+    static constexpr int LB = ND == 3 ? B2 : (ND == 2 ? B1 : B0);
+    static constexpr int kLines = B0 * B1 * B2 / B;
+};
+template <int ND, int B0, int B1, int B2, int D>
 __device__ __forceinline__ void space_axis_fixed(float* buf, int n, const float* M, bool square) {
-    constexpr int B = D == 0 ? B0 : (D == 1 ? B1 : B2);
-    constexpr int INNER = D == 0 ? (ND > 1 ? B1 : 1) * (ND > 2 ? B2 : 1) : (D == 1 ? (ND > 2 ? B2 : 1) : 1);
-    space_axis_reg<B, INNER>(buf, n * B0 * B1 * B2, M, square);
+    using A = Axis<ND, B0, B1, B2, D>;
+    space_axis_reg<A::B, A::INNER, A::LB>(buf, n * A::kLines, M, square);
 }
 
 template <int ND, int B0, int B1, int B2, int D>
-__device__ __forceinline__ void space_axis_fixed3(float* s, float* x, float* r, int n, const float* M) {
-    constexpr int B = D == 0 ? B0 : (D == 1 ? B1 : B2);
-    constexpr int INNER = D == 0 ? (ND > 1 ? B1 : 1) * (ND > 2 ? B2 : 1) : (D == 1 ? (ND > 2 ? B2 : 1) : 1);
-    space_axis_reg3<B, INNER>(s, x, r, n * B0 * B1 * B2, M);
+__device__ __forceinline__ void space_axis_fixed_all(float* s, float* x, float* r, int n, const float* M) {
+    using A = Axis<ND, B0, B1, B2, D>;
+    space_axis_reg_all<A::B, A::INNER, A::LB>(s, x, r, n * A::kLines, M);
 }
 
 // separable transform of an (n, block...) group in place: the group axis
@@ -611,18 +773,18 @@ __device__ void transform_group(const GM& geo, const FilterArgs& a, unsigned cha
     const float* G = sm<float>(smem, a.L.g);
     const float* F = sm<float>(smem, kind == 1 ? a.L.fi : (kind == 3 ? a.L.fit : a.L.fw));
     const bool fast_haar = a.sp.fast_group_transform && a.sp.group_transform == BMND_GROUP_HAAR &&
-                           (kind == 0 ? haar_axis_any<0>(buf, n, geo.P())
-                                      : kind == 1 ? haar_axis_any<1>(buf, n, geo.P())
-                                                  : kind == 2 ? haar_axis_any<2>(buf, n, geo.P())
-                                                              : haar_axis_any<0>(buf, n, geo.P()));
+                           (kind == 0 ? haar_axis_any<0, GM::LB>(buf, n, geo.P(), geo.PP())
+                                      : kind == 1 ? haar_axis_any<1, GM::LB>(buf, n, geo.P(), geo.PP())
+                                                  : kind == 2 ? haar_axis_any<2, GM::LB>(buf, n, geo.P(), geo.PP())
+                                                              : haar_axis_any<0, GM::LB>(buf, n, geo.P(), geo.PP()));
     if (!fast_haar && a.sp.group_transform != BMND_GROUP_NONE) {
         // kind 3 (transposed inverse): the group transforms are orthonormal, so
         // the transposed inverse of the group axis is the forward transform
         const bool sparse = a.sp.group_transform == BMND_GROUP_HAAR && kind != 3 && !a.den_ro &&
                             sm<int>(smem, a.L.misc)[kMiscWild] == 0;
-        if (kind == 0 || kind == 3) group_axis_any<0>(buf, n, geo.P(), G, sparse);
-        else if (kind == 1) group_axis_any<1>(buf, n, geo.P(), G, sparse);
-        else group_axis_any<2>(buf, n, geo.P(), G, sparse);
+        if (kind == 0 || kind == 3) group_axis_any<0, GM::LB>(buf, n, geo.P(), geo.PP(), G, sparse);
+        else if (kind == 1) group_axis_any<1, GM::LB>(buf, n, geo.P(), geo.PP(), G, sparse);
+        else group_axis_any<2, GM::LB>(buf, n, geo.P(), geo.PP(), G, sparse);
     }
     const bool square = kind == 2;
     if constexpr (ND > 0) {
@@ -636,25 +798,39 @@ __device__ void transform_group(const GM& geo, const FilterArgs& a, unsigned cha
     }
 }
 
-// The three forward transforms of the approximate path in one sweep of passes:
-// the variance group S squared (kind 2), the observation X and the pilot R
-// (kind 0, R may be null).  Only for compile-time patches with the Haar group
-// axis by its pyramid and a power-of-two group; returns false, having done
-// nothing, otherwise.  Every element goes through the same operations as in
+// The forward transforms of all the group's buffers in one sweep of passes: the
+// variance group S squared (kind 2), the observation X and the pilot R (kind 0,
+// R may be null): a barrier per pass instead of one per pass and buffer.  Only
+// for compile-time patches and Haar groups of a power of two (by the pyramid or
+// by the matrix without its zeros); returns false, having done nothing,
+// otherwise.  Every element goes through the same operations as in
 // transform_group, so the results are the same bits.
 template <int ND, int B0, int B1, int B2, class GM>
-__device__ bool transform_forward3(const GM& geo, const FilterArgs& a, unsigned char* smem, int n, float* S,
-                                   float* X, float* R) {
+__device__ bool transform_forward_all(const GM& geo, const FilterArgs& a, unsigned char* smem, int n, float* S,
+                                      float* X, float* R) {
     if constexpr (ND == 0) {
         return false;
     } else {
-        if (!(a.sp.fast_group_transform && a.sp.group_transform == BMND_GROUP_HAAR)) return false;
-        if (!haar_axis_any3(S, X, R, n, geo.P())) return false;
+        if (a.sp.group_transform != BMND_GROUP_HAAR || !is_pow2(n) || n < 2) return false;
+        const float* G = sm<float>(smem, a.L.g);
+        if (a.sp.fast_group_transform) {
+            if (!haar_axis_any3<GM::LB>(S, X, R, n, geo.P(), geo.PP())) return false;
+        } else {
+            if (a.den_ro || sm<int>(smem, a.L.misc)[kMiscWild] != 0) return false;
+            switch (n) {
+                case 2: haar_product_all<2, GM::LB>(S, X, R, geo.P(), geo.PP(), G); break;
+                case 4: haar_product_all<4, GM::LB>(S, X, R, geo.P(), geo.PP(), G); break;
+                case 8: haar_product_all<8, GM::LB>(S, X, R, geo.P(), geo.PP(), G); break;
+                case 16: haar_product_all<16, GM::LB>(S, X, R, geo.P(), geo.PP(), G); break;
+                case 32: haar_product_all<32, GM::LB>(S, X, R, geo.P(), geo.PP(), G); break;
+                default: return false;
+            }
+        }
         const float* F = sm<float>(smem, a.L.fw);
-        space_axis_fixed3<ND, B0, B1, B2, 0>(S, X, R, n, F);
-        if constexpr (ND > 1) space_axis_fixed3<ND, B0, B1, B2, 1>(S, X, R, n, F + BMND_MAX_EDGE * BMND_MAX_EDGE);
+        space_axis_fixed_all<ND, B0, B1, B2, 0>(S, X, R, n, F);
+        if constexpr (ND > 1) space_axis_fixed_all<ND, B0, B1, B2, 1>(S, X, R, n, F + BMND_MAX_EDGE * BMND_MAX_EDGE);
         if constexpr (ND > 2)
-            space_axis_fixed3<ND, B0, B1, B2, 2>(S, X, R, n, F + 2 * BMND_MAX_EDGE * BMND_MAX_EDGE);
+            space_axis_fixed_all<ND, B0, B1, B2, 2>(S, X, R, n, F + 2 * BMND_MAX_EDGE * BMND_MAX_EDGE);
         return true;
     }
 }
@@ -1344,14 +1520,6 @@ __device__ void exact_risk_any(const unsigned char* smem, const float* __restric
     else exact_risk<JR, 4>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
 }
 
-// f(member, patch element, index) over an n x P group: a warp takes whole rows
-template <typename F>
-__device__ __forceinline__ void for_members(int n, int P, F f) {
-    const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31, nw = blockDim.x >> 5;
-    for (int g = warp; g < n; g += nw)
-        for (int p = lane; p < P; p += 32) f(g, p, g * P + p);
-}
-
 // Exact Gaussian variances of planes 0 .. 3 of a Haar group (kk of them): with
 // plane magnitudes a (planes 0, 1) and b (2, 3), every product of the pair sums
 //   sum_i w_i C(0) w_i + sum_{j < i} (w_i w_j) 2 C(lag_ij)
@@ -1583,8 +1751,8 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     const bool gauss = sp.noise_model == BMND_NOISE_GAUSSIAN;
     const bool exact_risk = sp.exact_risk_weights != 0 && kk > 0;
     if ((!gauss || exact_risk) && kk > 0) {
-        // the exact phase's occupancy grid covers a union box of at most
-        // ucells_cap cells: members within the search window of their reference
+        // the exact phase's lists cover a union box of at most ucells_cap
+        // cells: members within the search window of their reference
         // always fit; a group spread wider is skipped and reported
         int64_t uc = 1;
         for (int d = 0; d < geo.nd(); ++d) uc *= misc[4 + d];
@@ -1653,7 +1821,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             X[c] = sqrtf(fmaxf(rest, 0.0f));
         }
         __syncthreads();
-        for_members(n, P, [&](int g, int c, int e) { S[e] = g < kk ? sqrtf(EX[e]) : X[c]; });
+        geo.each(n, [&](int g, int c, int e) { S[e] = g < kk ? sqrtf(EX[g * P + c]) : X[c]; });
         __syncthreads();
     }
 
@@ -1818,7 +1986,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     bool gathered = false, wild = false;
     bool fused = false;  // X and R already forward-transformed with S
     if (!gauss && need_approx) {
-        for_members(n, P, [&](int g, int p, int e) {
+        geo.each(n, [&](int g, int p, int e) {
             const int off = org0[g] + voff[p];
             const float vs = __ldg(varsrc + off);
             const float vv = variance_of(vs, scale_f, floor_f);
@@ -1832,12 +2000,12 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         if (wild) misc[kMiscWild] = 1;
         gathered = true;
         __syncthreads();
-        fused = transform_forward3<ND, B0, B1, B2>(geo, a, smem, n, S, X, wiener ? R : nullptr);
+        fused = transform_forward_all<ND, B0, B1, B2>(geo, a, smem, n, S, X, wiener ? R : nullptr);
         if (!fused) transform_group<ND, B0, B1, B2>(geo, a, smem, n, S, 2);
-        for (int e = tid; e < total; e += blockDim.x) {
+        geo.each(n, [&](int, int, int e) {
             const float v = S[e];
             S[e] = sqrtf(v > 0.0f ? v : 0.0f);
-        }
+        });
         __syncthreads();
     }
 
@@ -1845,7 +2013,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     if (gauss) {
         // done above
     } else if (k > 0 && kk == n) {
-        for (int e = tid; e < total; e += blockDim.x) S[e] = EX[e];
+        geo.each(n, [&](int g, int p, int e) { S[e] = EX[g * P + p]; });
     } else if (k > 0) {
         // TPJ threads per coefficient j (neighbouring lanes), each summing the
         // planes i = sub (mod TPJ); the partial sums are added by shuffles in
@@ -1858,7 +2026,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             float sum_a = 0.0f, sum_e = 0.0f, rem_a = 0.0f;
             if (live) {
                 for (int i = sub; i < n; i += TPJ) {
-                    const float sa = fmaxf(S[i * P + j], 0.0f);
+                    const float sa = fmaxf(S[geo.at(i, j)], 0.0f);
                     const float va = mul_rn(sa, sa);
                     sum_a = add_rn(sum_a, va);
                     if (i >= kk) rem_a = add_rn(rem_a, va);
@@ -1883,12 +2051,12 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
                     const float se = fmaxf(EX[i * P + j], 0.0f);
                     v = mul_rn(se, se);
                 } else if (rem_a > 0.0f) {
-                    const float sa = fmaxf(S[i * P + j], 0.0f);
+                    const float sa = fmaxf(S[geo.at(i, j)], 0.0f);
                     v = mul_rn(mul_rn(sa, sa), scl);
                 } else {
                     v = div_rn(target, static_cast<float>(n - kk));
                 }
-                S[i * P + j] = sqrtf(v > 0.0f ? v : 0.0f);
+                S[geo.at(i, j)] = sqrtf(v > 0.0f ? v : 0.0f);
             }
         }
     }
@@ -1896,7 +2064,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
 
     // ---- gather and forward-transform the observation (and the pilot) ----
     if (!gathered) {
-        for_members(n, P, [&](int g, int p, int e) {
+        geo.each(n, [&](int g, int p, int e) {
             const int off = org0[g] + voff[p];
             const float xv = __ldg(a.noisy + off);
             const float rv = wiener ? __ldg(a.pilot + off) : 0.0f;
@@ -1913,10 +2081,10 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     }
     const int64_t probe_base = gid * static_cast<int64_t>(a.nmax) * P;
     if (a.probe.active) {
-        for (int e = tid; e < total; e += blockDim.x) {
-            if (a.probe.coef) a.probe.coef[probe_base + e] = X[e];
-            if (a.probe.sigma) a.probe.sigma[probe_base + e] = S[e];
-        }
+        geo.each(n, [&](int g, int p, int e) {
+            if (a.probe.coef) a.probe.coef[probe_base + g * P + p] = X[e];
+            if (a.probe.sigma) a.probe.sigma[probe_base + g * P + p] = S[e];
+        });
     }
 
     // ---- shrinkage: coefficients in X, attenuation in V, and in S each
@@ -1925,7 +2093,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     const float eps_f = static_cast<float>(sp.eps);
     float* SG = sm<float>(smem, a.L.sg);
     float sig_sum = 0.0f;  // Wiener sigma map: this thread's share of the group's sigma sum
-    for (int e = tid; e < total; e += blockDim.x) {
+    geo.each(n, [&](int g, int p, int e) {
         float sig = S[e];
         if (a.sig_num) {
             if (wiener) sig_sum += sig;
@@ -1943,12 +2111,12 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             X[e] = copysignf(shr, X[e]);
             V[e] = att;
             S[e] = sp.weight_model == BMND_WEIGHT_CLASSIC ? att * att : att * att * nv;
-            if (exact_risk && e < kk * P) S[e] = 0.0f;  // the exact pass below holds these planes' noise
-            continue;
+            if (exact_risk && g < kk) S[e] = 0.0f;  // the exact pass below holds these planes' noise
+            return;
         } else if (!wiener && gauss) {
             // |c| >= lambda sigma, the group DC always kept (bmndalgo.py:462-475)
             float thr = mul_rn(sp.ht_lambda, sig);
-            att = (fabsf(X[e]) >= thr || e == 0) ? 1.0f : 0.0f;
+            att = (fabsf(X[e]) >= thr || (g == 0 && p == 0)) ? 1.0f : 0.0f;
         } else if (!wiener) {
             float thr = mul_rn(sp.ht_lambda, sig);
             att = ht_keep(fabsf(X[e]), thr, sp.count_scale, scale_f) ? 1.0f : 0.0f;
@@ -1981,13 +2149,13 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         if (sp.weight_model != BMND_WEIGHT_CLASSIC) err *= nv;
         // exact risk weights: the noise of the first kk planes comes from the
         // exact pass below; their bias term stays (wiener.py:760-797)
-        if (exact_risk && e < kk * P) err = 0.0f;
+        if (exact_risk && g < kk) err = 0.0f;
         if (sp.weight_model == BMND_WEIGHT_RISK) {
             const float rj = 1.0f - att;
             err += rj * rj * spw;
         }
         S[e] = err;
-    }
+    });
     __syncthreads();
 
     // ---- exact noise risk of the first kk planes (wiener.py:638-711) ----
@@ -2005,7 +2173,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     }
 
     if (a.probe.active && a.probe.atten)
-        for (int e = tid; e < total; e += blockDim.x) a.probe.atten[probe_base + e] = V[e];
+        geo.each(n, [&](int g, int p, int e) { a.probe.atten[probe_base + g * P + p] = V[e]; });
 
     // Wiener sigma map: the group's mean coefficient sigma (bmndalgo.py:874-875),
     // summed per warp and then over warps in warp order
@@ -2033,7 +2201,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         for (int g = warp; g < n; g += nwarps) {
             float risk = 0.0f;
             for (int j = lane; j < P; j += 32) {
-                float err = S[g * P + j];
+                float err = S[geo.at(g, j)];
                 if (sp.windowed_synthesis) err *= static_cast<float>(mdiag[j]);
                 risk += err;
             }
@@ -2086,13 +2254,12 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         // output functional O = w_g win[p] / den (float32 arithmetic, as the
         // reference's gather), into S; the target sum(O x noisy) in float64
         double t_target = 0.0;
-        for (int e = tid; e < total; e += blockDim.x) {
-            const int g = e / P, p = e - g * P;
+        geo.each(n, [&](int g, int p, int e) {
             const int64_t off = geo.offset(pos + g * BMND_MAX_DIMS, p, a.vstride);
             const float o = (wts[g] * win[p]) / static_cast<float>(a.den_ro[off]);
             S[e] = o;
             t_target += static_cast<double>(o) * static_cast<double>(__ldg(a.noisy + off));
-        }
+        });
         __syncthreads();
         transform_group<ND, B0, B1, B2>(geo, a, smem, n, S, 3);  // coefficient functional F
         __syncthreads();
@@ -2104,9 +2271,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             dmax_s *= m;
         }
         const float dmax = dmax_g * dmax_s;
-        auto dir_of = [&](int e) -> float {
-            const int g = e / P;
-            int p = e - g * P;
+        auto dir_of = [&](int g, int p) -> float {
             float v = dirv[g];
 #pragma unroll
             for (int d = BMND_MAX_DIMS - 1; d >= 0; --d) {
@@ -2119,13 +2284,13 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         };
         double t_cur = 0.0, t_den = 0.0, t_resp = 0.0;
         float t_max = 0.0f;
-        for (int e = tid; e < total; e += blockDim.x) {
+        geo.each(n, [&](int g, int p, int e) {
             const double f = static_cast<double>(S[e]);
             t_cur += f * static_cast<double>(X[e]);
             t_den += f * f;
-            t_resp += f * static_cast<double>(dir_of(e));
+            t_resp += f * static_cast<double>(dir_of(g, p));
             t_max = fmaxf(t_max, fabsf(S[e]));
-        }
+        });
         const int warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -2175,8 +2340,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         __syncthreads();
         const double corr = red[0];
         if (corr != 0.0)
-            for (int e = tid; e < total; e += blockDim.x)
-                X[e] = static_cast<float>(static_cast<double>(X[e]) + corr * static_cast<double>(dir_of(e)));
+            geo.each(n, [&](int g, int p, int e) {
+                X[e] = static_cast<float>(static_cast<double>(X[e]) + corr * static_cast<double>(dir_of(g, p)));
+            });
         __syncthreads();
     }
 
@@ -2185,7 +2351,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     if (a.probe.active) {
         if (a.probe.weights && tid < n) a.probe.weights[gid * static_cast<int64_t>(a.nmax) + tid] = wts[tid];
         if (a.probe.filt)
-            for (int e = tid; e < total; e += blockDim.x) a.probe.filt[probe_base + e] = X[e];
+            geo.each(n, [&](int g, int p, int e) { a.probe.filt[probe_base + g * P + p] = X[e]; });
         return;
     }
     if (a.store.store) {
@@ -2198,18 +2364,16 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             a.store.wstore[s] = wts[tid];
         }
         __syncthreads();
-        for_members(n, P, [&](int g, int p, int e) {
+        geo.each(n, [&](int g, int p, int e) {
             a.store.store[static_cast<int64_t>(slot[g]) * a.store.row + p] = mul_rn(X[e], mul_rn(wts[g], win[p]));
         });
         return;
     }
-    for (int e = tid; e < total; e += blockDim.x) {
-        const int g = e / P;
-        const int p = e - g * P;
+    geo.each(n, [&](int g, int p, int e) {
         const int64_t off = geo.offset(pos + g * BMND_MAX_DIMS, p, a.vstride);
         float ww = mul_rn(wts[g], win[p]);
         atomicAdd(a.num + off, widen_f64(mul_rn(X[e], ww)));
-        if (a.den_ro) continue;  // the re-aggregation pass adds to the numerator only
+        if (a.den_ro) return;  // the re-aggregation pass adds to the numerator only
         atomicAdd(a.den + off, widen_f64(ww));
         if (a.sig_num) {
             // sigma map numerator (patchaggregation.py:229-294): per coefficient
@@ -2217,13 +2381,19 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             const float sv = wiener ? sm<float>(smem, a.L.misc)[12] : SG[e];
             atomicAdd(a.sig_num + off, widen_f64(mul_rn(sv, ww)));
         }
-    }
+    });
 }
 
 // One CTA per group.  (Persistent CTAs walking the groups, which would set up the
 // constants once, spill: the compiler then keeps 1.9 KB of local memory a thread.)
+// Resident CTAs per SM cover each other's barriers and serial phases: 64
+// registers and 38 KB (16 members) or 56 KB (32) allow four for patches of 64
+// elements (against three: 75.1 -> 72.3 ms for 0.93 M groups of 8x8, 3.56 -> 3.38
+// ms for 42 K groups of 4x4x4, 14.3 -> 12.6 ms for a Gaussian image); 5x5x5
+// patches hold three.
 template <int ND, int B0, int B1, int B2, int NT>
-__global__ void __launch_bounds__(NT, NT == kThreads ? (ND >= 2 ? 3 : 2) : 1) group_filter_kernel(FilterArgs a) {
+__global__ void __launch_bounds__(NT, NT != kThreads ? 1 : ND == 2 || B0 == 4 ? 4 : ND == 3 ? 3 : 2)
+    group_filter_kernel(FilterArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     filter_group<ND, B0, B1, B2>(a, smem, blockIdx.x);
 }
@@ -2415,9 +2585,6 @@ int32_t launch_group_filter(const BmndStageParams& sp, const float* noisy, const
         BMND_LAUNCH_CHECK("group_filter_kernel");
         return BMND_OK;
     };
-    // two 256-thread CTAs per SM: one CTA's barrier and serial phases are
-    // covered by the other's work (a single 512-thread CTA per SM, which
-    // leaves L1 room for the 5x5x5 Kronecker table, measured 16% slower)
     const int* b = sp.block;
     if (sp.exact_risk_weights) return run(group_filter_kernel<0, 0, 0, 0, kThreads>, kThreads);
     if (sp.ndim == 2 && b[0] == 8 && b[1] == 8) return run(group_filter_kernel<2, 8, 8, 1, kThreads>, kThreads);
