@@ -30,11 +30,13 @@
 //
 // Measured (one GB300, matching of one stage, against one warp or CTA per
 // reference evaluating every term): 128 x 144 x 160, 5x5x5 patches of an
-// estimate 18.8 ms (rows 6.8, selection 8.8 + 3.2) against 78.6; 320 x 256,
-// 8x8 patches of an estimate 0.70 ms against 3.37; 96 x 104 x 113, 4x4x4
-// patches of counts 3.8 ms against 4.7 (each reference is the only one of its
+// estimate 16.7 ms (rows 6.3, selection 8.4 + 1.9) against 78.6; 320 x 256,
+// 8x8 patches of an estimate 0.68 ms against 3.37; 96 x 104 x 113, 4x4x4
+// patches of counts 3.0 ms against 4.7 (each reference is the only one of its
 // 27 origins there, so little is shared); SSD, both stages: 80 x 96 x 90
-// 4.7 ms against 15.0, 768 x 640 2.2 ms against 15.2 (tensor-core products).
+// 4.4 ms against 15.0, 768 x 640 2.2 ms against 15.2 (tensor-core products).
+// A low-count volume's smooth estimate leaves hundreds of candidates per
+// reference open: 90^3 at peak 5, both stages 15.3 ms against 19.4.
 // The row kernels are bound by FP32 issue and shared-memory loads (log form:
 // the SFU), the selection by the latency of its short dependent phases.
 #include <cuda_runtime.h>
@@ -53,7 +55,6 @@ constexpr int kTileX = 96;     // 2-D: last-axis origins per tile (32 columns of
 constexpr int kSelWarps = 4;   // references per CTA of the selection
 constexpr int kQueue = 192;    // exact rescoring queue per reference
 constexpr int kAmb = 384;      // candidates whose acceptance alone is open, per reference
-constexpr int kRefine = 96;    // more open candidates than this: the series form thins them out first
 constexpr int kRowThreads3 = 512, kRowThreads2 = 256;
 constexpr float kLn2x2 = 1.38629436f;
 constexpr float kTinyCount = 7.88860905e-31f;  // 2^-100
@@ -79,9 +80,11 @@ struct BoxArgs {
     float* rows;       // (hi - lo) x rowlen screening distances
     int32_t* heavy;    // references of the chunk with many open candidates
     int32_t* heavy_n;  // their number
+    float* cuts;       // 3 per entry of heavy: certain-accept, certain-reject and top-list cuts
     int32_t* mode;     // per reference of the chunk: 0 SSD, 1 sqrt form, 2 log form
     const float* noise;  // SSD bias per window offset, or null
     float gamma;
+    int32_t per_cta;   // selection: references per CTA (its other warps help with their rescoring)
     int32_t tz, per;   // tile origins along the first axis, first-axis offsets per CTA
     int32_t ytiles;
 };
@@ -268,25 +271,41 @@ __global__ void __launch_bounds__(kRowThreads3, 1) box_rows_3d_kernel(BoxArgs b)
     if (b.colflag[x0] < 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kRowThreads3 / 32;
     const int y0 = static_cast<int>(blockIdx.y % b.ytiles) * (33 - W);
-    const int z0 = static_cast<int>(blockIdx.y / b.ytiles) * b.tz;
+    int z0 = static_cast<int>(blockIdx.y / b.ytiles) * b.tz;
     const int dz0 = static_cast<int>(blockIdx.z) * b.per - b.rad[0];
     const int per = min(b.per, b.rad[0] + 1 - dz0);
-    const int ZA = b.tz + W - 1, ZB = ZA + b.per - 1, XB = W - 1 + b.px, YB = 32 + 2 * b.rad[1];
-    float* A = smf;                    // [ZA][W][32]
-    float* B = A + ZA * W * 32;        // [ZB][XB][YB]
-    int32_t* map_s = reinterpret_cast<int32_t*>(B + ZB * XB * YB);  // [tz][32]
-    bool any = false;
+    const int XB = W - 1 + b.px, YB = 32 + 2 * b.rad[1];
+    int32_t* map_s = reinterpret_cast<int32_t*>(smf);  // [tz][32]
+    float* A = smf + b.tz * 32;                        // [ZA][W][32]
+    // the tile shrinks to the first-axis range that holds references of this chunk
+    __shared__ int zrange[2];
+    if (tid == 0) {
+        zrange[0] = b.tz;
+        zrange[1] = -1;
+    }
+    __syncthreads();
+#pragma unroll 4
     for (int i = tid; i < b.tz * 32; i += kRowThreads3) {
         const int z = z0 + i / 32, l = i % 32, y = y0 + l;
         int m = -1;
         if (l < 33 - W && z < b.cnt[0] && y < b.cnt[1]) m = b.map[grid_lin(b, z, y, x0)];
         const bool in = m >= b.lo && m < b.hi;
         map_s[i] = in ? static_cast<int32_t>(m - b.lo) : -1;
-        any |= in;
+        if (__any_sync(0xffffffffu, in) && lane == 0) {
+            atomicMin(&zrange[0], i / 32);
+            atomicMax(&zrange[1], i / 32);
+        }
     }
-    if (!__syncthreads_or(any)) return;
+    __syncthreads();
+    const int zfirst = zrange[0], tz = zrange[1] - zfirst + 1;
+    if (zrange[1] < 0) return;
+    z0 += zfirst;
+    map_s += zfirst * 32;
+    const int ZA = tz + W - 1, ZB = ZA + per - 1;
+    float* B = A + ZA * W * 32;  // [ZB][XB][YB]
     // the tile's own values; all integers below 4096: the log form
     bool counts = b.fvox != nullptr;
+#pragma unroll 4
     for (int i = tid; i < ZA * W * 32; i += kRowThreads3) {
         const int l = i % 32, k = (i / 32) % W, z = z0 + i / (32 * W), y = y0 + l;
         float v = 0.0f;
@@ -302,19 +321,29 @@ __global__ void __launch_bounds__(kRowThreads3, 1) box_rows_3d_kernel(BoxArgs b)
         return term == 0 ? v : (term == 1 ? box_transform<1>(v, b.inv_scale) : box_transform<2>(v, b.inv_scale));
     };
     for (int i = tid; i < ZA * W * 32; i += kRowThreads3) A[i] = transform(A[i]);
-    for (int row = warp; row < ZB * YB; row += nwarps) {
-        const int zi = row / YB, yi = row - zi * YB;
-        const int z = z0 + dz0 + zi, y = y0 - b.rad[1] + yi;
-        const bool in = z >= 0 && z < b.n[0] && y >= 0 && y < b.n[1];
-        const float* src = b.src + (static_cast<int64_t>(in ? z : 0) * b.n[1] + (in ? y : 0)) * b.n[2];
-        for (int xi = lane; xi < XB; xi += 32) {
-            const int x = x0 - b.rad[2] + xi;
-            const float v = in && x >= 0 && x < b.n[2] ? __ldg(src + x) : 0.0f;
-            B[(zi * XB + xi) * YB + yi] = transform(v);
+    // eight rows a warp in flight: with one CTA per SM nothing else covers the
+    // loads' latency
+    for (int xi = lane; xi < XB; xi += 32) {
+        const int x = x0 - b.rad[2] + xi;
+        const bool inx = x >= 0 && x < b.n[2];
+        for (int row0 = warp * 8; row0 < ZB * YB; row0 += nwarps * 8) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int zi = (row0 + k) / YB, yi = row0 + k - zi * YB;
+                const int z = z0 + dz0 + zi, y = y0 - b.rad[1] + yi;
+                const bool in = inx && zi < ZB && z >= 0 && z < b.n[0] && y >= 0 && y < b.n[1];
+                v[k] = in ? __ldg(b.src + (static_cast<int64_t>(z) * b.n[1] + y) * b.n[2] + x) : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int zi = (row0 + k) / YB, yi = row0 + k - zi * YB;
+                if (zi < ZB) B[(zi * XB + xi) * YB + yi] = transform(v[k]);
+            }
         }
     }
     if (blockIdx.z == 0)
-        for (int i = tid; i < b.tz * 32; i += kRowThreads3)
+        for (int i = tid; i < tz * 32; i += kRowThreads3)
             if (map_s[i] >= 0) b.mode[map_s[i]] = term;
     __syncthreads();
     const int ng = b.px / kG;
@@ -387,6 +416,7 @@ __global__ void __launch_bounds__(kRowThreads2, 2) box_rows_2d_kernel(BoxArgs b)
     float* B = A + ZA * XA;       // [ZB][XB]
     int32_t* map_s = reinterpret_cast<int32_t*>(B + ZB * XB);  // [tz][kTileX]
     bool any = false;
+#pragma unroll 4
     for (int i = tid; i < b.tz * kTileX; i += kRowThreads2) {
         const int z = z0 + i / kTileX, x = x0 + i % kTileX;
         int m = -1;
@@ -408,6 +438,7 @@ __global__ void __launch_bounds__(kRowThreads2, 2) box_rows_2d_kernel(BoxArgs b)
         if (lane == 0) ncol_s = n;
     }
     bool counts = b.fvox != nullptr;
+#pragma unroll 4
     for (int i = tid; i < ZA * XA; i += kRowThreads2) {
         const int z = z0 + i / XA, x = x0 + i % XA;
         float v = 0.0f;
@@ -426,10 +457,17 @@ __global__ void __launch_bounds__(kRowThreads2, 2) box_rows_2d_kernel(BoxArgs b)
     for (int zi = warp; zi < ZB; zi += nwarps) {
         const int z = z0 + dz0 + zi;
         const bool in = z >= 0 && z < b.n[0];
-        for (int xi = lane; xi < XB; xi += 32) {
-            const int x = x0 - b.rad[2] + xi;
-            const float v = in && x >= 0 && x < b.n[2] ? __ldg(b.src + static_cast<int64_t>(z) * b.n[2] + x) : 0.0f;
-            B[zi * XB + xi] = transform(v);
+        const float* src = b.src + static_cast<int64_t>(in ? z : 0) * b.n[2];
+        for (int xi0 = lane; xi0 < XB; xi0 += 160) {
+            float v[5];
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                const int x = x0 - b.rad[2] + xi0 + k * 32;
+                v[k] = in && xi0 + k * 32 < XB && x >= 0 && x < b.n[2] ? __ldg(src + x) : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < 5; ++k)
+                if (xi0 + k * 32 < XB) B[zi * XB + xi0 + k * 32] = transform(v[k]);
         }
     }
     if (blockIdx.z == 0)
@@ -491,6 +529,16 @@ struct Bound {
             hi += mg;
             lo -= mg;
         }
+    }
+
+    // square-root form: every term's w = ((r - c) / s)^2 is at most 1/16, since
+    // 2 (sqrt r - sqrt c)^2 >= (r - c)^2 / s gives w <= Q / s <= Q / min r
+    __device__ __forceinline__ bool close(float Q) const {
+        if (mode != 1) return false;
+        const float U = 5.96046448e-8f, q = fmaxf(Q, 0.0f);
+        const float m = rtS + fast_sqrt(0.5f * q);
+        const float S = 1.001f * (Sr + m * m);
+        return (q + U * (6.0f * fast_sqrt(S * q) + 8.0f * U * S + 32.0f * q)) * irmin <= 0.0624f;
     }
 
     __device__ __forceinline__ void raw(float Q, float& lo, float& hi) const {
@@ -620,6 +668,7 @@ struct SelectSmem {
     float red[kSelWarps];
     Bound bound[kSelWarps];
     int want[kSelWarps];  // exact keys wanted
+    int gone[kSelWarps];
 };
 
 // one term of the exact kernel's float32 distance
@@ -651,29 +700,34 @@ __device__ __forceinline__ float exact_of(const MatchArgs& a, const float* ref, 
 // the deviance term s w f(w), w = ((r - c) / s)^2, by its power series (terms
 // w^(k-1) / (k (2k - 1)), k <= 12: truncated below 1.5e-6 for w <= 1/2), which
 // has no cancellation; farther apart the ratio form (its error, 1.4e-6 s, is
-// below 2.6e-6 of such a term)
-__device__ __forceinline__ float series_sum(const MatchArgs& a, const float* ref, const float* cand,
-                                            const int32_t* poff) {
+// below 2.6e-6 of such a term).  CLOSE: every w is at most 1/16, where five
+// coefficients truncate below 2e-8.
+template <bool CLOSE>
+__device__ __forceinline__ float series_terms(const MatchArgs& a, const float* ref, const float* cand,
+                                              const int32_t* poff) {
     float sum = 0.0f, unused = 0.0f;
 #pragma unroll 4
     for (int p = 0; p < a.P; ++p) {
         const float r = ref[p];
         const float c = count_of(__ldg(cand + poff[p]), a.inv_scale);
         const float d = r - c, u = d * sfu_rcp(fmaxf(r + c, 1.17549435e-38f)), w = u * u;
-        float f = 1.0f / 276.0f;
-        f = fmaf(f, w, 1.0f / 231.0f);
-        f = fmaf(f, w, 1.0f / 190.0f);
-        f = fmaf(f, w, 1.0f / 153.0f);
-        f = fmaf(f, w, 1.0f / 120.0f);
-        f = fmaf(f, w, 1.0f / 91.0f);
-        f = fmaf(f, w, 1.0f / 66.0f);
-        f = fmaf(f, w, 1.0f / 45.0f);
+        float f = 1.0f / 45.0f;
+        if (!CLOSE) {
+            f = 1.0f / 276.0f;
+            f = fmaf(f, w, 1.0f / 231.0f);
+            f = fmaf(f, w, 1.0f / 190.0f);
+            f = fmaf(f, w, 1.0f / 153.0f);
+            f = fmaf(f, w, 1.0f / 120.0f);
+            f = fmaf(f, w, 1.0f / 91.0f);
+            f = fmaf(f, w, 1.0f / 66.0f);
+            f = fmaf(f, w, 1.0f / 45.0f);
+        }
         f = fmaf(f, w, 1.0f / 28.0f);
         f = fmaf(f, w, 1.0f / 15.0f);
         f = fmaf(f, w, 1.0f / 6.0f);
         f = fmaf(f, w, 1.0f);
         float t = d * u * f;
-        if (w > 0.5f) t = kLn2x2 * ratio_term(r, r + r, c, unused);
+        if (!CLOSE && w > 0.5f) t = kLn2x2 * ratio_term(r, r + r, c, unused);
         sum += t;
     }
     return sum;
@@ -701,13 +755,16 @@ __device__ __forceinline__ void scan_row(const float* row, int n, int lane, F f)
     }
 }
 
-// HEAVY = false: one warp per reference, kSelWarps per CTA, over the chunk; a
-// reference with many open candidates goes to the heavy list.
-// HEAVY = true: one CTA per reference of that list.  Its warps make the same
-// passes and share the refinement of the row: every open candidate's value
-// becomes its series-form deviance (SSD: exact distance) and the passes run
-// again on the tighter bounds; if that is not enough (keys that tie), the
-// values become the exact keys.
+// HEAVY = false: one warp per reference, up to kSelWarps per CTA, over the chunk;
+// a reference with more open candidates than the queue holds goes to the heavy
+// list, with the cuts it found.
+// HEAVY = true: one CTA per reference of that list.  Its warps share the
+// refinement of the row: every open candidate's value becomes its series-form
+// deviance (SSD: exact distance) and the passes run again on the tighter bounds;
+// if that is not enough (keys that tie), the values become the exact keys.
+// 7.4 K references of a smooth 40 x 49 x 66 estimate, 6.1 K of them heavy: 2.7 ms
+// with every first pass made again and the queue tried up to 96 entries only,
+// 1.5 ms so.
 template <bool SSD, bool HEAVY>
 __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs a, BoxArgs b) {
     extern __shared__ __align__(16) unsigned char raw[];
@@ -735,11 +792,11 @@ __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs
         bias = fmaxf(fmaxf(s.red[0], s.red[1]), fmaxf(s.red[2], s.red[3]));
     }
     const int64_t items = HEAVY ? *b.heavy_n : b.hi - b.lo;
-    const int64_t per_cta = HEAVY ? 1 : kSelWarps;
+    const int per_cta = HEAVY ? 1 : b.per_cta;
     for (int64_t base = blockIdx.x * per_cta; base < items; base += gridDim.x * per_cta) {
         __syncthreads();  // the previous references' shared data is no longer read
-        const bool mine = HEAVY || base + warp < items;
-        const int64_t r = HEAVY ? b.heavy[base] : b.lo + base + warp;
+        const bool mine = HEAVY || (warp < per_cta && base + warp < items);
+        const int64_t r = HEAVY ? b.heavy[base] : b.lo + base + (mine ? warp : 0);
         int c[3] = {0, 0, 0};
         bool ok = mine && ref_position(a, b, r, c);
         int64_t center_lin = 0;
@@ -791,140 +848,167 @@ __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs
             for (int d = 0; d < 3; ++d)
                 window *= min(c[d] + b.rad[d], b.cnt[d] - 1) - max(c[d] - b.rad[d], 0) + 1;
             int settled = 0;  // HEAVY: accepted, and no longer in the row
+            float cuts[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll 1
             for (int level = 0; level < (HEAVY ? 2 : 1); ++level) {
-                // certainly accepted: Q <= q_cert; certainly rejected: Q >= q_rej
-                const float q_cert = below(bd, thr, q_thr, 1e-7f * fabsf(q_thr) + tiny, lane);
-                const float q_rej = above(bd, thr, q_thr, 1e-7f * fabsf(q_thr) + tiny, lane);
-                // pass 1: the certain accepts, and the 4 smallest of every lane
-                int finite = 0;
-                n_cert = 0;
-                float t[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
-                scan_row(row, n, lane, [&](int, float q) {
-                    finite += q < INFINITY ? 1 : 0;
-                    n_cert += q <= q_cert ? 1 : 0;
-                    if (q < t[3]) {
-                        t[3] = q;
-#pragma unroll
-                        for (int e = 3; e > 0; --e) {
-                            const float lo = fminf(t[e - 1], t[e]), hi = fmaxf(t[e - 1], t[e]);
-                            t[e - 1] = lo;
-                            t[e] = hi;
+                // the cuts of the first level come with the list: its refinement takes
+                // every candidate below them (of 4.4 M such candidates of a smooth
+                // estimate the race below left 4.1 M, at half of this kernel's work)
+                const bool handed = HEAVY && !SSD && level == 0;
+                float q_cert, q_rej, q_top;
+                uint64_t v_top = ~0ull;
+                if (handed) {
+                    q_cert = b.cuts[3 * base];
+                    q_rej = b.cuts[3 * base + 1];
+                    q_top = b.cuts[3 * base + 2];
+                } else {
+                    // certainly accepted: Q <= q_cert; certainly rejected: Q >= q_rej
+                    q_cert = below(bd, thr, q_thr, 1e-7f * fabsf(q_thr) + tiny, lane);
+                    q_rej = above(bd, thr, q_thr, 1e-7f * fabsf(q_thr) + tiny, lane);
+                    // pass 1: the certain accepts, and the 4 smallest of every lane
+                    int finite = 0;
+                    n_cert = 0;
+                    float t[4] = {INFINITY, INFINITY, INFINITY, INFINITY};
+                    scan_row(row, n, lane, [&](int, float q) {
+                        finite += q < INFINITY ? 1 : 0;
+                        n_cert += q <= q_cert ? 1 : 0;
+                        if (q < t[3]) {
+                            t[3] = q;
+    #pragma unroll
+                            for (int e = 3; e > 0; --e) {
+                                const float lo = fminf(t[e - 1], t[e]), hi = fmaxf(t[e - 1], t[e]);
+                                t[e - 1] = lo;
+                                t[e] = hi;
+                            }
                         }
+                    });
+                    finite = __reduce_add_sync(0xffffffffu, finite);
+                    n_cert = __reduce_add_sync(0xffffffffu, n_cert);
+                    if (level == 0 && finite != window) {
+                        ok = false;  // infinities or NaN among the values: the exact kernel decides
+                        break;
                     }
-                });
-                finite = __reduce_add_sync(0xffffffffu, finite);
-                n_cert = __reduce_add_sync(0xffffffffu, n_cert);
-                if (level == 0 && finite != window) {
-                    ok = false;  // infinities or NaN among the values: the exact kernel decides
-                    break;
-                }
-                // beyond q_top a candidate cannot reach the top K (nor the first R)
-                auto cut = [&](float v) {
-                    float lo, hi;
-                    bd.eval(v, lo, hi);
-                    return v < INFINITY ? above(bd, hi, v, 1e-7f * fabsf(v) + tiny, lane) : INFINITY;
-                };
-                float q_top = q_rej;
-                if (n_cert >= K) q_top = cut(kth_of_kept(t, K));
-                if (n_cert < R) q_top = fmaxf(q_top, R <= window ? cut(kth_of_kept(t, R)) : INFINITY);
-                // pass 2: queue what the bounds leave open
-                nq = 0;
-                na = 0;
-                scan_row(row, n, lane, [&](int i, float q) {
-                    const bool take = q < INFINITY && q <= q_top;
-                    const bool open = q > q_cert && q < q_rej;
-                    if (!__any_sync(0xffffffffu, take || open)) return;
-                    const unsigned mt = __ballot_sync(0xffffffffu, take);
-                    const unsigned ma = __ballot_sync(0xffffffffu, open && !take);
-                    if (take) {
-                        const int at = nq + __popc(mt & before);
-                        if (at < kQueue) s.idx[warp][at] = i;
-                    } else if (open) {
-                        const int at = na + __popc(ma & before);
-                        if (at < kAmb) s.amb[warp][at] = i;
-                    }
-                    nq += __popc(mt);
-                    na += __popc(ma);
-                });
-                // the race by keys: best holds the K smallest (upper key, position),
-                // sorted across the lanes; whoever's (lower key, position) lies above
-                // its last entry is out.  Where keys tie (flat regions) this leaves
-                // the first positions.
-                const bool listed = nq <= kQueue;
-                const int entries = listed ? nq : n;
-                uint64_t best = ~0ull;
-                __syncwarp();
-                for (int j0 = 0; j0 < entries; j0 += 32) {
-                    const int j = j0 + lane;
-                    const int i = listed && j < entries ? s.idx[warp][j] : j;
-                    const float q = j < entries ? row[i] : INFINITY;
-                    uint64_t k = ~0ull;
-                    if (q < INFINITY && q <= q_top) {
+                    // beyond q_top a candidate cannot reach the top K (nor the first R)
+                    auto cut = [&](float v) {
                         float lo, hi;
-                        bd.raw(q, lo, hi);
-                        k = composite_key(key_of<SSD>(hi), i);
-                    }
-                    keep_smallest(best, k, K, lane);
-                }
-                const uint64_t v_top = __shfl_sync(0xffffffffu, best, K - 1);
-                int kept = 0, known_acc = 0;
-                for (int j0 = 0; j0 < entries; j0 += 32) {
-                    const int j = j0 + lane;
-                    const int i = listed && j < entries ? s.idx[warp][j] : j;
-                    const float q = j < entries ? row[i] : INFINITY;
-                    bool race = false, amb = false;
-                    float klo = 0.0f, khi = 0.0f;
-                    const bool open = q > q_cert && q < q_rej;
-                    if (q < INFINITY && q <= q_top) {
-                        bd.raw(q, klo, khi);
-                        klo = key_of<SSD>(klo);
-                        khi = key_of<SSD>(khi);
-                        race = composite_key(klo, i) <= v_top;
-                        if (!race && open) {
-                            known_acc += khi < tkey ? 1 : 0;
-                            amb = khi >= tkey && klo < tkey;
+                        bd.eval(v, lo, hi);
+                        return v < INFINITY ? above(bd, hi, v, 1e-7f * fabsf(v) + tiny, lane) : INFINITY;
+                    };
+                    q_top = q_rej;
+                    if (n_cert >= K) q_top = cut(kth_of_kept(t, K));
+                    if (n_cert < R) q_top = fmaxf(q_top, R <= window ? cut(kth_of_kept(t, R)) : INFINITY);
+                    // pass 2: queue what the bounds leave open
+                    nq = 0;
+                    na = 0;
+                    scan_row(row, n, lane, [&](int i, float q) {
+                        const bool take = q < INFINITY && q <= q_top;
+                        const bool open = q > q_cert && q < q_rej;
+                        if (!__any_sync(0xffffffffu, take || open)) return;
+                        const unsigned mt = __ballot_sync(0xffffffffu, take);
+                        const unsigned ma = __ballot_sync(0xffffffffu, open && !take);
+                        if (take) {
+                            const int at = nq + __popc(mt & before);
+                            if (at < kQueue) s.idx[warp][at] = i;
+                        } else if (open) {
+                            const int at = na + __popc(ma & before);
+                            if (at < kAmb) s.amb[warp][at] = i;
+                        }
+                        nq += __popc(mt);
+                        na += __popc(ma);
+                    });
+                    // the race by keys: best holds the K smallest (upper key, position),
+                    // sorted across the lanes; whoever's (lower key, position) lies above
+                    // its last entry is out.  Where keys tie (flat regions) this leaves
+                    // the first positions.
+                    const bool listed = nq <= kQueue;
+                    if (!HEAVY && !SSD && !listed) {
+                        // the race pays off where keys tie, not where the bounds are wide
+                        float lo, hi;
+                        bd.raw(kth_of_kept(t, min(K, window)), lo, hi);
+                        if (!(key_of<false>(lo) == key_of<false>(hi))) {
+                            defer = 1;
+                            cuts[0] = q_cert;
+                            cuts[1] = q_rej;
+                            cuts[2] = q_top;
+                            break;
                         }
                     }
-                    const unsigned mr = __ballot_sync(0xffffffffu, race);
-                    const unsigned ma = __ballot_sync(0xffffffffu, amb);
-                    if (race) {
-                        const int at = kept + __popc(mr & before);
-                        if (at < kQueue) {
-                            s.idx[warp][at] = i | (open ? kOpenBit : 0);
-                            s.key[warp][at] = (static_cast<uint64_t>(__float_as_uint(klo)) << 32) | __float_as_uint(khi);
-                        }
-                    } else if (amb) {
-                        const int at = na + __popc(ma & before);
-                        if (at < kAmb) s.amb[warp][at] = i;
-                    }
-                    kept += __popc(mr);
-                    na += __popc(ma);
+                    const int entries = listed ? nq : n;
+                    uint64_t best = ~0ull;
                     __syncwarp();
-                }
-                nq = kept;
-                const bool fits = nq <= kQueue && na <= kAmb;
-                if (fits && (HEAVY ? level == 1 : nq <= kRefine)) {
-                    n_cert += __reduce_add_sync(0xffffffffu, known_acc);
-                    break;
-                }
-                if (!HEAVY) {
-                    defer = 1;
-                    break;
+                    for (int j0 = 0; j0 < entries; j0 += 32) {
+                        const int j = j0 + lane;
+                        const int i = listed && j < entries ? s.idx[warp][j] : j;
+                        const float q = j < entries ? row[i] : INFINITY;
+                        uint64_t k = ~0ull;
+                        if (q < INFINITY && q <= q_top) {
+                            float lo, hi;
+                            bd.raw(q, lo, hi);
+                            k = composite_key(key_of<SSD>(hi), i);
+                        }
+                        keep_smallest(best, k, K, lane);
+                    }
+                    v_top = __shfl_sync(0xffffffffu, best, K - 1);
+                    int kept = 0, known_acc = 0;
+                    for (int j0 = 0; j0 < entries; j0 += 32) {
+                        const int j = j0 + lane;
+                        const int i = listed && j < entries ? s.idx[warp][j] : j;
+                        const float q = j < entries ? row[i] : INFINITY;
+                        bool race = false, amb = false;
+                        float klo = 0.0f, khi = 0.0f;
+                        const bool open = q > q_cert && q < q_rej;
+                        if (q < INFINITY && q <= q_top) {
+                            bd.raw(q, klo, khi);
+                            klo = key_of<SSD>(klo);
+                            khi = key_of<SSD>(khi);
+                            race = composite_key(klo, i) <= v_top;
+                            if (!race && open) {
+                                known_acc += khi < tkey ? 1 : 0;
+                                amb = khi >= tkey && klo < tkey;
+                            }
+                        }
+                        const unsigned mr = __ballot_sync(0xffffffffu, race);
+                        const unsigned ma = __ballot_sync(0xffffffffu, amb);
+                        if (race) {
+                            const int at = kept + __popc(mr & before);
+                            if (at < kQueue) {
+                                s.idx[warp][at] = i | (open ? kOpenBit : 0);
+                                s.key[warp][at] = (static_cast<uint64_t>(__float_as_uint(klo)) << 32) | __float_as_uint(khi);
+                            }
+                        } else if (amb) {
+                            const int at = na + __popc(ma & before);
+                            if (at < kAmb) s.amb[warp][at] = i;
+                        }
+                        kept += __popc(mr);
+                        na += __popc(ma);
+                        __syncwarp();
+                    }
+                    nq = kept;
+                    const bool fits = nq <= kQueue && na <= kAmb;
+                    if (fits && (!HEAVY || level == 1)) {
+                        n_cert += __reduce_add_sync(0xffffffffu, known_acc);
+                        break;
+                    }
+                    if (!HEAVY) {
+                        defer = 1;
+                        cuts[0] = q_cert;
+                        cuts[1] = q_rej;
+                        cuts[2] = q_top;
+                        break;
+                    }
                 }
                 // refinement: this warp's quarter of the row
                 const bool exact = SSD || level == 1;
                 auto needed = [&](int i, float q) {
                     const bool open = q > q_cert && q < q_rej;
                     if (!(q < INFINITY) || open || q > q_top) return open;
+                    if (handed) return true;
                     float lo, hi;
                     bd.raw(q, lo, hi);
                     return composite_key(key_of<SSD>(lo), i) <= v_top;
                 };
-                int gone = 0;
-                scan_row(row, n, lane, [&](int i, float q) { gone += q <= q_cert && !needed(i, q) ? 1 : 0; });
-                settled += __reduce_add_sync(0xffffffffu, gone);
                 __syncthreads();  // every warp has read the row
+                int gone = 0;  // certain accepts of this quarter that leave the row
                 int fill = 0;
                 auto refine = [&](int to) {
                     for (int at = lane; at < to; at += 32) {
@@ -934,7 +1018,8 @@ __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs
                                             (dx - b.rad[2]);
                         float d;
                         if (!exact) {
-                            d = series_sum(a, s.ref[warp], cand, s.poff);
+                            d = bd.close(row[i]) ? series_terms<true>(a, s.ref[warp], cand, s.poff)
+                                             : series_terms<false>(a, s.ref[warp], cand, s.poff);
                         } else {
                             d = exact_of<SSD>(a, s.ref[warp], cand, s.poff, mode == 2);
                             if (SSD && b.noise) d = sub_rn(d, mul_rn(b.gamma, __ldg(b.noise + rem * b.nx + dx)));
@@ -947,6 +1032,7 @@ __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs
                     const int i = i0 + lane;
                     const float q = i < n ? row[i] : INFINITY;
                     bool open = needed(i, q);
+                    gone += q <= q_cert && !open ? 1 : 0;
                     if (!open && i < n) row[i] = INFINITY;
                     if (open && exact && !SSD) {
                         float lo, hi;
@@ -973,7 +1059,10 @@ __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs
                     }
                 }
                 refine(fill);
+                gone = __reduce_add_sync(0xffffffffu, gone);
+                if (lane == 0) s.gone[warp] = gone;
                 __syncthreads();  // the row is complete
+                settled += s.gone[0] + s.gone[1] + s.gone[2] + s.gone[3];
                 bd.mode = 3;
                 if (exact) {
                     // the K smallest by (exact key, position); row order is position order
@@ -999,7 +1088,12 @@ __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs
                 }
             }
             n_cert += settled;
-            if (defer && lane == 0) b.heavy[atomicAdd(b.heavy_n, 1)] = static_cast<int32_t>(r);
+            if (defer && lane == 0) {
+                const int at = atomicAdd(b.heavy_n, 1);
+                b.heavy[at] = static_cast<int32_t>(r);
+#pragma unroll
+                for (int e = 0; e < 3; ++e) b.cuts[3 * static_cast<int64_t>(at) + e] = cuts[e];
+            }
             if (lane == 0) {
                 bd.mode = SSD ? 0 : 3;
                 s.bound[warp] = bd;
@@ -1044,7 +1138,7 @@ __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs
                 int widx;
                 const float* cand = locate(w, ri, lin, widx);
                 float lo, hi;
-                s.bound[w].raw(series_sum(a, s.ref[w], cand, s.poff), lo, hi);
+                s.bound[w].raw(series_terms<false>(a, s.ref[w], cand, s.poff), lo, hi);
                 const float klo = key_of<false>(lo), khi = key_of<false>(hi);
                 const uint64_t kb = (static_cast<uint64_t>(__float_as_uint(klo)) << 32) | __float_as_uint(khi);
                 if (!amb) {
@@ -1242,6 +1336,17 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
     // the shared terms pay off while references are dense: up to one per 64
     // origins (the schedules have one per 4.5 to 27)
     if (b.rowlen > (1 << 20) || a.n_refs * 64 < n_lins) return BMND_OK;
+    // Few references of a stage on counts: the kernel of tabulated terms has no
+    // phases that wait on each other.  One GB300, that kernel against this file's:
+    // 64 x 64 34 against 115 us, 140 x 140 (3.9 K references) 164 against 169,
+    // 200 x 180 (7.5 K) 312 against 214; 40 x 49 x 66 (4.4 K) 454 against 590,
+    // 51 x 65 x 74 (9 K) 955 against 918, 72 x 80 x 60 1359 against 1086.
+    // Real-valued stages come here whatever their size: few references gain
+    // 0.1 ms at best in the screened kernel, and those it cannot settle cost
+    // 3.1 ms there (24 x 24 x 40, peak 30; here 0.5 in all).
+    const bool want_f = !ssd && precision != BMND_MATCH_REAL_VALUED && a.inv_scale == 1.0f;
+    const bool few = a.n_refs < (shape2 ? 4096 : 8192);
+    if (want_f && precision == BMND_MATCH_EXACT && a.use_table && few) return BMND_OK;
 
     // tiles: the largest whose shared memory fits; first-axis offsets are split
     // over CTAs until every SM has several
@@ -1260,6 +1365,11 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
     b.ytiles = shape2 ? 1 : (b.cnt[1] + 32 - W) / (33 - W);
     const int64_t columns = shape2 ? (b.cnt[2] + kTileX - 1) / kTileX : (b.cnt[2] + 2) / 3;
     auto tiles = [&]() { return columns * b.ytiles * ztiles; };
+    // (small grids: shorter tiles until there is a CTA or two for every SM)
+    while (b.tz > 2 * W && tiles() * b.nz < 152 * 2) {
+        b.tz = (b.tz + 1) / 2;
+        ztiles = (b.cnt[0] + b.tz - 1) / b.tz;
+    }
     int splits = static_cast<int>(std::min<int64_t>(b.nz, (152 * 8 + tiles() - 1) / tiles()));
     b.per = (b.nz + splits - 1) / splits;
     while (smem_of(b.tz, b.per) > limit && b.per > 1) --b.per;
@@ -1273,12 +1383,11 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
     if (static_cast<int64_t>(b.ytiles) * ztiles > 65535 || splits > 65535) return BMND_OK;
 
     // scratch: origin map and column flags, the counts' box sums, the rows of a chunk of references
-    const bool want_f = !ssd && precision != BMND_MATCH_REAL_VALUED && a.inv_scale == 1.0f;
     const uint64_t o_flag = round256(4ull * n_lins);
     const uint64_t o_fvox = o_flag + round256(4ull * b.cnt[2]);
     const uint64_t o_fbox = o_fvox + (want_f ? round256(4ull * b.nvox) : 0);
     const uint64_t o_rows = o_fbox + (want_f ? round256(4ull * n_lins) : 0);
-    const uint64_t per_ref = 4ull * b.rowlen + 8;
+    const uint64_t per_ref = 4ull * b.rowlen + 20;
     char* base = nullptr;
     uint64_t bytes = 0;
     bool owned = false;
@@ -1310,6 +1419,7 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
     b.mode = reinterpret_cast<int32_t*>(base + o_rows + round256(4ull * b.rowlen * chunk));
     b.heavy_n = b.mode + chunk;
     b.heavy = b.heavy_n + 1;
+    b.cuts = reinterpret_cast<float*>(b.heavy + chunk);
 
     auto run = [&]() -> int32_t {
         BMND_CUDA_TRY(cudaMemsetAsync(base, 0xff, o_fvox, stream));
@@ -1352,7 +1462,10 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
                 else box_rows_3d_kernel<4><<<grid, kRowThreads3, smem, stream>>>(b);
             }
             BMND_LAUNCH_CHECK("box_rows_kernel");
-            const unsigned ctas = static_cast<unsigned>(std::min<int64_t>((b.hi - b.lo + kSelWarps - 1) / kSelWarps, sel_ctas));
+            // few references: fewer per CTA, whose warps then share their rescoring
+            b.per_cta = static_cast<int32_t>(std::clamp<int64_t>((b.hi - b.lo + sel_ctas - 1) / sel_ctas, 1, kSelWarps));
+            const int64_t sel_items = (b.hi - b.lo + b.per_cta - 1) / b.per_cta;
+            const unsigned ctas = static_cast<unsigned>(std::min(sel_items, sel_ctas));
             const unsigned hctas = static_cast<unsigned>(std::min<int64_t>(b.hi - b.lo, heavy_ctas));
             const size_t ss = sizeof(SelectSmem);
             if (ssd) box_select_kernel<true, false><<<ctas, kSelWarps * 32, ss, stream>>>(a, b);

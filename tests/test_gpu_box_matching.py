@@ -132,3 +132,54 @@ def test_ssd_matching_equals_exact(cuda, native, shape, block, radius, kind, max
     want = _few_at_a_time(cuda, native, vol, block, *args, refs=refs, noise=noise, gamma=0.7)
     for g, w in zip(got, want):
         np.testing.assert_array_equal(g, w)
+
+
+# enough references for the stages on counts, too, to take the box-sum kernels
+DENSE = [
+    ((57, 203), (8, 8), (19, 19)),
+    ((150, 40), (8, 8), (5, 12)),
+    ((13, 37, 45), (5, 5, 5), (7, 7, 7)),
+    ((33, 12, 40), (4, 4, 4), (7, 3, 5)),
+    ((5, 130, 70), (5, 5, 5), (2, 7, 1)),
+    ((300, 9, 9), (4, 4, 4), (0, 2, 7)),
+]
+
+
+@pytest.mark.parametrize("shape,block,radius", DENSE)
+@pytest.mark.parametrize("kind,max_m,min_m,thr", [
+    ("counts", 16, 2, 2.9527), ("bright", 16, 2, 2.9527), ("estimate", 32, 2, 0.3937), ("zeros", 32, 2, 0.7689),
+])
+def test_dense_references_equal_exact(cuda, native, shape, block, radius, kind, max_m, min_m, thr):
+    from bmnd_gb300 import _abi
+
+    rng = np.random.default_rng(zlib.crc32(repr((shape, kind)).encode()))
+    vol = _volume(kind, shape, rng).astype(np.float32)
+    counts = [s - b + 1 for s, b in zip(shape, block)]
+    refs = np.stack(np.meshgrid(*[np.arange(c) for c in counts], indexing="ij"), -1).reshape(-1, len(shape))
+    args = (radius, max_m, min_m, thr, DEV, _abi.MATCH_EXACT)
+    got = _match(cuda, native, vol, block, *args, refs)
+    some = rng.choice(len(refs), size=min(len(refs), 2000), replace=False)
+    want = _few_at_a_time(cuda, native, vol, block, *args, refs=refs[some])
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g[some], w)
+
+
+@pytest.mark.parametrize("shape,block,radius", SHAPES)
+@pytest.mark.parametrize("kind,max_m,min_m,thr", [
+    ("counts", 16, 2, 2.9527), ("estimate", 32, 2, 0.3937), ("estimate", 32, 2, 0.01), ("low", 32, 2, 0.7689),
+    ("flat", 32, 2, 0.7689), ("zeros", 32, 2, 0.7689), ("overflow", 16, 2, 2.0),
+])
+def test_real_valued_matching_equals_exact(cuda, native, shape, block, radius, kind, max_m, min_m, thr):
+    """Estimates, also smooth ones that leave most of the window open."""
+    from bmnd_gb300 import _abi
+
+    rng = np.random.default_rng(zlib.crc32(repr((shape, kind, thr)).encode()))
+    vol = 4.0 + rng.normal(0, 0.01, size=shape) if kind == "flat" else _volume(kind, shape, rng)
+    vol = vol.astype(np.float32)
+    refs = _refs(shape, block, rng)
+    # a count scale other than 1: no integer-count form, whatever the values
+    args = (radius, max_m, min_m, thr, DEV, _abi.MATCH_EXACT)
+    got = _match(cuda, native, vol, block, *args, refs, scale=0.75)
+    want = _few_at_a_time(cuda, native, vol, block, *args, refs=refs, scale=0.75)
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g, w)
