@@ -644,14 +644,24 @@ def bmnd(
     if torch_input:
         torch = _torch()
         dev_vol = volume.detach()
-        if not bool(torch.isfinite(dev_vol).all()):
-            raise ValueError("volume must contain only finite values.")
-        dev_vol = dev_vol.to(torch.float32)
-        if not bool(torch.isfinite(dev_vol).all()):
-            raise ValueError("volume values must be representable as finite float32 values.")
-        if resolved.is_poisson and bool((dev_vol < 0).any()):
-            raise ValueError("Direct Poisson input must contain only non-negative values.")
-        all_zero = not bool((dev_vol != 0).any())
+        if dev_vol.is_cuda and dev_vol.dtype == torch.float32 and dev_vol.numel():
+            # one pass and one read-back for all four checks (see the NumPy branch)
+            mm = torch.aminmax(dev_vol)
+            lo, hi = (float(v) for v in torch.stack([mm.min, mm.max]).cpu())
+            if not (np.isfinite(lo) and np.isfinite(hi)):
+                raise ValueError("volume must contain only finite values.")
+            if resolved.is_poisson and lo < 0.0:
+                raise ValueError("Direct Poisson input must contain only non-negative values.")
+            all_zero = lo == 0.0 and hi == 0.0
+        else:
+            if not bool(torch.isfinite(dev_vol).all()):
+                raise ValueError("volume must contain only finite values.")
+            dev_vol = dev_vol.to(torch.float32)
+            if not bool(torch.isfinite(dev_vol).all()):
+                raise ValueError("volume values must be representable as finite float32 values.")
+            if resolved.is_poisson and bool((dev_vol < 0).any()):
+                raise ValueError("Direct Poisson input must contain only non-negative values.")
+            all_zero = not bool((dev_vol != 0).any())
     else:
         arr = np.asarray(volume)
         if arr.dtype == np.float32 and arr.size:

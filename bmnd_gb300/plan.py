@@ -67,6 +67,37 @@ def spatial_forward(profile, ndim: int, stage: str) -> list:
     return [None if kind is None else axis_matrices(kind, block[a])[0] for a, kind in enumerate(spatial)]
 
 
+@lru_cache(maxsize=64)
+def _stage_tables(kinds: tuple, block: tuple[int, ...], beta: float, metric: bool):
+    """The spatial matrices, the window and (``metric``) the synthesis metric as
+    the bytes of their ``StageParams`` fields.  They depend on nothing but a
+    profile's transforms, patch and window shape; built anew for each call they
+    took 0.5 of the 1.4 ms of a 64 x 64 denoising, with the GPU idle."""
+    fwd_bytes, inv_bytes, inverse = [], [], []
+    for kind, n in zip(kinds, block):
+        if kind is None:
+            fwd = np.eye(n, dtype=np.float32)
+            inv = fwd
+        else:
+            fwd, inv = axis_matrices(kind, n)
+        inverse.append(inv)
+        for m, out in ((fwd, fwd_bytes), (inv, inv_bytes)):
+            flat = np.zeros(_abi.MAX_EDGE * _abi.MAX_EDGE, dtype=np.float32)
+            flat[: n * n] = np.asarray(m, dtype=np.float32).reshape(-1)
+            out.append(flat.tobytes())
+    window = kaiser_window(block, beta).reshape(-1)
+    if window.size > _abi.MAX_PATCH:
+        raise unsupported(f"patch volume {window.size} exceeds {_abi.MAX_PATCH}")
+    wbuf = np.zeros(_abi.MAX_PATCH, dtype=np.float32)
+    wbuf[: window.size] = window
+    diag = None
+    if metric:
+        diag = np.zeros(_abi.MAX_PATCH, dtype=np.float64)
+        diag[: window.size] = _spatial_metric_diag(inverse, window)
+        diag = diag.tobytes()
+    return tuple(fwd_bytes), tuple(inv_bytes), wbuf.tobytes(), diag
+
+
 def stage_params(profile, shape: tuple[int, ...], stage: str, distance: BlockMatchDistance,
                  variance_k: int, match_precision: int = _abi.MATCH_EXACT, gauss: dict | None = None,
                  null_table=None, fast_transforms: bool = False) -> _abi.StageParams:
@@ -172,31 +203,14 @@ def stage_params(profile, shape: tuple[int, ...], stage: str, distance: BlockMat
         if gauss.get("ssd") is not None:
             p.match_noise_ssd = gauss["ssd"].data_ptr()
             p.ssd_gamma = float(gauss["gamma"])
-    inverse = []
+    fwd, inv, window, metric = _stage_tables(tuple(spatial), block, float(getattr(profile, f"{stage}_kaiser_beta")),
+                                             bool(p.windowed_synthesis))
     for a in range(ndim):
-        kind = spatial[a]
-        if kind is None:
-            fwd = np.eye(block[a], dtype=np.float32)
-            inv = fwd
-        else:
-            fwd, inv = axis_matrices(kind, block[a])
-        inverse.append(inv)
-        flat_f = np.zeros(_abi.MAX_EDGE * _abi.MAX_EDGE, dtype=np.float32)
-        flat_i = np.zeros(_abi.MAX_EDGE * _abi.MAX_EDGE, dtype=np.float32)
-        flat_f[: block[a] * block[a]] = np.asarray(fwd, dtype=np.float32).reshape(-1)
-        flat_i[: block[a] * block[a]] = np.asarray(inv, dtype=np.float32).reshape(-1)
-        ctypes.memmove(p.spatial_fwd[a], flat_f.ctypes.data, flat_f.nbytes)
-        ctypes.memmove(p.spatial_inv[a], flat_i.ctypes.data, flat_i.nbytes)
-    window = kaiser_window(block, float(getattr(profile, f"{stage}_kaiser_beta"))).reshape(-1)
-    if window.size > _abi.MAX_PATCH:
-        raise unsupported(f"patch volume {window.size} exceeds {_abi.MAX_PATCH}")
-    wbuf = np.zeros(_abi.MAX_PATCH, dtype=np.float32)
-    wbuf[: window.size] = window
-    ctypes.memmove(p.window, wbuf.ctypes.data, wbuf.nbytes)
-    if p.windowed_synthesis:
-        diag = np.zeros(_abi.MAX_PATCH, dtype=np.float64)
-        diag[: window.size] = _spatial_metric_diag(inverse, window)
-        ctypes.memmove(p.spatial_metric_diag, diag.ctypes.data, diag.nbytes)
+        ctypes.memmove(p.spatial_fwd[a], fwd[a], len(fwd[a]))
+        ctypes.memmove(p.spatial_inv[a], inv[a], len(inv[a]))
+    ctypes.memmove(p.window, window, len(window))
+    if metric is not None:
+        ctypes.memmove(p.spatial_metric_diag, metric, len(metric))
     return p
 
 
