@@ -30,6 +30,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <type_traits>
 #include <vector>
 
@@ -959,7 +960,7 @@ __global__ void __launch_bounds__(224, 1) conv_mid_tc_kernel(const __grid_consta
 // are discarded.  The CTAs split the taps into groups of 9, so one group's
 // accumulators (9 x C columns) fit the 512 columns of tensor memory, and each
 // CTA accumulates its share of the tiles for the whole launch; the per-CTA
-// sums are added by reduce_partials_kernel.  Roles: warp 0 issues the TMA
+// sums are added by reduce_groups_kernel.  Roles: warp 0 issues the TMA
 // loads (two stages); one thread each of warps 1 and 2 issues the MMAs of the
 // first 5 taps of the group and of the other 4 (one issuing thread cannot keep
 // the tensor core busy with MMAs this small); at the end warps 0-1 read
@@ -1199,78 +1200,236 @@ __global__ void __launch_bounds__(128, 1) wgrad_tc_kernel(const __grid_constant_
 
 // bias gradient of a C-channel layer: per-CTA partial sums of the output
 // gradient over a contiguous share of the voxels, into the bias slots of the
-// partial records; a thread reads the 8 channels of a voxel as 16 bytes
+// partial records.  Four warps take one 8-channel chunk plane each, four 16-byte
+// loads a thread in flight: with the planes one after another and one load, 4 x
+// 48^3 voxels of 48 channels (42 MB, in the L2 since the layer above wrote them)
+// took 27 us.
 template <int C>
-__global__ void __launch_bounds__(256) bias_partial_kernel(const bf16* __restrict__ gout, int64_t nv,
-                                                           float* __restrict__ partial, int64_t nparams,
-                                                           int64_t wparams) {
-    __shared__ float red[8][8];
+__global__ void __launch_bounds__(C * 16) bias_partial_kernel(const bf16* __restrict__ gout, int64_t nv,
+                                                              float* __restrict__ partial, int64_t nparams,
+                                                              int64_t wparams) {
+    __shared__ float red[4][C];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ch = warp >> 2, sub = warp & 3;
     const int64_t per = (nv + gridDim.x - 1) / gridDim.x;
     const int64_t v0 = static_cast<int64_t>(blockIdx.x) * per, v1 = min(nv, v0 + per);
-    for (int ch = 0; ch < C / 8; ++ch) {
-        const uint4* src = reinterpret_cast<const uint4*>(gout + static_cast<int64_t>(ch) * nv * 8);
-        float s[8];
+    const uint4* src = reinterpret_cast<const uint4*>(gout + static_cast<int64_t>(ch) * nv * 8);
+    float s[4][8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) s[e] = 0.0f;
-        for (int64_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-            const uint4 q = src[v];
-            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[k][e] = 0.0f;
+    for (int64_t v = v0 + sub * 32 + lane; v < v1; v += 512) {
+        uint4 q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = v + k * 128 < v1 ? src[v + k * 128] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t w[4] = {q[k].x, q[k].y, q[k].z, q[k].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                s[2 * e] += __uint_as_float(w[e] << 16);
-                s[2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
+                s[k][2 * e] += __uint_as_float(w[e] << 16);
+                s[k][2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
             }
         }
+    }
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
+    for (int e = 0; e < 8; ++e) {
+        float t = (s[0][e] + s[1][e]) + (s[2][e] + s[3][e]);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
-        if (lane == 0)
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) red[sub][ch * 8 + e] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < C)
+        partial[static_cast<int64_t>(blockIdx.x) * nparams + wparams + threadIdx.x] =
+            (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
+}
+
+// ---------------------------------------------------------------------------
+// weight gradients of the one-channel layers (CUDA cores).  Both are the
+// correlation of a scalar volume s with a C-channel volume h,
+//   A[i][c] = sum_u s[u + off(i)] h[u][c],
+// the first layer's with its input and output gradient (tap i), the last
+// layer's with its output gradient and input (tap T - 1 - i).  One persistent
+// CTA per SM; a warp owns one 8-channel chunk and one tap plane (9 taps) for the
+// whole launch and keeps its 72 sums in registers: per 32 voxels it loads 16
+// bytes a lane, reads 9 scalars from the shared halo (double buffered, rows 16
+// banks apart) and issues 36 packed multiply-adds, which bound it.  4 x 48^3
+// voxels, 48 channels: a thread per tap and channel group walking the tile in
+// shared memory took 445 us (last layer) and 158 us (first).
+// ---------------------------------------------------------------------------
+template <int ND, int C>
+struct EdgeTile {
+    static constexpr int chunks = C / 8, planes = ND == 3 ? 3 : 1;
+    static constexpr int vs = ND == 3 ? 1 : 2;  // warps that share a tile's voxels
+    static constexpr int warps = chunks * planes * vs, threads = 32 * warps;
+    static constexpr int pitch = 48;            // >= hx, 16 modulo 32
+    static constexpr int buf = Tile<ND>::hz * Tile<ND>::hy * pitch;
+};
+
+// partial[cta][p]: p = t * C + c for the weights, then T * C + c (FIRST) or
+// T * C (last layer) for the bias
+template <int ND, int C, bool FIRST>
+__global__ void __launch_bounds__(EdgeTile<ND, C>::threads, 1) edge_wgrad_kernel(const float* __restrict__ scalar,
+                                                                                const bf16* __restrict__ h,
+                                                                                float* __restrict__ partial, NetGeo g,
+                                                                                int64_t ntiles) {
+    using TL = Tile<ND>;
+    using ET = EdgeTile<ND, C>;
+    constexpr int T = TL::taps, np = T * C + (FIRST ? C : 1);
+    constexpr int kPer = (TL::halo + ET::threads - 1) / ET::threads;
+    __shared__ float buf[2][ET::buf];
+    __shared__ float red[ET::vs][np];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int chunk = warp % ET::chunks, plane = (warp / ET::chunks) % ET::planes;
+    const int share = warp / (ET::chunks * ET::planes);
+    const int tiles_x = (g.W + TL::tx - 1) / TL::tx;
+    const int tiles_y = (g.H + TL::ty - 1) / TL::ty;
+    const int tiles_z = (g.D + TL::tz - 1) / TL::tz;
+    const int64_t nv = g.voxels();
+    const uint4* hc = reinterpret_cast<const uint4*>(h + static_cast<int64_t>(chunk) * nv * 8);
+    auto decode = [&](int64_t r, int& b, int& z0, int& y0, int& x0) {
+        x0 = static_cast<int>(r % tiles_x) * TL::tx;
+        r /= tiles_x;
+        y0 = static_cast<int>(r % tiles_y) * TL::ty;
+        r /= tiles_y;
+        z0 = static_cast<int>(r % tiles_z) * TL::tz;
+        b = static_cast<int>(r / tiles_z);
+    };
+    float next[kPer];
+    auto fetch = [&](int64_t tile) {
+        int b, z0, y0, x0;
+        decode(tile, b, z0, y0, x0);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) red[warp][e] = s[e];
-        __syncthreads();
-        if (threadIdx.x < 8) {
-            float t = 0.0f;
-            for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += red[w][threadIdx.x];
-            partial[static_cast<int64_t>(blockIdx.x) * nparams + wparams + ch * 8 + threadIdx.x] = t;
+        for (int k = 0; k < kPer; ++k) {
+            const int j = tid + k * ET::threads;
+            const int hx = j % TL::hx, hy = (j / TL::hx) % TL::hy, hz = j / (TL::hx * TL::hy);
+            const int x = x0 + hx - 1, y = y0 + hy - 1, z = ND == 3 ? z0 + hz - 1 : z0;
+            const bool in = j < TL::halo && x >= 0 && x < g.W && y >= 0 && y < g.H && z >= 0 && z < g.D;
+            next[k] = in ? __ldg(scalar + vox_index(g, b, z, y, x)) : 0.0f;
         }
+    };
+    auto keep = [&](float* dst) {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int j = tid + k * ET::threads;
+            if (j < TL::halo) dst[(j / TL::hx) * ET::pitch + j % TL::hx] = next[k];
+        }
+    };
+    float2 acc[9][4], bsum[4];
+    float ssum = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        bsum[e] = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) acc[i][e] = make_float2(0.0f, 0.0f);
+    }
+    if (blockIdx.x < ntiles) {
+        fetch(blockIdx.x);
+        keep(buf[0]);
+    }
+    __syncthreads();
+    int it = 0;
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+        const bool more = tile + gridDim.x < ntiles;
+        if (more) fetch(tile + gridDim.x);
+        int b, z0, y0, x0;
+        decode(tile, b, z0, y0, x0);
+        const float* sb = buf[it & 1];
+#pragma unroll 2
+        for (int st = share; st < 8; st += ET::vs) {
+            const int m = st * 32 + lane;
+            const int mx = m % TL::tx, my = (m / TL::tx) % TL::ty, mz = m / (TL::tx * TL::ty);
+            const int x = x0 + mx, y = y0 + my, z = z0 + mz;
+            uint4 q = make_uint4(0, 0, 0, 0);
+            if (x < g.W && y < g.H && z < g.D) q = __ldg(hc + vox_index(g, b, z, y, x));
+            const float* sp = sb + ((ND == 3 ? mz + plane : 0) * TL::hy + my) * ET::pitch + mx;
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+            float2 c[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                c[e] = make_float2(__uint_as_float(w[e] << 16), __uint_as_float(w[e] & 0xffff0000u));
+#pragma unroll
+            for (int i = 0; i < 9; ++i) {
+                const float v = sp[(i / 3) * ET::pitch + i % 3];
+                if (!FIRST && i == 4) ssum += v;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[i][e] = __ffma2_rn(make_float2(v, v), c[e], acc[i][e]);
+            }
+            if (FIRST) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) bsum[e] = __fadd2_rn(bsum[e], c[e]);
+            }
+        }
+        if (more) keep(buf[(it + 1) & 1]);
         __syncthreads();
+    }
+    auto sum_lanes = [](float v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        const int t = FIRST ? plane * 9 + i : T - 1 - (plane * 9 + i);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float a0 = sum_lanes(acc[i][e].x), a1 = sum_lanes(acc[i][e].y);
+            if (lane == 0) {
+                red[share][t * C + chunk * 8 + 2 * e] = a0;
+                red[share][t * C + chunk * 8 + 2 * e + 1] = a1;
+            }
+        }
+    }
+    if (plane == ET::planes / 2) {  // its centre tap is the voxel itself
+        if (FIRST) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float a0 = sum_lanes(bsum[e].x), a1 = sum_lanes(bsum[e].y);
+                if (lane == 0) {
+                    red[share][T * C + chunk * 8 + 2 * e] = a0;
+                    red[share][T * C + chunk * 8 + 2 * e + 1] = a1;
+                }
+            }
+        } else if (chunk == 0) {
+            const float a0 = sum_lanes(ssum);
+            if (lane == 0) red[share][T * C] = a0;
+        }
+    }
+    __syncthreads();
+    for (int p = tid; p < np; p += ET::threads) {
+        float v = red[0][p];
+        if (ET::vs == 2) v += red[ET::vs - 1][p];
+        partial[static_cast<int64_t>(blockIdx.x) * np + p] = v;
     }
 }
 
 // ---------------------------------------------------------------------------
-// weight gradients (CUDA cores): per-CTA partial sums over a tile of 256
-// voxels, summed over CTAs by reduce_partials_kernel
+// C -> C weight gradients without tensor memory (CUDA cores): per-CTA partial
+// sums over a tile of 256 voxels, summed over CTAs by reduce_partials_kernel
 // ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ float to_f(T v);
-template <>
-__device__ __forceinline__ float to_f<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float to_f<bf16>(bf16 v) { return __bfloat162float(v); }
-
-template <int ND, int CIN, int COUT, typename TI, typename TG>
+template <int ND, int C>
 struct WgradSmem {
-    static constexpr size_t in_floats = static_cast<size_t>(Tile<ND>::halo) * CIN;
-    static constexpr size_t g_floats = 256 * static_cast<size_t>(COUT);
+    static constexpr size_t in_floats = static_cast<size_t>(Tile<ND>::halo) * C;
+    static constexpr size_t g_floats = 256 * static_cast<size_t>(C);
     static constexpr size_t bytes = (in_floats + g_floats) * 4;
 };
 
-// partial[cta][p]: p = (t * CIN + ci) * COUT + co for the weights, then
-// T * CIN * COUT + co for the bias
-template <int ND, int CIN, int COUT, typename TI, typename TG>
-__global__ void __launch_bounds__(256) wgrad_kernel(const TI* __restrict__ in, const TG* __restrict__ gout,
+// partial[cta][p]: p = (t * C + ci) * C + co for the weights, then T * C * C + co
+// for the bias
+template <int ND, int C>
+__global__ void __launch_bounds__(256) wgrad_kernel(const bf16* __restrict__ in, const bf16* __restrict__ gout,
                                                     float* __restrict__ partial, NetGeo g) {
     using TL = Tile<ND>;
     constexpr int T = TL::taps;
-    constexpr int BI = CIN >= 4 ? 4 : 1, BO = COUT >= 4 ? 4 : 1;
-    constexpr int nw_items = T * (CIN / BI) * (COUT / BO);
-    constexpr int nitems = nw_items + COUT / BO;
-    constexpr int nparams = T * CIN * COUT + COUT;
+    constexpr int BI = 4, BO = 4;
+    constexpr int nw_items = T * (C / BI) * (C / BO);
+    constexpr int nitems = nw_items + C / BO;
+    constexpr int nparams = T * C * C + C;
     extern __shared__ __align__(16) unsigned char smem[];
     float* sin = reinterpret_cast<float*>(smem);
-    float* sg = sin + static_cast<size_t>(TL::halo) * CIN;
+    float* sg = sin + static_cast<size_t>(TL::halo) * C;
     const int tiles_x = (g.W + TL::tx - 1) / TL::tx;
     const int tiles_y = (g.H + TL::ty - 1) / TL::ty;
     const int tiles_z = (g.D + TL::tz - 1) / TL::tz;
@@ -1282,22 +1441,22 @@ __global__ void __launch_bounds__(256) wgrad_kernel(const TI* __restrict__ in, c
     const int z0 = static_cast<int>(r % tiles_z) * TL::tz;
     const int b = static_cast<int>(r / tiles_z);
     const int64_t nv = g.voxels();
-    for (int j = threadIdx.x; j < TL::halo * CIN; j += blockDim.x) {
+    for (int j = threadIdx.x; j < TL::halo * C; j += blockDim.x) {
         const int c = j / TL::halo, vox = j - c * TL::halo;  // channel-major: coalesced reads
-        const int i = vox * CIN + c;
+        const int i = vox * C + c;
         const int hxi = vox % TL::hx, hyi = (vox / TL::hx) % TL::hy, hzi = vox / (TL::hx * TL::hy);
         const int xx = x0 + hxi - 1, yy = y0 + hyi - 1, zz = ND == 3 ? z0 + hzi - 1 : z0;
         float v = 0.0f;
         if (xx >= 0 && xx < g.W && yy >= 0 && yy < g.H && zz >= 0 && zz < g.D)
-            v = to_f<TI>(in[hid<CIN>(vox_index(g, b, zz, yy, xx), c, nv)]);
+            v = __bfloat162float(in[hid<C>(vox_index(g, b, zz, yy, xx), c, nv)]);
         sin[i] = v;
     }
-    for (int j = threadIdx.x; j < 256 * COUT; j += blockDim.x) {
+    for (int j = threadIdx.x; j < 256 * C; j += blockDim.x) {
         const int c = j / 256, m = j - c * 256;
         const int xx = x0 + m % TL::tx, yy = y0 + (m / TL::tx) % TL::ty, zz = z0 + m / (TL::tx * TL::ty);
         float v = 0.0f;
-        if (xx < g.W && yy < g.H && zz < g.D) v = to_f<TG>(gout[hid<COUT>(vox_index(g, b, zz, yy, xx), c, nv)]);
-        sg[m * COUT + c] = v;
+        if (xx < g.W && yy < g.H && zz < g.D) v = __bfloat162float(gout[hid<C>(vox_index(g, b, zz, yy, xx), c, nv)]);
+        sg[m * C + c] = v;
     }
     __syncthreads();
     float* out = partial + static_cast<int64_t>(blockIdx.x) * nparams;
@@ -1308,9 +1467,9 @@ __global__ void __launch_bounds__(256) wgrad_kernel(const TI* __restrict__ in, c
 #pragma unroll
             for (int o = 0; o < BO; ++o) acc[i][o] = 0.0f;
         if (item < nw_items) {
-            const int cob = item % (COUT / BO);
-            const int cib = (item / (COUT / BO)) % (CIN / BI);
-            const int t = item / ((COUT / BO) * (CIN / BI));
+            const int cob = item % (C / BO);
+            const int cib = (item / (C / BO)) % (C / BI);
+            const int t = item / ((C / BO) * (C / BI));
             int dz, dy, dx;
             tap_offsets<ND>(t, dz, dy, dx);
             for (int m = 0; m < 256; ++m) {
@@ -1319,9 +1478,9 @@ __global__ void __launch_bounds__(256) wgrad_kernel(const TI* __restrict__ in, c
                 const int vox = (hz * TL::hy + my + dy + 1) * TL::hx + mx + dx + 1;
                 float iv[BI], gv[BO];
 #pragma unroll
-                for (int i = 0; i < BI; ++i) iv[i] = sin[vox * CIN + cib * BI + i];
+                for (int i = 0; i < BI; ++i) iv[i] = sin[vox * C + cib * BI + i];
 #pragma unroll
-                for (int o = 0; o < BO; ++o) gv[o] = sg[m * COUT + cob * BO + o];
+                for (int o = 0; o < BO; ++o) gv[o] = sg[m * C + cob * BO + o];
 #pragma unroll
                 for (int i = 0; i < BI; ++i)
 #pragma unroll
@@ -1331,40 +1490,31 @@ __global__ void __launch_bounds__(256) wgrad_kernel(const TI* __restrict__ in, c
             for (int i = 0; i < BI; ++i)
 #pragma unroll
                 for (int o = 0; o < BO; ++o)
-                    out[(t * CIN + cib * BI + i) * COUT + cob * BO + o] = acc[i][o];
+                    out[(t * C + cib * BI + i) * C + cob * BO + o] = acc[i][o];
         } else {
             const int cob = item - nw_items;
             for (int m = 0; m < 256; ++m)
 #pragma unroll
-                for (int o = 0; o < BO; ++o) acc[0][o] += sg[m * COUT + cob * BO + o];
+                for (int o = 0; o < BO; ++o) acc[0][o] += sg[m * C + cob * BO + o];
 #pragma unroll
-            for (int o = 0; o < BO; ++o) out[T * CIN * COUT + cob * BO + o] = acc[0][o];
+            for (int o = 0; o < BO; ++o) out[T * C * C + cob * BO + o] = acc[0][o];
         }
     }
 }
 
 // Sums the per-CTA partial records into the gradient.  Block b owns the 32
 // parameters 32 b .. 32 b + 31 (lane = parameter, coalesced 128-byte rows);
-// warp w adds the records w, w + 32, ... of the range, and the warps' sums are
-// added in warp order, so the result does not depend on timing.  With cpg > 0
-// (tensor-core weight gradients) parameter p < wparams is summed over the cpg
-// records of its tap group, p / group_params; otherwise over all records.
+// warp w adds the records w, w + 32, ..., and the warps' sums are added in warp
+// order, so the result does not depend on timing.
 __global__ void __launch_bounds__(1024) reduce_partials_kernel(const float* __restrict__ partial, int64_t nparts,
-                                                               int64_t nparams, float* __restrict__ grad, int cpg,
-                                                               int64_t group_params, int64_t wparams) {
+                                                               int64_t nparams, float* __restrict__ grad) {
     __shared__ float red[32][33];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t p0 = static_cast<int64_t>(blockIdx.x) * 32;
-    const int64_t p = p0 + lane;
-    int64_t c0 = 0, c1 = nparts;
-    if (cpg > 0 && p0 < wparams) {  // group_params and wparams are multiples of 32
-        c0 = (p0 / group_params) * cpg;
-        c1 = c0 + cpg;
-    }
+    const int64_t p = static_cast<int64_t>(blockIdx.x) * 32 + lane;
     float s = 0.0f;
     if (p < nparams) {
-        int64_t c = c0 + warp;
-        for (; c + 96 < c1; c += 128) {
+        int64_t c = warp;
+        for (; c + 96 < nparts; c += 128) {
             const float a0 = partial[c * nparams + p], a1 = partial[(c + 32) * nparams + p];
             const float a2 = partial[(c + 64) * nparams + p], a3 = partial[(c + 96) * nparams + p];
             s += a0;
@@ -1372,7 +1522,7 @@ __global__ void __launch_bounds__(1024) reduce_partials_kernel(const float* __re
             s += a2;
             s += a3;
         }
-        for (; c < c1; c += 32) s += partial[c * nparams + p];
+        for (; c < nparts; c += 32) s += partial[c * nparams + p];
     }
     red[warp][lane] = s;
     __syncthreads();
@@ -1381,6 +1531,40 @@ __global__ void __launch_bounds__(1024) reduce_partials_kernel(const float* __re
         for (int w = 0; w < 32; ++w) t += red[w][lane];
         if (p < nparams) grad[p] = t;
     }
+}
+
+// The same for the tensor-core weight gradients: parameter p < wparams is
+// summed over the cpg records of its tap group, p / group_params, one thread
+// each and ten loads in flight (50 records of 62 K parameters; a block of 1024
+// threads per 32 parameters, most of them with one load or none, took 14 us);
+// a bias, over all nparts records by the lanes of a warp.  The order is fixed.
+__global__ void __launch_bounds__(256) reduce_groups_kernel(const float* __restrict__ partial, int nparts,
+                                                            int64_t nparams, float* __restrict__ grad, int cpg,
+                                                            int64_t group_params, int64_t wparams, int wblocks) {
+    if (static_cast<int>(blockIdx.x) < wblocks) {
+        const int64_t p = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+        if (p >= wparams) return;
+        const float* src = partial + (p / group_params) * cpg * nparams + p;
+        float s = 0.0f;
+        int c = 0;
+        for (; c + 10 <= cpg; c += 10) {
+            float a[10];
+#pragma unroll
+            for (int k = 0; k < 10; ++k) a[k] = src[(c + k) * nparams];
+            s += ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7])) + (a[8] + a[9]);
+        }
+        for (; c < cpg; ++c) s += src[c * nparams];
+        grad[p] = s;
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    const int64_t p = wparams + (static_cast<int64_t>(blockIdx.x) - wblocks) * 8 + (threadIdx.x >> 5);
+    if (p >= nparams) return;
+    float s = 0.0f;
+    for (int c = lane; c < nparts; c += 32) s += partial[c * nparams + p];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) grad[p] = s;
 }
 
 __global__ void round_bf16_kernel(const float* __restrict__ src, float* __restrict__ dst, int64_t n) {
@@ -1788,19 +1972,36 @@ int32_t forward_impl(const NetPlan& P, const unsigned char* packed, const float*
     return BMND_OK;
 }
 
-template <int ND, int CIN, int COUT, typename TI, typename TG>
-int32_t run_wgrad(const TI* in, const TG* gout, float* partial, float* grad, int64_t tiles, NetGeo g,
+template <int ND, int C>
+int32_t run_wgrad(const bf16* in, const bf16* gout, float* partial, float* grad, int64_t tiles, NetGeo g,
                   cudaStream_t stream) {
-    using S = WgradSmem<ND, CIN, COUT, TI, TG>;
-    auto kernel = wgrad_kernel<ND, CIN, COUT, TI, TG>;
+    using S = WgradSmem<ND, C>;
+    auto kernel = wgrad_kernel<ND, C>;
     int sms = 0, per_sm = 0;
     if (int32_t rc = kernel_residency(reinterpret_cast<const void*>(kernel), 256, S::bytes, false, &per_sm, &sms))
         return rc;
     kernel<<<static_cast<unsigned>(tiles), 256, S::bytes, stream>>>(in, gout, partial, g);
     BMND_LAUNCH_CHECK("wgrad_kernel");
-    constexpr int64_t np = static_cast<int64_t>(Tile<ND>::taps) * CIN * COUT + COUT;
-    reduce_partials_kernel<<<static_cast<unsigned>((np + 31) / 32), 1024, 0, stream>>>(partial, tiles, np, grad, 0,
-                                                                                      np, np);
+    constexpr int64_t np = static_cast<int64_t>(Tile<ND>::taps) * C * C + C;
+    reduce_partials_kernel<<<static_cast<unsigned>((np + 31) / 32), 1024, 0, stream>>>(partial, tiles, np, grad);
+    BMND_LAUNCH_CHECK("reduce_partials_kernel");
+    return BMND_OK;
+}
+
+// a one-channel layer: `scalar` is the first layer's input or the last one's output gradient
+template <int ND, int C, bool FIRST>
+int32_t run_edge_wgrad(const float* scalar, const bf16* h, float* partial, float* grad, int64_t tiles, NetGeo g,
+                       cudaStream_t stream) {
+    using ET = EdgeTile<ND, C>;
+    auto kernel = edge_wgrad_kernel<ND, C, FIRST>;
+    int sms = 0, per_sm = 0;
+    if (int32_t rc = kernel_residency(reinterpret_cast<const void*>(kernel), ET::threads, 0, false, &per_sm, &sms))
+        return rc;
+    const int64_t ctas = std::min<int64_t>(static_cast<int64_t>(sms) * (per_sm > 0 ? per_sm : 1), tiles);
+    kernel<<<static_cast<unsigned>(ctas), ET::threads, 0, stream>>>(scalar, h, partial, g, tiles);
+    BMND_LAUNCH_CHECK("edge_wgrad_kernel");
+    constexpr int64_t np = static_cast<int64_t>(Tile<ND>::taps) * C + (FIRST ? C : 1);
+    reduce_partials_kernel<<<static_cast<unsigned>((np + 31) / 32), 1024, 0, stream>>>(partial, ctas, np, grad);
     BMND_LAUNCH_CHECK("reduce_partials_kernel");
     return BMND_OK;
 }
@@ -1837,11 +2038,15 @@ int32_t run_wgrad_tc(const bf16* in, const bf16* gout, float* partial, int64_t c
     kernel<<<static_cast<unsigned>(nparts), WT::threads, WT::bytes, stream>>>(xmaps, ymaps, partial, np, g, err,
                                                                              g_wait_probe_ns);
     BMND_LAUNCH_CHECK("wgrad_tc_kernel");
-    bias_partial_kernel<C><<<static_cast<unsigned>(nparts), 256, 0, stream>>>(gout, g.voxels(), partial, np, wparams);
+    bias_partial_kernel<C><<<static_cast<unsigned>(nparts), C * 16, 0, stream>>>(gout, g.voxels(), partial, np,
+                                                                                wparams);
     BMND_LAUNCH_CHECK("bias_partial_kernel");
-    reduce_partials_kernel<<<static_cast<unsigned>((np + 31) / 32), 1024, 0, stream>>>(
-        partial, nparts, np, grad, static_cast<int>(cpg), static_cast<int64_t>(WT::taps_per_cta) * C * C, wparams);
-    BMND_LAUNCH_CHECK("reduce_partials_kernel");
+    constexpr int wblocks = static_cast<int>((wparams + 255) / 256);
+    reduce_groups_kernel<<<wblocks + C / 8, 256, 0, stream>>>(partial, static_cast<int>(nparts), np, grad,
+                                                              static_cast<int>(cpg),
+                                                              static_cast<int64_t>(WT::taps_per_cta) * C * C, wparams,
+                                                              wblocks);
+    BMND_LAUNCH_CHECK("reduce_groups_kernel");
     return BMND_OK;
 }
 
@@ -1865,7 +2070,7 @@ int32_t gradient_impl(const NetPlan& P, const unsigned char* packed, const float
     const int L = P.L;
     constexpr int64_t wg_params = static_cast<int64_t>(TL::taps) * C * C + C;  // one C -> C layer
     // last layer: weight gradient from h_{L-1} and gy, data gradient into h_{L-1}
-    rc = run_wgrad<ND, C, 1, bf16, float>(act(L - 2), B.gy, B.partial, grad + P.w_off[L - 1], tiles, g, stream);
+    rc = run_edge_wgrad<ND, C, false>(B.gy, act(L - 2), B.partial, grad + P.w_off[L - 1], tiles, g, stream);
     if (rc) return rc;
     int cur = 0;
     conv_out_dgrad_kernel<ND, C><<<eb, 256, 0, stream>>>(B.gy, wr + P.w_off[L - 1], act(L - 2), B.grad[cur], g);
@@ -1877,15 +2082,14 @@ int32_t gradient_impl(const NetPlan& P, const unsigned char* packed, const float
             rc = run_wgrad_tc<ND, C>(act(l - 1), B.grad[cur], B.partial, tiles * P.max_layer_params / wg_params,
                                      grad + P.w_off[l], g, B.err, stream);
         if (rc == BMND_ERR_UNSUPPORTED)
-            rc = run_wgrad<ND, C, C, bf16, bf16>(act(l - 1), B.grad[cur], B.partial, grad + P.w_off[l], tiles, g,
-                                                 stream);
+            rc = run_wgrad<ND, C>(act(l - 1), B.grad[cur], B.partial, grad + P.w_off[l], tiles, g, stream);
         if (rc) return rc;
         rc = run_layer<ND, C>(P, packed, l, true, B.grad[cur], nullptr, act(l - 1), B.grad[cur ^ 1], B, stream);
         if (rc) return rc;
         cur ^= 1;
     }
     // first layer: weight gradient only
-    return run_wgrad<ND, 1, C, float, bf16>(B.a, B.grad[cur], B.partial, grad + P.w_off[0], tiles, g, stream);
+    return run_edge_wgrad<ND, C, true>(B.a, B.grad[cur], B.partial, grad + P.w_off[0], tiles, g, stream);
 }
 
 template <typename F>
