@@ -62,6 +62,31 @@ def test_forward_and_gradient_match_oracle(cuda, engine, ndim, channels, layers,
         off += n
 
 
+@pytest.mark.parametrize("ndim,channels,shape", [
+    (3, 48, (2, 3, 9, 17)), (3, 32, (1, 2, 8, 16)), (3, 48, (1, 1, 1, 1)), (3, 32, (2, 5, 7, 33)),
+    (3, 48, (1, 4, 16, 30)), (2, 48, (1, 1, 3)), (2, 32, (2, 16, 15)), (2, 48, (3, 17, 49)), (2, 32, (1, 40, 34)),
+])
+def test_one_channel_layers_at_tile_edges(cuda, ndim, channels, shape):
+    """First and last layer at the edges of their 16 x 8 x 2 (2-D 16 x 16) tiles
+    and of the 4-voxel groups, against the oracle with the bound of the layer
+    test above (BF16 roundings that fall the other way)."""
+    rng = np.random.default_rng(sum(shape) + channels)
+    x = rng.poisson(rng.uniform(1, 30, size=shape)).astype(np.float32)
+    t = (0.7 * x + 2.0).astype(np.float32)
+    net, params = _net(cuda, ndim, channels, 3, seed=5)
+    loss, grad = net.gradient(cuda.from_numpy(x).cuda(), cuda.from_numpy(t).cuda())
+    net.check_status(training=True)
+    loss_o, grad_o, _ = R.loss_and_gradient(params, x, t, ndim, channels, 3, bf16=True)
+    assert abs(float(loss.item()) - loss_o) <= 1e-3 * loss_o + 1e-7
+    grad = grad.cpu().numpy().astype(np.float64)
+    off = 0
+    for layer, (taps, cin, cout) in enumerate(R.layer_shapes(ndim, channels, 3)):
+        n = taps * cin * cout + cout
+        rel = np.linalg.norm(grad[off:off + n] - grad_o[off:off + n]) / max(np.linalg.norm(grad_o[off:off + n]), 1e-12)
+        assert rel < 3e-2, (layer, rel)
+        off += n
+
+
 @pytest.mark.parametrize("ndim,channels,layers,shape", [
     (3, 48, 6, (2, 40, 70, 66)),    # thousands of tiles per launch, ragged x and y edges
     (2, 32, 5, (3, 300, 129)),
