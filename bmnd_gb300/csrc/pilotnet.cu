@@ -988,8 +988,12 @@ __global__ void __launch_bounds__(224, 1) conv_mid_tc_kernel(const __grid_consta
 // are discarded.  The CTAs split the taps into groups of 9, so one group's
 // accumulators (9 x C columns) fit the 512 columns of tensor memory, and each
 // CTA accumulates its share of the tiles for the whole launch; the per-CTA
-// sums are added by reduce_groups_kernel.  Roles: warp 0 issues the TMA
-// loads (two stages); one thread each of warps 1 and 2 issues the MMAs of the
+// sums are added by reduce_groups_kernel.  A group of 9 taps is one tap plane, so
+// a CTA loads only that plane of the input halo (all three, in two stages, made
+// the loads its bound: 64 KB per tile, 175 us per layer of 4 x 48^3 voxels and 48
+// channels; one plane, in four, 151).  A plane outside the volume is loaded from
+// a coordinate outside the tensor, as zeros.  Roles: warp 0 issues the TMA loads;
+// one thread each of warps 1 and 2 issues the MMAs of the
 // first 5 taps of the group and of the other 4 (one issuing thread cannot keep
 // the tensor core busy with MMAs this small); at the end warps 0-1 read
 // tensor-memory lanes 0-63.  Every mbarrier wait is bounded.
@@ -997,15 +1001,19 @@ __global__ void __launch_bounds__(224, 1) conv_mid_tc_kernel(const __grid_consta
 template <int ND, int C>
 struct WgTile {
     using TT = TcTile<ND, C>;
-    static constexpr int taps_per_cta = 9;
-    static constexpr int tsplit = 5;  // taps of the first issuing thread
+    static constexpr int taps_per_cta = 9;             // one tap plane
+    static constexpr int tsplit = 5;                   // taps of the first issuing thread
     static constexpr int groups = TT::taps / taps_per_cta;
-    static constexpr uint32_t xbytes = TT::tbytes;                                   // one input-halo stage
-    static constexpr uint32_t ybytes = TT::chunks * TT::tx * TT::ty * 16;            // one output-gradient stage
-    // A of stage 1 reads 16 chunk planes from its start (M = 128)
-    static constexpr uint32_t bytes = xbytes + 16 * TT::cbytes > 2 * (xbytes + ybytes)
-                                          ? xbytes + 16 * TT::cbytes
-                                          : 2 * (xbytes + ybytes);
+    static constexpr int stages = 4;
+    static constexpr int plane = TT::hx * TT::hy;      // voxels of a halo plane
+    static constexpr uint32_t cbytes = static_cast<uint32_t>((plane + 7) / 8 * 8) * 16;  // one chunk in shared memory
+    static constexpr uint32_t cbox = static_cast<uint32_t>(plane) * 16;                  // one chunk by TMA
+    static constexpr uint32_t xbytes = TT::chunks * cbytes;                              // one input-halo stage
+    static constexpr uint32_t ybytes = TT::chunks * TT::tx * TT::ty * 16;  // one output-gradient stage
+    // A of the last stage reads 16 chunk planes from its start (M = 128)
+    static constexpr uint32_t bytes = (stages - 1) * xbytes + 16 * cbytes > stages * (xbytes + ybytes)
+                                          ? (stages - 1) * xbytes + 16 * cbytes
+                                          : stages * (xbytes + ybytes);
     static constexpr uint32_t acc_cols = taps_per_cta * C;
     static constexpr int threads = 128;
 };
@@ -1018,7 +1026,8 @@ __global__ void __launch_bounds__(128, 1) wgrad_tc_kernel(const __grid_constant_
     using TT = TcTile<ND, C>;
     using WT = WgTile<ND, C>;
     extern __shared__ __align__(128) unsigned char wg_smem[];
-    __shared__ __align__(8) uint64_t bars[6];  // full[2], empty[2], done, never
+    constexpr int S = WT::stages;
+    __shared__ __align__(8) uint64_t bars[2 * S + 2];  // full[S], empty[S], done, never
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     volatile int* abort_v = &abort_flag;
@@ -1026,18 +1035,18 @@ __global__ void __launch_bounds__(128, 1) wgrad_tc_kernel(const __grid_constant_
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(wg_smem));
     // stage s: the input halo at xs(s), the output gradient at ys(s)
     auto xs = [&](int st) { return sbase + static_cast<uint32_t>(st) * WT::xbytes; };
-    auto ys = [&](int st) { return sbase + 2 * WT::xbytes + static_cast<uint32_t>(st) * WT::ybytes; };
+    auto ys = [&](int st) { return sbase + S * WT::xbytes + static_cast<uint32_t>(st) * WT::ybytes; };
     const uint32_t bar0 = static_cast<uint32_t>(__cvta_generic_to_shared(bars));
     auto full = [&](int st) { return bar0 + 8u * st; };
-    auto empty = [&](int st) { return bar0 + 16u + 8u * st; };
-    const uint32_t done = bar0 + 32u, never = bar0 + 40u;
+    auto empty = [&](int st) { return bar0 + 8u * (S + st); };
+    const uint32_t done = bar0 + 16u * S, never = bar0 + 16u * S + 8u;
     constexpr uint64_t kWaitNs = 1000000000ull;
     const int cpg = static_cast<int>(gridDim.x) / WT::groups;  // CTAs per tap group
     const int group = static_cast<int>(blockIdx.x) / cpg;
     const int gidx = static_cast<int>(blockIdx.x) - group * cpg;
 
     if (tid == 0) {
-        for (int st = 0; st < 2; ++st) {
+        for (int st = 0; st < S; ++st) {
             mbar_init(full(st), 1);
             mbar_init(empty(st), 2);  // one commit per issuing thread
         }
@@ -1087,79 +1096,58 @@ __global__ void __launch_bounds__(128, 1) wgrad_tc_kernel(const __grid_constant_
         if (lane == 0 && !*abort_v) {
             int it = 0;
             for (int64_t tl = gidx; tl < ntiles; tl += cpg, ++it) {
-                const int st = it & 1;
-                if (!mbar_wait(empty(st), ((it >> 1) & 1) ^ 1, kWaitNs)) {
+                const int st = it % S;
+                if (!mbar_wait(empty(st), ((it / S) & 1) ^ 1, kWaitNs)) {
                     fail(1);
                     break;
                 }
                 if (*abort_v) break;
                 int b, z0, y0, x0;
                 decode(tl, b, z0, y0, x0);
-                mbar_expect_tx(full(st), TT::chunks * (TT::box_bytes + TT::tx * TT::ty * 16));
+                mbar_expect_tx(full(st), TT::chunks * (WT::cbox + TT::tx * TT::ty * 16));
+                // the tap plane's input plane; outside the volume (the next one of the batch
+                // begins there) a coordinate outside the tensor reads as zero
+                const int zi = z0 + group - 1;
+                const int zx = ND != 3 ? b : (zi >= 0 && zi < g.D ? b * g.D + zi : -1);
 #pragma unroll
                 for (int ch = 0; ch < TT::chunks; ++ch) {
-                    tma_load_3d(xs(st) + ch * TT::cbytes, &xmaps.m[ch], 8 * (x0 - 1), y0 - 1,
-                                ND == 3 ? b * g.D + z0 - 1 : b, full(st));
+                    tma_load_3d(xs(st) + ch * WT::cbytes, &xmaps.m[ch], 8 * (x0 - 1), y0 - 1, zx, full(st));
                     tma_load_3d(ys(st) + ch * (TT::tx * TT::ty * 16), &ymaps.m[ch], 8 * x0, y0,
                                 ND == 3 ? b * g.D + z0 : b, full(st));
                 }
                 issued = it + 1;
             }
             if (*abort_v) {
-                // copies in flight: wait (bounded) for the last two stages
-                for (int j = issued - 2; j < issued; ++j)
-                    if (j >= 0) (void)mbar_wait(full(j & 1), (j >> 1) & 1, kWaitNs);
+                // copies in flight: wait (bounded) for the last stages
+                for (int j = issued - S; j < issued; ++j)
+                    if (j >= 0) (void)mbar_wait(full(j % S), (j / S) & 1, kWaitNs);
             }
         }
         __syncwarp();
     } else if (warp == 1 || warp == 2) {
-        // ---- MMA issuers; each warp zeroes the batch-boundary planes before
-        // its own MMAs (both write the same zeros) ----
+        // ---- MMA issuers ----
         const int t_lo = warp == 1 ? 0 : WT::tsplit, t_hi = warp == 1 ? WT::tsplit : WT::taps_per_cta;
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                                    (static_cast<uint32_t>(C >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
         int it = 0;
         for (int64_t tl = gidx; !*abort_v && tl < ntiles; tl += cpg, ++it) {
-            const int st = it & 1;
+            const int st = it % S;
             bool got = true;
-            if (lane == 0) got = mbar_wait(full(st), (it >> 1) & 1, kWaitNs);
+            if (lane == 0) got = mbar_wait(full(st), (it / S) & 1, kWaitNs);
             got = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
             if (!got || *abort_v) {
                 if (lane == 0 && !got) fail(1);
                 break;
             }
-            if (ND == 3 && g.nb > 1) {
-                // planes of the neighbouring volume in the batch read as zero padding
-                int b, z0, y0, x0;
-                decode(tl, b, z0, y0, x0);
-                const bool below = z0 == 0 && b > 0, above = z0 == g.D - 1 && b < g.nb - 1;
-                if (below || above) {
-                    constexpr int pv = TT::hx * TT::hy;
-                    for (int plane = 0; plane < 3; plane += 2) {
-                        if (plane == 0 ? !below : !above) continue;
-                        for (int i = lane; i < TT::chunks * pv; i += 32) {
-                            const int ch = i / pv, v = plane * pv + i % pv;
-                            const uint32_t a = xs(st) + ch * TT::cbytes + static_cast<uint32_t>(v) * 16u;
-                            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};\n" ::"r"(a), "r"(0) : "memory");
-                        }
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                    __syncwarp();
-                }
-            }
             tc_fence_after();
             if (lane == 0) {
                 // A: MN-major, SBO = chunk plane (next 8 input channels), LBO = halo row (next 8 voxels)
-                const uint64_t a_base = umma_desc(xs(st), TT::hx * 16, TT::cbytes);
+                const uint64_t a_base = umma_desc(xs(st), TT::hx * 16, WT::cbytes);
                 // B: MN-major, SBO = chunk plane of the gradient tile, LBO = one tile row (128 bytes)
                 const uint64_t b_base = umma_desc(ys(st), 128, TT::tx * TT::ty * 16);
 #pragma unroll 1
                 for (int tt = t_lo; tt < t_hi; ++tt) {
-                    const int t = group * WT::taps_per_cta + tt;
-                    const int dz = ND == 3 ? t / 9 : 0;
-                    const int dy = ND == 3 ? (t / 3) % 3 : t / 3;
-                    const int dx = t % 3;
-                    const int vox0 = (dz * TT::hy + dy) * TT::hx + dx;
+                    const int vox0 = (tt / 3) * TT::hx + tt % 3;
                     const uint32_t d_tmem = tmem + static_cast<uint32_t>(tt * C);
 #pragma unroll
                     for (int ks = 0; ks < TT::ty / 2; ++ks) {
@@ -2060,7 +2048,7 @@ int32_t run_wgrad_tc(const bf16* in, const bf16* gout, float* partial, int64_t c
     if (cpg * WT::groups > capacity) cpg = capacity / WT::groups;
     if (cpg < 1) return BMND_ERR_UNSUPPORTED;
     TcMaps xmaps, ymaps;
-    const uint32_t xbox[3] = {TT::hx, TT::hy, TT::hz};
+    const uint32_t xbox[3] = {TT::hx, TT::hy, 1};
     const uint32_t ybox[3] = {TT::tx, TT::ty, 1};
     if (int32_t rc = encode_chunk_maps(in, g, C, xbox, xmaps)) return rc;
     if (int32_t rc = encode_chunk_maps(gout, g, C, ybox, ymaps)) return rc;
