@@ -119,7 +119,7 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     const bool wiener = sp.filter == BMND_FILTER_WIENER;
     const int kpad = (kmax + 3) / 4 * 4;
     L.g = take(4 * nmax * nmax);
-    L.gt2 = take(8 * nmax * (kpad > 0 ? kpad : 4));  // exact planes' G entries in pairs (g, g) for packed products
+    L.gt2 = take(kpad > 0 ? 8 * nmax * kpad : 16);  // exact planes' G entries in pairs (g, g) for packed products
     L.fw = take(4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE);
     L.fi = take(4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE);
     // group-mass conservation: transposed inverse spatial matrices, and the
@@ -144,7 +144,7 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     // Gaussian noise: covariance-map row of every member pair (i > j)
     const bool gauss = sp.noise_model == BMND_NOISE_GAUSSIAN;
     L.lag = take(gauss && kmax > 0 ? 4 * static_cast<int64_t>(nmax) * ((nmax + 3) / 4 * 4) : 16);
-    L.scan = take(8 * (kThreads + 1));
+    L.scan = take(8 * (kThreads / 32 + 1));  // the warps' totals, then the block's
     L.plane = take(8 * (nmax > 40 ? nmax : 40));  // also the mass phase's 8 warps x 5 sums
     L.wts = take(4 * nmax);
     L.misc = take(64);
@@ -1586,8 +1586,8 @@ __device__ __forceinline__ void gauss_haar(const float* __restrict__ cm, const i
     }
 }
 
-// One group, by a whole CTA.
-template <int ND, int B0, int B1, int B2>
+// One group, by a whole CTA.  APPROX: no exact planes (variance_k = 0).
+template <int ND, int B0, int B1, int B2, bool APPROX>
 __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char* smem, int64_t gid) {
     using GM = Geom<ND, B0, B1, B2>;
     const BmndStageParams& sp = a.sp;
@@ -1626,9 +1626,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     float* wts = sm<float>(smem, a.L.wts);
     int* misc = sm<int>(smem, a.L.misc);
 
-    const int k = sp.variance_k;
+    const int k = APPROX ? 0 : sp.variance_k;
     const int kk = k < n ? k : n;
-    const int kpad = (a.kmax + 3) / 4 * 4;
+    const int kpad = APPROX ? 0 : (a.kmax + 3) / 4 * 4;
 
     // ---- setup: constants of the launch, positions, group matrix ----
     {
@@ -1946,13 +1946,13 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
                 } while (m);
             });
             if (tid == 0) {
-                scan[blockDim.x] = make_int2(static_cast<int>(all >> 16), static_cast<int>(all & 0xffffu));
+                scan[kThreads / 32] = make_int2(static_cast<int>(all >> 16), static_cast<int>(all & 0xffffu));
                 lent[all & 0xffffu] = lent[(all & 0xffffu) + 1] = quarters ? 0u : gt2_off;  // read ahead, never used
             }
         }
         __syncthreads();
-        U = scan[blockDim.x].x;
-        if (tid == 0) lstart[U] = scan[blockDim.x].y;
+        U = scan[kThreads / 32].x;
+        if (tid == 0) lstart[U] = scan[kThreads / 32].y;
         __syncthreads();
         // variance of every union voxel, all loads in flight together
         for (int u = tid; u < U; u += blockDim.x) {
@@ -2390,12 +2390,13 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
 // registers and 38 KB (16 members) or 56 KB (32) allow four for patches of 64
 // elements (against three: 75.1 -> 72.3 ms for 0.93 M groups of 8x8, 3.56 -> 3.38
 // ms for 42 K groups of 4x4x4, 14.3 -> 12.6 ms for a Gaussian image); 5x5x5
-// patches hold three.
-template <int ND, int B0, int B1, int B2, int NT>
-__global__ void __launch_bounds__(NT, NT != kThreads ? 1 : ND == 2 || B0 == 4 ? 4 : ND == 3 ? 3 : 2)
+// patches hold three, and four where there are no exact planes (55 KB; 17.2 ->
+// 14.8 ms for 250 K groups).
+template <int ND, int B0, int B1, int B2, int NT, bool APPROX = false>
+__global__ void __launch_bounds__(NT, NT != kThreads ? 1 : ND == 2 || B0 == 4 || APPROX ? 4 : ND == 3 ? 3 : 2)
     group_filter_kernel(FilterArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    filter_group<ND, B0, B1, B2>(a, smem, blockIdx.x);
+    filter_group<ND, B0, B1, B2, APPROX>(a, smem, blockIdx.x);
 }
 
 // S^T[p * stride + j] = S[j, p] with S = kron(F_0, ..., F_{nd-1}) built axis by
@@ -2591,7 +2592,8 @@ int32_t launch_group_filter(const BmndStageParams& sp, const float* noisy, const
     if (sp.ndim == 3 && b[0] == 4 && b[1] == 4 && b[2] == 4)
         return run(group_filter_kernel<3, 4, 4, 4, kThreads>, kThreads);
     if (sp.ndim == 3 && b[0] == 5 && b[1] == 5 && b[2] == 5)
-        return run(group_filter_kernel<3, 5, 5, 5, kThreads>, kThreads);
+        return sp.variance_k > 0 ? run(group_filter_kernel<3, 5, 5, 5, kThreads>, kThreads)
+                                 : run(group_filter_kernel<3, 5, 5, 5, kThreads, true>, kThreads);
     return run(group_filter_kernel<0, 0, 0, 0, kThreads>, kThreads);
 }
 
