@@ -1335,7 +1335,7 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
     const int64_t n_lins = static_cast<int64_t>(b.cnt[0]) * b.cnt[1] * b.cnt[2];
     // the shared terms pay off while references are dense: up to one per 64
     // origins (the schedules have one per 4.5 to 27)
-    if (b.rowlen > (1 << 20) || a.n_refs * 64 < n_lins) return BMND_OK;
+    if (b.rowlen > (1 << 20) || a.n_refs * 64 < n_lins || a.n_refs > 0x7fffffffLL) return BMND_OK;
     // Few references of a stage on counts: the kernel of tabulated terms has no
     // phases that wait on each other.  One GB300, that kernel against this file's:
     // 64 x 64 34 against 115 us, 140 x 140 (3.9 K references) 164 against 169,
