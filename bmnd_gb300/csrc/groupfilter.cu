@@ -1546,7 +1546,7 @@ __device__ __forceinline__ void gauss_haar(const float* __restrict__ cm, const i
         for (int j = j0; j < j1; j += 8) {
             float cv[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) cv[u] = j + u < j1 ? __ldg(cc + row[j + u]) : 0.0f;
+            for (int u = 0; u < 8; ++u) cv[u] = j + u < j1 ? __ldg(cc + static_cast<int64_t>(row[j + u]) * P) : 0.0f;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 if (j + u < j1) {
@@ -1766,7 +1766,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         // exact planes g < kk: sum_{i,j} G[g,i] G[g,j] C_c((x_i - x_j) mod domain),
         // C_c the covariance map of spatial coefficient c; the other planes
         // share what is left of n times the patch variance C_c(0)
-        int* lag = sm<int>(smem, a.L.lag);  // lag[i * lrow + j]: first element of the pair's map row
+        // lag[i * lrow + j]: the pair's map row; rows x P may exceed 32 bits (a lag
+        // domain of 258^3 and 125 coefficients do), so offsets are formed in 64
+        int* lag = sm<int>(smem, a.L.lag);
         const int lrow = (n + 3) / 4 * 4;
         if (kk > 0) {
             for (int q = tid; q < n * n; q += blockDim.x) {
@@ -1779,7 +1781,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
                     if (l < 0) l += D;
                     flat = flat * D + l;
                 }
-                lag[i * lrow + j] = flat * P;
+                lag[i * lrow + j] = flat;
             }
             __syncthreads();
         }
@@ -1800,7 +1802,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
                     for (int j = 0; j < i; ++j) {
                         const float wj = Gr[j];
                         if (wj == 0.0f) continue;
-                        const float cv = __ldg(cm + lag[i * lrow + j] + c);
+                        const float cv = __ldg(cm + static_cast<int64_t>(lag[i * lrow + j]) * P + c);
                         value = add_rn(value, mul_rn(mul_rn(wi, wj), add_rn(cv, cv)));
                     }
                 }
