@@ -56,6 +56,7 @@ struct Layout {
     int64_t g, gt2, fw, fi, fit, dir, win, mdiag, voff, kron, pos, org0, shf, shl, sg, ex, part, lag, uni, s, x, r, v, grid, lval,
         lstart, lent, scan, plane, wts, misc, risk, total;
     int32_t part_over;  // the exact phase's partial sums overwrite its lists
+    int32_t kron_used;  // S^T is copied to `kron`
 };
 
 struct FilterArgs {
@@ -86,8 +87,21 @@ struct FilterArgs {
     AggStore store;      // deterministic aggregation: rows of the entry store, or store.store == null
 };
 
-__host__ __device__ inline bool kron_in_smem(const BmndStageParams& sp, int P, int kmax) {
-    return kron_jr(P) == 2 && kmax > 0 && sp.noise_model == BMND_NOISE_POISSON;
+// Whether launch_group_filter takes an instantiation for the patch shape
+__host__ inline bool specialised_shape(const BmndStageParams& sp) {
+    const int32_t* b = sp.block;
+    if (sp.exact_risk_weights) return false;
+    if (sp.ndim == 2) return b[0] == 8 && b[1] == 8;
+    return sp.ndim == 3 && b[0] == b[1] && b[0] == b[2] && (b[0] == 4 || b[0] == 5);
+}
+// S^T of patches of 33-64 voxels (16 KB) lies in shared memory for the Haar form
+// of the exact phase (exact_haar), which reads it with 32-bit addresses and no L1
+// tags; the other forms read the table in global memory, so a copy would only
+// take residency (8x8 patches of a 384 x 416 image, 16 exact planes: stage 1 takes
+// 8.2 ms without it, 10.6 with it; stage 2 18.0 against 20.8)
+__host__ inline bool kron_in_smem(const BmndStageParams& sp, int P, int kmax) {
+    return specialised_shape(sp) && kron_jr(P) == 2 && kmax > 0 && sp.variance_k <= 4 &&
+           sp.noise_model == BMND_NOISE_POISSON && sp.group_transform == BMND_GROUP_HAAR;
 }
 
 // The group buffers (S, X, R, V, SG) of 8x8 patches keep one spare word after
@@ -101,8 +115,7 @@ __host__ __device__ __forceinline__ constexpr int padded(int p) {
     return LB == 8 ? p + p / 8 : p;
 }
 __host__ inline int64_t padded_patch(const BmndStageParams& sp, int P) {
-    const int32_t* b = sp.block;
-    return sp.ndim == 2 && b[0] == 8 && b[1] == 8 && !sp.exact_risk_weights ? padded<8>(P) : P;
+    return sp.ndim == 2 && specialised_shape(sp) ? padded<8>(P) : P;
 }
 
 __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax, int64_t ucells, bool sigma) {
@@ -130,9 +143,8 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.win = take(4 * P);
     L.mdiag = take(sp.windowed_synthesis ? 8 * P : 16);
     L.voff = take(4 * P);
-    // S^T of patches of 33-64 voxels (16 KB): the exact phase reads it with
-    // 32-bit addresses and no L1 tags
-    L.kron = take(kron_in_smem(sp, P, kmax) ? 4 * static_cast<int64_t>(P) * kron_stride(P) : 16);
+    L.kron_used = kron_in_smem(sp, P, kmax);
+    L.kron = take(L.kron_used ? 4 * static_cast<int64_t>(P) * kron_stride(P) : 16);
     L.pos = take(4 * nmax * BMND_MAX_DIMS);
     L.org0 = take(4 * nmax);
     L.shf = take(4 * nmax * BMND_MAX_DIMS);
@@ -1629,7 +1641,6 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     const int k = APPROX ? 0 : sp.variance_k;
     const int kk = k < n ? k : n;
     const int kpad = APPROX ? 0 : (a.kmax + 3) / 4 * 4;
-
     // ---- setup: constants of the launch, positions, group matrix ----
     {
         float* Fi = sm<float>(smem, a.L.fi);
@@ -1667,7 +1678,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         }
         if (sp.windowed_synthesis)  // the only reader of the metric diagonal
             for (int e = tid; e < P; e += blockDim.x) mdiag[e] = sp.spatial_metric_diag[e];
-        if (kron_in_smem(sp, P, kmax)) {
+        if (ND > 0 && a.L.kron_used) {
             float4* kron = sm<float4>(smem, a.L.kron);
             const int words = P * kron_stride(P) / 4;
             for (int e = tid; e < words; e += blockDim.x) kron[e] = __ldg(reinterpret_cast<const float4*>(a.st) + e);
@@ -2588,15 +2599,11 @@ int32_t launch_group_filter(const BmndStageParams& sp, const float* noisy, const
         BMND_LAUNCH_CHECK("group_filter_kernel");
         return BMND_OK;
     };
-    const int* b = sp.block;
-    if (sp.exact_risk_weights) return run(group_filter_kernel<0, 0, 0, 0, kThreads>, kThreads);
-    if (sp.ndim == 2 && b[0] == 8 && b[1] == 8) return run(group_filter_kernel<2, 8, 8, 1, kThreads>, kThreads);
-    if (sp.ndim == 3 && b[0] == 4 && b[1] == 4 && b[2] == 4)
-        return run(group_filter_kernel<3, 4, 4, 4, kThreads>, kThreads);
-    if (sp.ndim == 3 && b[0] == 5 && b[1] == 5 && b[2] == 5)
-        return sp.variance_k > 0 ? run(group_filter_kernel<3, 5, 5, 5, kThreads>, kThreads)
-                                 : run(group_filter_kernel<3, 5, 5, 5, kThreads, true>, kThreads);
-    return run(group_filter_kernel<0, 0, 0, 0, kThreads>, kThreads);
+    if (!specialised_shape(sp)) return run(group_filter_kernel<0, 0, 0, 0, kThreads>, kThreads);
+    if (sp.ndim == 2) return run(group_filter_kernel<2, 8, 8, 1, kThreads>, kThreads);
+    if (sp.block[0] == 4) return run(group_filter_kernel<3, 4, 4, 4, kThreads>, kThreads);
+    return sp.variance_k > 0 ? run(group_filter_kernel<3, 5, 5, 5, kThreads>, kThreads)
+                             : run(group_filter_kernel<3, 5, 5, 5, kThreads, true>, kThreads);
 }
 
 int32_t launch_finalize_sigma(const BmndStageParams& sp, const double* sig_num, const double* den,
