@@ -130,9 +130,16 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     const int64_t np = static_cast<int64_t>(nmax) * P;
     const int64_t npp = static_cast<int64_t>(nmax) * padded_patch(sp, P);
     const bool wiener = sp.filter == BMND_FILTER_WIENER;
+    const bool gauss = sp.noise_model == BMND_NOISE_GAUSSIAN;
+    const bool keep = sp.exact_risk_weights != 0;
+    // exact planes' G entries in pairs (g, g) for packed products: the exact risk
+    // reads them after the shrinkage, the exact variance before (they may lie behind
+    // its lists, see below), stationary Gaussian noise without it never
+    const bool early = keep || specialised_shape(sp);  // the entries count from the start of shared memory
     const int kpad = (kmax + 3) / 4 * 4;
+    const int64_t gt2_bytes = 8 * static_cast<int64_t>(nmax) * kpad;
     L.g = take(4 * nmax * nmax);
-    L.gt2 = take(kpad > 0 ? 8 * nmax * kpad : 16);  // exact planes' G entries in pairs (g, g) for packed products
+    if (early) L.gt2 = take(gt2_bytes > 0 ? gt2_bytes : 16);
     L.fw = take(4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE);
     L.fi = take(4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE);
     // group-mass conservation: transposed inverse spatial matrices, and the
@@ -153,9 +160,6 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.sg = take(sigma && !wiener ? 4 * npp : 16);
     L.ex = take(4 * static_cast<int64_t>(kmax) * P);
 
-    // Gaussian noise: covariance-map row of every member pair (i > j)
-    const bool gauss = sp.noise_model == BMND_NOISE_GAUSSIAN;
-    L.lag = take(gauss && kmax > 0 ? 4 * static_cast<int64_t>(nmax) * ((nmax + 3) / 4 * 4) : 16);
     L.scan = take(8 * (kThreads / 32 + 1));  // the warps' totals, then the block's
     L.plane = take(8 * (nmax > 40 ? nmax : 40));  // also the mass phase's 8 warps x 5 sums
     L.wts = take(4 * nmax);
@@ -168,11 +172,14 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.x = L.s + buf;
     L.r = L.x + buf;  // Wiener: pilot coefficients, then the attenuation
     L.v = L.r;        // hard thresholding: the attenuation
-    const int64_t group_bytes = 3 * buf;
+    // Gaussian noise: covariance-map row of every member pair (i > j), needed
+    // before R or V is, in their place where they are large enough
+    const int64_t lag_bytes = gauss && kmax > 0 ? 4 * static_cast<int64_t>(nmax) * ((nmax + 3) / 4 * 4) : 0;
+    L.lag = L.r;
+    const int64_t group_bytes = 2 * buf + (buf > lag_bytes ? buf : round16(lag_bytes));
     // union-voxel lists of the exact phase (Poisson noise, or white Gaussian
     // noise with exact risk weights), kept apart from the group buffers when
     // the exact risk reads them after the shrinkage
-    const bool keep = sp.exact_risk_weights != 0;
     const int kl = (gauss && !keep) ? 0 : kmax;
     const int64_t umax = kl > 0 ? (np < ucells ? np : ucells) : 0;
     // member masks per union coordinate of every axis: a union box of at most
@@ -182,24 +189,28 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
         const int64_t most = ucells * sp.block[d] / P;
         axis_masks += most < sp.shape[d] ? most : sp.shape[d];
     }
-    L.grid = keep ? L.uni + group_bytes : L.uni;
+    // exact variance: per-warp partial sums of one tile of 4 planes x 32 JR
+    // coefficients, added in warp order afterwards.  They take the group buffers'
+    // place, as the lists do, behind them; with a single tile (k <= 4 and P <= its
+    // width: the default profiles) the lists are done with by then and give
+    // theirs.  (Apart from the union region they made 8x8x8 patches at the default
+    // stack of 32 need 233 728 bytes, above the limit of 232 448; so, 216 304.)
+    const int tile_w = 32 * kron_jr(P);
+    const int64_t part_bytes = !gauss && kmax > 0 ? 4 * (kThreads / 32) * 4 * static_cast<int64_t>(tile_w) : 0;
+    L.part_over = !keep && kmax <= 4 && P <= tile_w;
+    const int64_t ahead = keep ? (group_bytes > part_bytes ? group_bytes : part_bytes) : 0;
+    L.grid = L.uni + ahead;
     L.lval = L.grid + round16(kl > 0 ? 4 * axis_masks : 0);
     L.lstart = L.lval + round16(4 * umax);
     L.lent = L.lstart + round16(4 * (umax + 1));
-    const int64_t list_end = L.lent + round16(kl > 0 ? 4 * (np + 2) : 0);
-    off = keep ? list_end : L.uni + (group_bytes > list_end - L.uni ? group_bytes : list_end - L.uni);
-    // exact variance: per-warp partial sums of one tile of 4 planes x 32 JR
-    // coefficients (64 for the half-warp form), added in warp order afterwards.
-    // With a single tile (k <= 4 and P <= its width: the default profiles) the
-    // lists are done with by then and give their place.
-    const int tile_w = kron_jr(P) == 2 ? 64 : 32 * kron_jr(P);
-    const int64_t part_bytes = 4 * (kThreads / 32) * 4 * static_cast<int64_t>(tile_w);
-    L.part_over = !keep && kmax <= 4 && P <= tile_w;
-    if (gauss || kmax <= 0) L.part = L.grid;
-    else if (L.part_over) {
-        L.part = L.grid;
-        if (off < L.part + part_bytes) off = L.part + part_bytes;
-    } else L.part = take(part_bytes);
+    int64_t end = L.lent + round16(kl > 0 ? 4 * (np + 2) : 0);
+    if (!early) {
+        L.gt2 = end;
+        if (kl > 0) end += gt2_bytes;
+    }
+    L.part = keep ? L.uni : (L.part_over ? L.grid : end);
+    if (!keep && end < L.part + part_bytes) end = L.part + part_bytes;
+    off = end > L.uni + group_bytes ? end : L.uni + group_bytes;
     L.total = off;
     return L;
 }
@@ -975,9 +986,9 @@ struct PlaneVec {
 template <int RL, int NQ>
 __device__ __forceinline__ void exact_stream(const float* __restrict__ lval, const int* __restrict__ lstart,
                                              const uint32_t* __restrict__ lent, int u_lo, int u_hi,
-                                             const unsigned char* smem, uint32_t plane_byte, uint32_t stride,
+                                             const unsigned char* base, uint32_t plane_byte, uint32_t stride,
                                              const float* __restrict__ stl, float (&var)[RL][NQ]) {
-    const unsigned char* gb = smem + plane_byte;
+    const unsigned char* gb = base + plane_byte;
 #pragma unroll
     for (int r = 0; r < RL; ++r)
 #pragma unroll
@@ -1037,8 +1048,8 @@ __device__ __forceinline__ void exact_stream(const float* __restrict__ lval, con
 // multiply-adds per instruction, each rounded as its scalar form).  It is bound
 // by instruction issue, so addresses are kept in 32-bit shared-memory form (the
 // generic 64-bit pointers cost more integer instructions than the products):
-// an entry word holds the shared-memory byte offset of the member's paired G
-// entries and the patch element; two words past the last one are readable.  A
+// an entry word holds the byte offset of the member's entries in the table of
+// paired G entries and the patch element; two words past the last one are readable.  A
 // voxel's first entry starts its sums with a product.
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     uint32_t v;
@@ -1073,14 +1084,14 @@ __device__ __forceinline__ void load_row(float2 (&sv)[2], const char* row0, uint
 }
 
 template <int NQ>
-__device__ __forceinline__ void exact_pairs(const unsigned char* smem, const float* lval, const int* lstart,
+__device__ __forceinline__ void exact_pairs(const unsigned char* base, const float* lval, const int* lstart,
                                             const uint32_t* lent, int u_lo, int u_hi, uint32_t plane_byte,
                                             const float* __restrict__ st, uint32_t stride_b,
                                             float2 (&var)[2][NQ]) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) var[0][q] = var[1][q] = make_float2(0.0f, 0.0f);
     if (u_lo >= u_hi) return;
-    const uint32_t plane = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + plane_byte;
+    const uint32_t plane = static_cast<uint32_t>(__cvta_generic_to_shared(base)) + plane_byte;
     const uint32_t ents = static_cast<uint32_t>(__cvta_generic_to_shared(lent));
     uint32_t ls = static_cast<uint32_t>(__cvta_generic_to_shared(lstart + u_lo));
     const uint32_t lv = static_cast<uint32_t>(__cvta_generic_to_shared(lval)) -
@@ -1286,7 +1297,7 @@ __device__ __forceinline__ void exact_haar(const float* lval, const int* lstart,
 // halves' sums are added at the end.  (A whole warp per half, without the
 // divergence where only one half ends a voxel, took 14 % more instructions.)
 template <int JR, int NQ, bool HAAR>
-__device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint32_t kron_byte, const float* __restrict__ lval,
+__device__ void exact_planes(const unsigned char* base, float a0, float b0, uint32_t kron_byte, const float* __restrict__ lval,
                              const int* __restrict__ lstart, const uint32_t* __restrict__ lent, int U,
                              int kk, const float* __restrict__ st, int P,
                              float* __restrict__ EX, float* __restrict__ part, bool part_over) {
@@ -1317,7 +1328,7 @@ __device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint
                 // sums are added as in the generic form below)
                 constexpr int RP = JR / 2;
                 const int u_mid = JR == 2 ? first_voxel((lstart[u_lo] + lstart[u_hi]) >> 1, u_lo, u_hi) : u_hi;
-                const uint32_t kron_lane = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + kron_byte + 8u * lane;
+                const uint32_t kron_lane = static_cast<uint32_t>(__cvta_generic_to_shared(base)) + kron_byte + 8u * lane;
                 float2 var[RP][NQ];
                 exact_haar<RP, NQ>(lval, lstart, lent, u_lo, u_mid, a0, b0, st + JR * lane, kron_lane, var);
 #pragma unroll
@@ -1336,7 +1347,7 @@ __device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint
                     }
                 }
             } else if constexpr (JR == 1) {
-                exact_stream<1, NQ>(lval, lstart, lent, u_lo, u_hi, smem, 8u * i0, stride, st + j0 + lane, out);
+                exact_stream<1, NQ>(lval, lstart, lent, u_lo, u_hi, base, 8u * i0, stride, st + j0 + lane, out);
             } else {
                 float2 var[2][NQ];
                 int lo = u_lo, hi = u_hi;
@@ -1346,7 +1357,7 @@ __device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint
                     if (lane >> 4) lo = u_mid;
                     else hi = u_mid;
                 }
-                exact_pairs<NQ>(smem, lval, lstart, lent, lo, hi, 8u * i0, st + j0 + jl, 4u * stride, var);
+                exact_pairs<NQ>(base, lval, lstart, lent, lo, hi, 8u * i0, st + j0 + jl, 4u * stride, var);
 #pragma unroll
                 for (int q = 0; q < NQ; ++q)
 #pragma unroll
@@ -1385,15 +1396,15 @@ __device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint
 }
 
 template <int JR>
-__device__ void exact_planes_any(const unsigned char* smem, bool haar, float a0, float b0, uint32_t kron_byte,
+__device__ void exact_planes_any(const unsigned char* base, bool haar, float a0, float b0, uint32_t kron_byte,
                                  const float* __restrict__ lval, const int* __restrict__ lstart,
                                  const uint32_t* __restrict__ lent, int U, int kk, const float* __restrict__ st, int P,
                                  float* __restrict__ EX, float* __restrict__ part, bool part_over) {
     auto run = [&](auto h) {
         constexpr bool H = decltype(h)::value;
-        if (kk == 1) exact_planes<JR, 1, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
-        else if (kk == 2) exact_planes<JR, 2, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
-        else exact_planes<JR, 4, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        if (kk == 1) exact_planes<JR, 1, H>(base, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        else if (kk == 2) exact_planes<JR, 2, H>(base, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        else exact_planes<JR, 4, H>(base, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
     };
     if (JR > 1 && haar) run(BoolTag<JR != 1>{});
     else run(BoolTag<false>{});
@@ -1408,7 +1419,7 @@ __device__ void exact_planes_any(const unsigned char* smem, bool haar, float a0,
 // one tile); (f SM)[j] = sum_p f[p] SM[p][j] takes f[p] from its lane by a
 // shuffle.  The voxel terms are float32, their sum over voxels float64.
 template <int JR, int NQ>
-__device__ double exact_risk_tile(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
+__device__ double exact_risk_tile(const unsigned char* base, const float* __restrict__ lval, const int* __restrict__ lstart,
                                   const uint32_t* __restrict__ lent, int u_lo, int u_hi,
                                   int i0, int kk,
                                   const float* __restrict__ st, const float* __restrict__ smt,
@@ -1432,7 +1443,7 @@ __device__ double exact_risk_tile(const unsigned char* smem, const float* __rest
         {
             const uint32_t ent = lent[e];
             PlaneVec<NQ> gv;
-            gv.load_pairs(smem + 8 * i0 + (ent & 0xffffu));
+            gv.load_pairs(base + 8 * i0 + (ent & 0xffffu));
             KronVec<JR> sv;
             sv.load(stl + (ent >> 16) * static_cast<uint32_t>(stride));
 #pragma unroll
@@ -1443,7 +1454,7 @@ __device__ double exact_risk_tile(const unsigned char* smem, const float* __rest
         for (++e; e < e1; ++e) {
             const uint32_t ent = lent[e];
             PlaneVec<NQ> gv;
-            gv.load_pairs(smem + 8 * i0 + (ent & 0xffffu));
+            gv.load_pairs(base + 8 * i0 + (ent & 0xffffu));
             KronVec<JR> sv;
             sv.load(stl + (ent >> 16) * static_cast<uint32_t>(stride));
 #pragma unroll
@@ -1490,7 +1501,7 @@ __device__ double exact_risk_tile(const unsigned char* smem, const float* __rest
 // warp w takes the voxels whose entry lists start in its share of all entries
 // (the exact variance's split); lanes, then warps, add in a fixed order
 template <int JR, int NQ>
-__device__ void exact_risk(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
+__device__ void exact_risk(const unsigned char* base, const float* __restrict__ lval, const int* __restrict__ lstart,
                            const uint32_t* __restrict__ lent, int U, int kk, const float* __restrict__ st, const float* __restrict__ smt,
                            const float* __restrict__ att, int P, double* __restrict__ part) {
     const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
@@ -1509,7 +1520,7 @@ __device__ void exact_risk(const unsigned char* smem, const float* __restrict__ 
     const int u_hi = warp == nw - 1 ? U : first_voxel(static_cast<int>(static_cast<int64_t>(E) * (warp + 1) / nw));
     double acc = 0.0;
     for (int i0 = 0; i0 < kk; i0 += NQ)
-        acc += exact_risk_tile<JR, NQ>(smem, lval, lstart, lent, u_lo, u_hi, i0, kk, st, smt, att, P);
+        acc += exact_risk_tile<JR, NQ>(base, lval, lstart, lent, u_lo, u_hi, i0, kk, st, smt, att, P);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) part[warp] = acc;
@@ -1523,13 +1534,13 @@ __device__ void exact_risk(const unsigned char* smem, const float* __restrict__ 
 }
 
 template <int JR>
-__device__ void exact_risk_any(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
+__device__ void exact_risk_any(const unsigned char* base, const float* __restrict__ lval, const int* __restrict__ lstart,
                                const uint32_t* __restrict__ lent, int U,
                                int kk, const float* __restrict__ st, const float* __restrict__ smt,
                                const float* __restrict__ att, int P, double* __restrict__ part) {
-    if (kk == 1) exact_risk<JR, 1>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
-    else if (kk == 2) exact_risk<JR, 2>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
-    else exact_risk<JR, 4>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
+    if (kk == 1) exact_risk<JR, 1>(base, lval, lstart, lent, U, kk, st, smt, att, P, part);
+    else if (kk == 2) exact_risk<JR, 2>(base, lval, lstart, lent, U, kk, st, smt, att, P, part);
+    else exact_risk<JR, 4>(base, lval, lstart, lent, U, kk, st, smt, att, P, part);
 }
 
 // Exact Gaussian variances of planes 0 .. 3 of a Haar group (kk of them): with
@@ -1617,6 +1628,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
 
     float* G = sm<float>(smem, a.L.g);
     float2* GT2 = sm<float2>(smem, a.L.gt2);
+    // what the entries' 16-bit offsets into GT2 count from: it may lie above 64 KB
+    // in the runtime geometry
+    const int64_t ent_base = ND > 0 ? 0 : a.L.gt2;
     float* Fw = sm<float>(smem, a.L.fw);
     float* win = sm<float>(smem, a.L.win);
     double* mdiag = sm<double>(smem, a.L.mdiag);
@@ -1724,7 +1738,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         for (int e = tid; e < n * n; e += blockDim.x) G[e] = __ldg(gtab + e);
         // G^T restricted to the exact planes, padded to 4, each entry twice:
         // GT2[g * kpad + i] = (G[i, g], G[i, g])
-        for (int e = tid; !quarters && e < n * kpad; e += blockDim.x) {
+        // (the runtime geometry has no room for them where nothing reads them)
+        const bool pairs = !quarters && (ND > 0 || sp.noise_model == BMND_NOISE_POISSON || sp.exact_risk_weights);
+        for (int e = tid; pairs && e < n * kpad; e += blockDim.x) {
             const int g = e / kpad, i = e % kpad;
             const float v = i < kk ? __ldg(gtab + i * n + g) : 0.0f;
             GT2[e] = make_float2(v, v);
@@ -1945,7 +1961,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             base += incl - mine;
             int w = static_cast<int>(base >> 16), we = static_cast<int>(base & 0xffffu);
             const int* shl = sm<int>(smem, a.L.shl);
-            const uint32_t gt2_off = static_cast<uint32_t>(a.L.gt2), row_b = 4u * static_cast<uint32_t>(kron_stride(P));
+            const uint32_t gt2_off = static_cast<uint32_t>(a.L.gt2 - ent_base), row_b = 4u * static_cast<uint32_t>(kron_stride(P));
             const int lg = ilog2_floor(n);
             walk([&](uint32_t m, int vox, int lin) {
                 reinterpret_cast<int*>(lval)[w] = vox;
@@ -1986,9 +2002,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         } else {
             const int jr = kron_jr(P);
             float* part = sm<float>(smem, a.L.part);
-            if (jr == 1) exact_planes_any<1>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
-            else if (jr == 2) exact_planes_any<2>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
-            else exact_planes_any<4>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            if (jr == 1) exact_planes_any<1>(smem + ent_base, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            else if (jr == 2) exact_planes_any<2>(smem + ent_base, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            else exact_planes_any<4>(smem + ent_base, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
         }
     }
 
@@ -2179,9 +2195,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         if (exact_risk) {
             const float* smt = a.st + static_cast<int64_t>(P) * kron_stride(P);
             const int jr = kron_jr(P);
-            if (jr == 1) exact_risk_any<1>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
-            else if (jr == 2) exact_risk_any<2>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
-            else exact_risk_any<4>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
+            if (jr == 1) exact_risk_any<1>(smem + ent_base, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
+            else if (jr == 2) exact_risk_any<2>(smem + ent_base, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
+            else exact_risk_any<4>(smem + ent_base, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
         }
     }
 
