@@ -255,7 +255,8 @@ def time_kernels(torch, noisy_t, profile, reps: int = 2, stages=("ht", "wiener")
     res = {}
     if precision is None:
         if gauss is not None:
-            # SSD: the pipeline's choice (tensor-core screening in 2-D, the exact kernel in 3-D)
+            # SSD: the pipeline's choice (where the box-sum kernels leave the stage,
+            # tensor-core screening in 2-D and the exact kernel in 3-D)
             ssd = _abi.MATCH_FAST if len(shape) == 2 else _abi.MATCH_EXACT
             precision = {"ht": ssd, "wiener": ssd}
         else:

@@ -232,12 +232,18 @@ struct StageWorkspace {
     int64_t aux_floats;
     char* ssd;       // tensor-core SSD matching: norms, screening distances, tiles
     uint64_t ssd_bytes;
-    uint64_t bytes;
+    uint64_t bytes;      // what the stage cannot do without
+    uint64_t box_bytes;  // behind it, for the box-sum matching where no region above serves as its scratch
 };
 
 uint64_t align256(uint64_t v) { return (v + 255) & ~uint64_t(255); }
 
 BmndMatchParams match_params_of(const BmndStageParams& sp);
+
+// hard thresholding with distances standardised by their null moments
+bool standardised(const BmndStageParams& sp) {
+    return sp.filter == BMND_FILTER_HARD_THRESHOLD && sp.match_policy == BMND_POLICY_CANDIDATE_STANDARDIZED;
+}
 
 StageWorkspace carve(const BmndStageParams& sp, int64_t n_refs, void* base) {
     StageWorkspace w{};
@@ -264,9 +270,14 @@ StageWorkspace carve(const BmndStageParams& sp, int64_t n_refs, void* base) {
     const BmndMatchParams mp = match_params_of(sp);
     w.aux_floats = approx_scratch_floats(mp, sp.shape, sp.block);
     uint64_t o_aux = take(w.aux_floats > 0 ? 4ull * static_cast<uint64_t>(w.aux_floats) : 16);
-    w.ssd_bytes = ssd_tc_scratch_bytes(mp, sp.block, n_refs, sp.ssd_poisson_bias != 0);
+    // The box-sum matching takes the aggregation's region, which is written after
+    // it; the stages it takes need no tensor-core scratch (4 n_refs x window
+    // bytes: 5.6 GB at 2048 x 2048).
+    const BoxScratch box = box_scratch(mp, sp.block, n_refs, sp.ssd_poisson_bias != 0, standardised(sp));
+    w.ssd_bytes = box.least ? 0 : ssd_tc_scratch_bytes(mp, sp.block, n_refs, sp.ssd_poisson_bias != 0);
     uint64_t o_ssd = take(w.ssd_bytes > 0 ? w.ssd_bytes : 16);
     w.bytes = off;
+    w.box_bytes = det && w.agg.bytes >= box.least ? 0 : box.full;
     if (base) {
         char* b = static_cast<char*>(base);
         w.num = det ? nullptr : reinterpret_cast<double*>(b + o_num);
@@ -287,13 +298,14 @@ StageWorkspace carve(const BmndStageParams& sp, int64_t n_refs, void* base) {
 
 BmndMatchParams match_params_of(const BmndStageParams& sp) {
     BmndMatchParams mp{};
-    // SSD matching of a 2-D image: the tensor-core screening with exact
-    // rescoring gives the exact kernel's match sets (see ssd_select_kernel), so
-    // exact requests take it.  In 3-D the exact kernel stays: a tile's union box
-    // of candidates is 8x a reference's window (about 6 % of the tensor
-    // products are used), and on a denoised pilot the screening bound leaves
-    // most of the window to rescore; measured at 256^3 the whole Gaussian call
-    // took 810 ms with the screening and 780 ms without.
+    // SSD matching that the box-sum kernels leave (few references, a radius above
+    // 64): in 2-D the tensor-core screening with exact rescoring gives the exact
+    // kernel's match sets (see ssd_select_kernel), so exact requests take it.  In
+    // 3-D the exact kernel stays: a tile's union box of candidates is 8x a
+    // reference's window (about 6 % of the tensor products are used), and on a
+    // denoised pilot the screening bound leaves most of the window to rescore;
+    // measured at 256^3 before the box-sum kernels the whole Gaussian call took
+    // 810 ms with the screening and 780 ms without.
     mp.ndim = sp.ndim;
     for (int d = 0; d < sp.ndim; ++d) {
         mp.counts[d] = sp.shape[d] - sp.block[d] + 1;
@@ -308,6 +320,12 @@ BmndMatchParams match_params_of(const BmndStageParams& sp) {
     if (sp.distance == BMND_DIST_SSD && sp.match_precision == BMND_MATCH_EXACT && !sp.ssd_poisson_bias &&
         sp.ndim == 2)
         mp.precision = BMND_MATCH_FAST;
+    // the real-valued pilot: the bounded screening of the Poisson deviance
+    // (SSD matching takes any values)
+    if (sp.filter == BMND_FILTER_WIENER && sp.wiener_match_source == BMND_SOURCE_PILOT &&
+        sp.match_precision == BMND_MATCH_EXACT && sp.distance != BMND_DIST_SSD)
+        mp.precision = BMND_MATCH_REAL_VALUED;
+    if (standardised(sp)) mp.precision = BMND_MATCH_EXACT;
     mp.count_scale = sp.count_scale;
     return mp;
 }
@@ -354,10 +372,6 @@ int32_t run_stage(const BmndStageParams& sp, const float* noisy, const float* pi
     BmndMatchParams mp = match_params_of(sp);
     const bool on_pilot = sp.filter == BMND_FILTER_WIENER && sp.wiener_match_source == BMND_SOURCE_PILOT;
     const float* match_src = on_pilot ? pilot : noisy;
-    // the real-valued pilot: the bounded screening of the Poisson deviance
-    // (SSD matching keeps its tensor-core screening, which any values suit)
-    if (on_pilot && sp.match_precision == BMND_MATCH_EXACT && sp.distance != BMND_DIST_SSD)
-        mp.precision = BMND_MATCH_REAL_VALUED;
     const float* thr_dev = nullptr;
     if (sp.distance == BMND_DIST_SSD) {
         rc = launch_ssd_threshold(match_src, static_cast<int64_t>(vox), sp.ssd_threshold, w.mm, w.thr, stream);
@@ -375,15 +389,20 @@ int32_t run_stage(const BmndStageParams& sp, const float* noisy, const float* pi
                                          sp.policy_beta, sp.policy_power, w.thr_ref, stream);
         if (rc) return rc;
         thr_per_ref = w.thr_ref;
-    } else if (sp.filter == BMND_FILTER_HARD_THRESHOLD && sp.match_policy == BMND_POLICY_CANDIDATE_STANDARDIZED) {
+    } else if (standardised(sp)) {
         null_moments = sp.null_moments;
-        mp.precision = BMND_MATCH_EXACT;
+    }
+    char* box_ws = w.agg_base;
+    uint64_t box_ws_bytes = w.agg_base ? w.agg.bytes : 0;
+    if (w.box_bytes && !sigma_out) {  // (with a sigma map that space holds its accumulators)
+        box_ws = static_cast<char*>(ws) + w.bytes;
+        box_ws_bytes = std::min(w.box_bytes, ws_bytes - w.bytes);
     }
     rc = launch_blockmatch_volume(mp, match_src, sp.shape, sp.block, refs, n_refs, thr_per_ref,
                                   sp.match_threshold, w.sel, w.count, w.accepted, stream, thr_dev,
                                   sp.match_noise_ssd, sp.ssd_gamma, allow_alloc, null_moments,
                                   sp.null_max_count, sp.ssd_poisson_bias != 0, w.aux, w.aux_floats, w.ssd,
-                                  w.ssd_bytes, w.agg_base, w.agg_base ? w.agg.bytes : 0);
+                                  w.ssd_bytes, box_ws, box_ws_bytes);
     if (rc) return rc;
     if (det) {
         rc = launch_entry_index(sp, w.sel, w.count, n_refs, w.agg_base, w.agg, stream);
@@ -615,7 +634,8 @@ int32_t bmnd_stage_workspace_bytes(const BmndStageParams* params, int64_t n_refs
     if (!params || !out_bytes || n_refs < 0) return fail(BMND_ERR_INVALID_ARG, "bad argument");
     int32_t rc = validate_stage(*params);
     if (rc) return rc;
-    *out_bytes = carve(*params, n_refs, nullptr).bytes;
+    const StageWorkspace w = carve(*params, n_refs, nullptr);
+    *out_bytes = w.bytes + w.box_bytes;
     return BMND_OK;
 }
 

@@ -2096,6 +2096,18 @@ uint64_t ssd_tc_scratch_bytes(const BmndMatchParams& mp, const int32_t* block, i
     return ssd_scratch_layout(mp.ndim, mp.counts, block, mp.search_radius, n_refs).bytes;
 }
 
+BoxScratch box_scratch(const BmndMatchParams& mp, const int32_t* block, int64_t n_refs, bool poisson_bias,
+                       bool null_moments) {
+    MatchArgs a{};
+    fill_common(a, mp);
+    for (int d = 0; d < mp.ndim; ++d) a.block[d] = block[d];
+    a.n_refs = n_refs;
+    a.poisson_bias = poisson_bias ? 1 : 0;
+    static const double some = 0.0;
+    a.null_moments = null_moments ? &some : nullptr;  // (its presence counts)
+    return box_match_scratch(a, mp.distance, mp.precision);
+}
+
 int64_t approx_scratch_floats(const BmndMatchParams& mp, const int32_t* shape, const int32_t* block) {
     const bool approx = mp.precision == BMND_MATCH_APPROX || mp.precision == BMND_MATCH_SUBSAMPLED;
     if (!approx || mp.distance != BMND_DIST_POISSON_DEVIANCE || mp.count_scale != 1.0 ||

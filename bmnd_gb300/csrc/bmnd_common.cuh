@@ -229,6 +229,13 @@ __device__ __forceinline__ float centred_norm(float s2, float s1, float mu, int 
 }
 // bytes of workspace the tensor-core SSD matching of a volume needs (0: it does not apply)
 uint64_t ssd_tc_scratch_bytes(const BmndMatchParams& mp, const int32_t* block, int64_t n_refs, bool poisson_bias);
+// scratch bytes of the box-sum matching: the least it runs with, and what lets it
+// take all references in one or a few chunks; zero where it does not run
+struct BoxScratch {
+    uint64_t least, full;
+};
+BoxScratch box_scratch(const BmndMatchParams& mp, const int32_t* block, int64_t n_refs, bool poisson_bias,
+                       bool null_moments);
 // floats of workspace the approximate screening form of a volume needs (0: none)
 int64_t approx_scratch_floats(const BmndMatchParams& mp, const int32_t* shape, const int32_t* block);
 int32_t launch_reference_thresholds(const float* volume, const int32_t* refs, int64_t n_refs, int ndim,

@@ -56,6 +56,8 @@ constexpr int kSelWarps = 4;   // references per CTA of the selection
 constexpr int kQueue = 192;    // exact rescoring queue per reference
 constexpr int kAmb = 384;      // candidates whose acceptance alone is open, per reference
 constexpr int kRowThreads3 = 512, kRowThreads2 = 256;
+// rows of a chunk of references where no workspace bounds them
+constexpr uint64_t kRowScratch = 1ull << 30;
 constexpr float kLn2x2 = 1.38629436f;
 constexpr float kTinyCount = 7.88860905e-31f;  // 2^-100
 
@@ -1299,27 +1301,37 @@ __global__ void __launch_bounds__(kSelWarps * 32, 8) box_select_kernel(MatchArgs
 
 uint64_t round256(uint64_t v) { return (v + 255) & ~uint64_t(255); }
 
-}  // namespace
+// Whether a matching takes these kernels, its tiles and its scratch
+struct BoxPlan {
+    bool applies, want_f;
+    BoxArgs b;  // geometry and tiles; no pointers but the source's
+    int ztiles, splits;
+    int64_t columns;
+    size_t smem;
+    // scratch: origin map and column flags, the counts' box sums, the rows of a chunk of references
+    uint64_t o_flag, o_fvox, o_fbox, o_rows, per_ref;
+    uint64_t least, full;  // bytes: for a few references at a time, for chunks of up to kRowScratch
+};
 
-int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t stream, bool* done) {
-    *done = false;
+BoxPlan plan_box_match(const MatchArgs& a, int code, int precision) {
+    BoxPlan p{};
+    BoxArgs& b = p.b;
     const bool ssd = code == BMND_DIST_SSD;
     const int* bl = a.block;
     const bool shape2 = a.ndim == 2 && bl[0] == 8 && bl[1] == 8;
     const bool shape5 = a.ndim == 3 && bl[0] == 5 && bl[1] == 5 && bl[2] == 5;
     const bool shape4 = a.ndim == 3 && bl[0] == 4 && bl[1] == 4 && bl[2] == 4;
-    if (a.table || a.fixup || a.null_moments || a.max_m > 32 || !(shape2 || shape4 || shape5)) return BMND_OK;
-    if (ssd ? a.poisson_bias != 0 : (code != BMND_DIST_POISSON_DEVIANCE || !a.stab)) return BMND_OK;
+    if (a.table || a.fixup || a.null_moments || a.max_m > 32 || !(shape2 || shape4 || shape5)) return p;
+    if (ssd ? a.poisson_bias != 0 : (code != BMND_DIST_POISSON_DEVIANCE || !a.stab)) return p;
     if (precision != BMND_MATCH_EXACT && precision != BMND_MATCH_FAST && precision != BMND_MATCH_REAL_VALUED)
-        return BMND_OK;
-    BoxArgs b{};
+        return p;
     const int W = shape2 ? 8 : (shape5 ? 5 : 4);
     const int ax[3] = {0, a.ndim == 3 ? 1 : -1, a.ndim - 1};
     for (int d = 0; d < 3; ++d) {
         b.cnt[d] = ax[d] < 0 ? 1 : a.counts[ax[d]];
         b.rad[d] = ax[d] < 0 ? 0 : a.radius[ax[d]];
         b.n[d] = ax[d] < 0 ? 1 : a.counts[ax[d]] + bl[ax[d]] - 1;
-        if (b.rad[d] > 64) return BMND_OK;
+        if (b.rad[d] > 64) return p;
     }
     b.src = a.src;
     b.inv_scale = a.inv_scale;
@@ -1335,7 +1347,7 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
     const int64_t n_lins = static_cast<int64_t>(b.cnt[0]) * b.cnt[1] * b.cnt[2];
     // the shared terms pay off while references are dense: up to one per 64
     // origins (the schedules have one per 4.5 to 27)
-    if (b.rowlen > (1 << 20) || a.n_refs * 64 < n_lins || a.n_refs > 0x7fffffffLL) return BMND_OK;
+    if (b.rowlen > (1 << 20) || a.n_refs * 64 < n_lins || a.n_refs > 0x7fffffffLL) return p;
     // Few references of a stage on counts: the kernel of tabulated terms has no
     // phases that wait on each other.  One GB300, that kernel against this file's:
     // 64 x 64 34 against 115 us, 140 x 140 (3.9 K references) 164 against 169,
@@ -1344,9 +1356,9 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
     // Real-valued stages come here whatever their size: few references gain
     // 0.1 ms at best in the screened kernel, and those it cannot settle cost
     // 3.1 ms there (24 x 24 x 40, peak 30; here 0.5 in all).
-    const bool want_f = !ssd && precision != BMND_MATCH_REAL_VALUED && a.inv_scale == 1.0f;
+    p.want_f = !ssd && precision != BMND_MATCH_REAL_VALUED && a.inv_scale == 1.0f;
     const bool few = a.n_refs < (shape2 ? 4096 : 8192);
-    if (want_f && precision == BMND_MATCH_EXACT && a.use_table && few) return BMND_OK;
+    if (p.want_f && precision == BMND_MATCH_EXACT && a.use_table && few) return p;
 
     // tiles: the largest whose shared memory fits; first-axis offsets are split
     // over CTAs until every SM has several
@@ -1360,44 +1372,64 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
     };
     const size_t limit = shape2 ? 110 * 1024 : 220 * 1024;
     const int tz_cap = shape2 ? 48 : 29;
-    int ztiles = (b.cnt[0] + tz_cap - 1) / tz_cap;
+    int& ztiles = p.ztiles;
+    ztiles = (b.cnt[0] + tz_cap - 1) / tz_cap;
     b.tz = (b.cnt[0] + ztiles - 1) / ztiles;
     b.ytiles = shape2 ? 1 : (b.cnt[1] + 32 - W) / (33 - W);
-    const int64_t columns = shape2 ? (b.cnt[2] + kTileX - 1) / kTileX : (b.cnt[2] + 2) / 3;
-    auto tiles = [&]() { return columns * b.ytiles * ztiles; };
+    p.columns = shape2 ? (b.cnt[2] + kTileX - 1) / kTileX : (b.cnt[2] + 2) / 3;
+    auto tiles = [&]() { return p.columns * b.ytiles * ztiles; };
     // (small grids: shorter tiles until there is a CTA or two for every SM)
     while (b.tz > 2 * W && tiles() * b.nz < 152 * 2) {
         b.tz = (b.tz + 1) / 2;
         ztiles = (b.cnt[0] + b.tz - 1) / b.tz;
     }
-    int splits = static_cast<int>(std::min<int64_t>(b.nz, (152 * 8 + tiles() - 1) / tiles()));
+    int& splits = p.splits;
+    splits = static_cast<int>(std::min<int64_t>(b.nz, (152 * 8 + tiles() - 1) / tiles()));
     b.per = (b.nz + splits - 1) / splits;
     while (smem_of(b.tz, b.per) > limit && b.per > 1) --b.per;
     while (smem_of(b.tz, b.per) > limit && b.tz > 4) {
         b.tz = (b.tz + 1) / 2;
         ztiles = (b.cnt[0] + b.tz - 1) / b.tz;
     }
-    const size_t smem = smem_of(b.tz, b.per);
-    if (smem > limit) return BMND_OK;
+    p.smem = smem_of(b.tz, b.per);
+    if (p.smem > limit) return p;
     splits = (b.nz + b.per - 1) / b.per;
-    if (static_cast<int64_t>(b.ytiles) * ztiles > 65535 || splits > 65535) return BMND_OK;
+    if (static_cast<int64_t>(b.ytiles) * ztiles > 65535 || splits > 65535) return p;
 
-    // scratch: origin map and column flags, the counts' box sums, the rows of a chunk of references
-    const uint64_t o_flag = round256(4ull * n_lins);
-    const uint64_t o_fvox = o_flag + round256(4ull * b.cnt[2]);
-    const uint64_t o_fbox = o_fvox + (want_f ? round256(4ull * b.nvox) : 0);
-    const uint64_t o_rows = o_fbox + (want_f ? round256(4ull * n_lins) : 0);
-    const uint64_t per_ref = 4ull * b.rowlen + 20;
+    p.o_flag = round256(4ull * n_lins);
+    p.o_fvox = p.o_flag + round256(4ull * b.cnt[2]);
+    p.o_fbox = p.o_fvox + (p.want_f ? round256(4ull * b.nvox) : 0);
+    p.o_rows = p.o_fbox + (p.want_f ? round256(4ull * n_lins) : 0);
+    p.per_ref = 4ull * b.rowlen + 20;
+    p.least = p.o_rows + 1024 + p.per_ref * std::min<int64_t>(a.n_refs, 512);
+    p.full = std::max(p.least, p.o_rows + 1024 + std::min<uint64_t>(p.per_ref * a.n_refs, kRowScratch));
+    p.applies = true;
+    return p;
+}
+
+}  // namespace
+
+BoxScratch box_match_scratch(const MatchArgs& a, int code, int precision) {
+    const BoxPlan p = plan_box_match(a, code, precision);
+    return p.applies ? BoxScratch{p.least, p.full} : BoxScratch{0, 0};
+}
+
+int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t stream, bool* done) {
+    *done = false;
+    const BoxPlan p = plan_box_match(a, code, precision);
+    if (!p.applies) return BMND_OK;
+    BoxArgs b = p.b;
+    const bool ssd = code == BMND_DIST_SSD, want_f = p.want_f;
+    const bool shape2 = a.ndim == 2, shape5 = a.ndim == 3 && a.block[0] == 5;
+    const int64_t n_lins = static_cast<int64_t>(b.cnt[0]) * b.cnt[1] * b.cnt[2];
     char* base = nullptr;
     uint64_t bytes = 0;
     bool owned = false;
-    const uint64_t least = o_rows + 1024 + per_ref * std::min<int64_t>(a.n_refs, 512);
-    if (a.box_ws && a.box_ws_bytes >= least) {
+    if (a.box_ws && a.box_ws_bytes >= p.least) {
         base = a.box_ws;
         bytes = a.box_ws_bytes;
     } else if (!a.no_alloc) {
-        bytes = o_rows + 1024 + std::max(std::min<uint64_t>(per_ref * a.n_refs, 1ull << 30),
-                                        per_ref * std::min<int64_t>(a.n_refs, 512));
+        bytes = p.full;
         if (cudaMallocAsync(reinterpret_cast<void**>(&base), bytes, stream) == cudaSuccess) {
             owned = true;
             note_device_alloc();
@@ -1407,22 +1439,22 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
         }
     }
     if (!base) return BMND_OK;
-    int64_t chunk = static_cast<int64_t>((bytes - o_rows - 1024) / per_ref);
+    int64_t chunk = static_cast<int64_t>((bytes - p.o_rows - 1024) / p.per_ref);
     if (chunk > a.n_refs) chunk = a.n_refs;
     const int64_t nchunks = (a.n_refs + chunk - 1) / chunk;
     chunk = (a.n_refs + nchunks - 1) / nchunks;
     b.map = reinterpret_cast<int32_t*>(base);
-    b.colflag = reinterpret_cast<int32_t*>(base + o_flag);
-    b.fvox = want_f ? reinterpret_cast<float*>(base + o_fvox) : nullptr;
-    b.fbox = want_f ? reinterpret_cast<float*>(base + o_fbox) : nullptr;
-    b.rows = reinterpret_cast<float*>(base + o_rows);
-    b.mode = reinterpret_cast<int32_t*>(base + o_rows + round256(4ull * b.rowlen * chunk));
+    b.colflag = reinterpret_cast<int32_t*>(base + p.o_flag);
+    b.fvox = want_f ? reinterpret_cast<float*>(base + p.o_fvox) : nullptr;
+    b.fbox = want_f ? reinterpret_cast<float*>(base + p.o_fbox) : nullptr;
+    b.rows = reinterpret_cast<float*>(base + p.o_rows);
+    b.mode = reinterpret_cast<int32_t*>(base + p.o_rows + round256(4ull * b.rowlen * chunk));
     b.heavy_n = b.mode + chunk;
     b.heavy = b.heavy_n + 1;
     b.cuts = reinterpret_cast<float*>(b.heavy + chunk);
 
     auto run = [&]() -> int32_t {
-        BMND_CUDA_TRY(cudaMemsetAsync(base, 0xff, o_fvox, stream));
+        BMND_CUDA_TRY(cudaMemsetAsync(base, 0xff, p.o_fvox, stream));
         const int64_t work = std::max<int64_t>(a.n_refs, want_f ? b.nvox : 1);
         const unsigned nb = static_cast<unsigned>(std::min<int64_t>((work + 255) / 256, 152 * 16));
         box_prepare_kernel<<<nb, 256, 0, stream>>>(a, b);
@@ -1438,7 +1470,7 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
         const void* rows_fn = shape2 ? reinterpret_cast<const void*>(box_rows_2d_kernel)
                                      : (shape5 ? reinterpret_cast<const void*>(box_rows_3d_kernel<5>)
                                                : reinterpret_cast<const void*>(box_rows_3d_kernel<4>));
-        if (int32_t rc = kernel_residency(rows_fn, shape2 ? kRowThreads2 : kRowThreads3, smem, false, &per_sm, &sms))
+        if (int32_t rc = kernel_residency(rows_fn, shape2 ? kRowThreads2 : kRowThreads3, p.smem, false, &per_sm, &sms))
             return rc;
         const void* sel_fn = ssd ? reinterpret_cast<const void*>(box_select_kernel<true, false>)
                                  : reinterpret_cast<const void*>(box_select_kernel<false, false>);
@@ -1452,14 +1484,14 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
             b.hi = std::min<int64_t>(b.lo + chunk, a.n_refs);
             BMND_CUDA_TRY(cudaMemsetAsync(b.heavy_n, 0, 4, stream));
             if (shape2) {
-                const dim3 grid(static_cast<unsigned>(columns), static_cast<unsigned>(ztiles),
-                                static_cast<unsigned>(splits));
-                box_rows_2d_kernel<<<grid, kRowThreads2, smem, stream>>>(b);
+                const dim3 grid(static_cast<unsigned>(p.columns), static_cast<unsigned>(p.ztiles),
+                                static_cast<unsigned>(p.splits));
+                box_rows_2d_kernel<<<grid, kRowThreads2, p.smem, stream>>>(b);
             } else {
-                const dim3 grid(static_cast<unsigned>(b.cnt[2]), static_cast<unsigned>(b.ytiles * ztiles),
-                                static_cast<unsigned>(splits));
-                if (shape5) box_rows_3d_kernel<5><<<grid, kRowThreads3, smem, stream>>>(b);
-                else box_rows_3d_kernel<4><<<grid, kRowThreads3, smem, stream>>>(b);
+                const dim3 grid(static_cast<unsigned>(b.cnt[2]), static_cast<unsigned>(b.ytiles * p.ztiles),
+                                static_cast<unsigned>(p.splits));
+                if (shape5) box_rows_3d_kernel<5><<<grid, kRowThreads3, p.smem, stream>>>(b);
+                else box_rows_3d_kernel<4><<<grid, kRowThreads3, p.smem, stream>>>(b);
             }
             BMND_LAUNCH_CHECK("box_rows_kernel");
             // few references: fewer per CTA, whose warps then share their rescoring

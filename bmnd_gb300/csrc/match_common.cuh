@@ -162,5 +162,7 @@ int32_t launch_exact(MatchArgs& a, int code, cudaStream_t stream);
 // Box-sum matching (boxmatch.cu): *done is set when it ran; the references it
 // leaves to the exact kernel have count = -1
 int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t stream, bool* done);
+// the scratch it would use (zero: it does not take the matching)
+BoxScratch box_match_scratch(const MatchArgs& a, int code, int precision);
 
 }  // namespace bmnd

@@ -296,7 +296,9 @@ int32_t bmnd_blockmatch_volume_poisson_biased(const BmndMatchParams* params, con
                                               uint64_t stream);
 
 /*
- * Workspace bytes bmnd_stage() needs for `params` and n_refs references.
+ * Workspace bytes of bmnd_stage() for `params` and n_refs references.  Stages
+ * without the deterministic aggregation (mass conservation) count scratch for
+ * the matching in; with a workspace that lacks it they allocate it on the stream.
  */
 int32_t bmnd_stage_workspace_bytes(const BmndStageParams* params, int64_t n_refs,
                                    uint64_t* out_bytes);
@@ -385,8 +387,8 @@ int32_t bmnd_group_probe(const BmndStageParams* params, const float* d_noisy, co
  * fixed array of BMND_STATIC_SCRATCH_BYTES compiled into
  * this library, held by every GPU that loads it until the process exits.
  *   - A stage needing more scratch than that is rejected with
- *     BMND_ERR_WORKSPACE before any device work (see
- *     bmnd_stage_workspace_bytes for the requirement).
+ *     BMND_ERR_WORKSPACE before any device work (the message says how much it
+ *     needs; of bmnd_stage_workspace_bytes, all but the matching's scratch).
  *   - The first call on a device looks up the array's device address (once
  *     per CUDA context, with that device current; a context re-created after
  *     cudaDeviceReset is looked up again); make that first call before any

@@ -44,3 +44,43 @@ def test_large_patches_with_options_fit(native, noise, windowed, mass, k):
         for d in range(3):
             p.cov_domain[d] = 8
     _accepted(native, p)
+
+
+def _bytes(native, prof, shape, stage, n_refs, **fields):
+    res = resolve_profile(prof, shape)
+    p = plan.stage_params(prof, shape, stage, res.blockmatch_distance, res.variance_k)
+    for name, value in fields.items():
+        setattr(p, name, value)
+    n = ctypes.c_uint64(0)
+    assert native.bmnd_stage_workspace_bytes(ctypes.byref(p), n_refs, ctypes.byref(n)) == _abi.OK
+    return n.value
+
+
+@pytest.mark.parametrize("stage", ["ht", "wiener"])
+def test_tensor_core_scratch_only_where_it_is_used(native, stage):
+    """A 2-D SSD stage whose matching the box-sum kernels take reserves what the
+    deviance stage does; few references or a wide window keep the tensor-core
+    kernels and their 4 x window bytes per reference."""
+    shape, n = (2048, 2048), 900_000
+    poisson = bg.BM3DProfile(noise_model="poisson", gamma=0.0)
+    ssd = bg.BM3DProfile(noise_model="poisson", blockmatch_distance="ssd", gamma=0.0)
+    assert _bytes(native, ssd, shape, stage, n) == _bytes(native, poisson, shape, stage, n)
+    few = 2000
+    assert (_bytes(native, ssd, shape, stage, few) - _bytes(native, poisson, shape, stage, few)
+            >= 4 * few * 39 * 39)
+    wide = bg.BM3DProfile(noise_model="poisson", blockmatch_distance="ssd", gamma=0.0,
+                          **{f"{stage}_search_window": (65, 65)})
+    assert _bytes(native, wide, shape, stage, n) >= 4 * n * 131 * 131
+
+
+@pytest.mark.parametrize("prof,shape,n", [(bg.BM3DProfile, (512, 512), 50_000), (bg.BM4DProfile, (96, 96, 96), 60_000)])
+def test_mass_conserving_stage_counts_its_matching_scratch(native, prof, shape, n):
+    """Without the aggregation's region the rows of a chunk of references come from
+    the workspace, not from an allocation on the stream."""
+    r = (19, 19) if len(shape) == 2 else (7, 7, 7)
+    extra = _bytes(native, prof(noise_model="poisson"), shape, "ht", n, mass_conserve=1)
+    base = 16 * shape[0] * shape[1] * (shape[2] if len(shape) == 3 else 1)
+    rows = 4 * n
+    for d, v in enumerate(r):
+        rows *= 2 * v + 1 if d < len(r) - 1 else (2 * v + 8) // 8 * 8
+    assert extra >= base + min(rows, 1 << 28)
