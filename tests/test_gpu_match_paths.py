@@ -1,0 +1,88 @@
+"""Each matching path against another kernel, on references that really take it.
+
+The box-sum kernels take dense reference lists, so the tensor-core and the
+screened kernels are reached with sparse ones: fewer than one reference per 64
+patch origins.  Their expected tables come from the exact warp kernel (sparse
+lists of precision exact, or the patch-table entry); the number of launches
+tells the paths apart.
+"""
+
+import zlib
+
+import numpy as np
+import pytest
+from test_gpu_box_matching import DEV, SHAPES, SSD, _few_at_a_time, _match, _refs, _volume
+
+pytestmark = pytest.mark.gpu
+
+
+def _sparse(shape, block, rng):
+    counts = [s - b + 1 for s, b in zip(shape, block)]
+    lins = rng.choice(int(np.prod(counts)), size=(int(np.prod(counts)) - 1) // 64, replace=False)
+    return np.stack(np.unravel_index(lins, counts), -1).astype(np.int32)
+
+
+def _both(cuda, native, vol, block, radius, max_m, min_m, thr, code, refs, fast_launches, **kw):
+    # (the exact warp kernel is one launch)
+    from bmnd_gb300 import _abi
+
+    runs = []
+    for precision, launches in ((_abi.MATCH_EXACT, {1}), (_abi.MATCH_FAST, fast_launches)):
+        before = _abi.launch_count()
+        runs.append(_match(cuda, native, vol, block, radius, max_m, min_m, thr, code, precision, refs, **kw))
+        assert _abi.launch_count() - before in launches
+    for want, got in zip(*runs):
+        np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("shape,block,radius", [((72, 80), (8, 8), (19, 19)), ((61, 150), (8, 8), (5, 30)),
+                                                ((30, 34, 38), (5, 5, 5), (7, 7, 7)),
+                                                ((32, 30, 36), (4, 4, 4), (7, 3, 5))])
+@pytest.mark.parametrize("kind,max_m,frac", [("smooth", 32, 0.4), ("noise", 16, 3.0), ("offset", 32, 0.05)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_tensor_core_ssd_of_sparse_references(cuda, native, shape, block, radius, kind, max_m, frac, bias):
+    rng = np.random.default_rng(zlib.crc32(repr((shape, kind, bias)).encode()))
+    vol = _volume("estimate", shape, rng)
+    if kind == "noise":
+        vol = rng.normal(10.0, 3.0, size=shape)
+    elif kind == "offset":  # small distances under large norms
+        vol = 3000.0 + 0.2 * vol
+    vol = vol.astype(np.float32)
+    P = int(np.prod(block))
+    thr = frac * P * (float(vol.max() - vol.min()) / 8.0) ** 2
+    noise = rng.uniform(0.0, 2.0, size=int(np.prod([2 * r + 1 for r in radius]))) * P if bias else None
+    # norms, tile means and lists, screening, selection, exact kernel
+    _both(cuda, native, vol, block, radius, max_m, 2, thr, SSD, _sparse(shape, block, rng), range(5, 20),
+          noise=noise, gamma=1.5)
+
+
+@pytest.mark.parametrize("shape,block,radius", [((60, 64), (8, 8), (19, 19)), ((26, 28, 30), (5, 5, 5), (7, 7, 7)),
+                                                ((28, 30, 26), (4, 4, 4), (7, 7, 7)), ((20, 18, 21), (3, 4, 2), (5, 4, 6))])
+@pytest.mark.parametrize("kind,max_m,min_m,thr", [("estimate", 32, 2, 0.3937), ("low", 16, 2, 0.7689),
+                                                  ("counts", 16, 2, 2.9527), ("zeros", 32, 2, 0.7689),
+                                                  ("estimate", 8, 4, 0.0)])
+def test_screened_matching_of_sparse_references(cuda, native, shape, block, radius, kind, max_m, min_m, thr):
+    rng = np.random.default_rng(zlib.crc32(repr((shape, kind, max_m)).encode()))
+    vol = _volume(kind, shape, rng).astype(np.float32)
+    # screening with rescoring, then the exact kernel; a count scale keeps exact requests from the tabulated terms
+    _both(cuda, native, vol, block, radius, max_m, min_m, thr, DEV, _sparse(shape, block, rng), {2}, scale=1.25)
+
+
+@pytest.mark.parametrize("shape,block,radius", SHAPES)
+@pytest.mark.parametrize("kind,max_m,min_m,frac", [("estimate", 32, 2, 0.02), ("zeros", 32, 2, 0.4), ("low", 6, 4, 1e-7)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_box_ssd_of_few_dense_references(cuda, native, shape, block, radius, kind, max_m, min_m, frac, bias):
+    """Precision fast takes the box-sum kernels whatever the number of references;
+    exact requests of so few leave them to the exact kernel."""
+    from bmnd_gb300 import _abi
+
+    rng = np.random.default_rng(zlib.crc32(repr((shape, kind, bias)).encode()))
+    vol = (_volume(kind, shape, rng) - 11.0).astype(np.float32)
+    refs = _refs(shape, block, rng)
+    P = int(np.prod(block))
+    noise = rng.uniform(0.0, 2.0, size=int(np.prod([2 * r + 1 for r in radius]))) * P if bias else None
+    args = (radius, max_m, min_m, frac * P * 4.0, SSD)
+    got = _match(cuda, native, vol, block, *args, _abi.MATCH_FAST, refs, noise=noise, gamma=0.7)
+    want = _few_at_a_time(cuda, native, vol, block, *args, _abi.MATCH_EXACT, refs=refs, noise=noise, gamma=0.7)
+    for k in (1, 2, 0):
+        np.testing.assert_array_equal(got[k], want[k])
