@@ -11,6 +11,7 @@ import zlib
 
 import numpy as np
 import pytest
+from test_gpu_blockmatch import _patch_table, gpu_match_patches
 from test_gpu_box_matching import DEV, SHAPES, SSD, _few_at_a_time, _match, _refs, _volume
 
 pytestmark = pytest.mark.gpu
@@ -84,5 +85,33 @@ def test_box_ssd_of_few_dense_references(cuda, native, shape, block, radius, kin
     args = (radius, max_m, min_m, frac * P * 4.0, SSD)
     got = _match(cuda, native, vol, block, *args, _abi.MATCH_FAST, refs, noise=noise, gamma=0.7)
     want = _few_at_a_time(cuda, native, vol, block, *args, _abi.MATCH_EXACT, refs=refs, noise=noise, gamma=0.7)
+    for k in (1, 2, 0):
+        np.testing.assert_array_equal(got[k], want[k])
+
+
+@pytest.mark.parametrize("shape,block,radius", SHAPES[:1] + SHAPES[3:5])
+@pytest.mark.parametrize("kind,max_m,min_m,thr", [
+    ("counts", 16, 2, 2.9527), ("bright", 16, 3, 2.9527), ("zeros", 32, 2, 0.7689), ("zeros", 7, 4, 0.0),
+    ("background", 16, 2, 2.9527), ("background", 32, 4, 0.0), ("tinies", 16, 2, 2.9527), ("overflow", 16, 2, 2.0),
+])
+def test_log_form_equals_patch_table(cuda, native, shape, block, radius, kind, max_m, min_m, thr):
+    """The screening of integer counts (precision fast takes it whatever the number
+    of references), also over an empty background, whose candidates tie, and with
+    values far below one among the zeros' candidates."""
+    from bmnd_gb300 import _abi
+
+    rng = np.random.default_rng(zlib.crc32(repr((shape, kind, max_m)).encode()))
+    if kind in ("background", "tinies"):
+        grids = np.meshgrid(*[np.linspace(-1, 1, s) for s in shape], indexing="ij")
+        vol = rng.poisson(np.where(grids[0] ** 2 + grids[-1] ** 2 < 0.5, 6.0, 0.0)).astype(np.float32)
+        if kind == "tinies":
+            some = rng.random(shape) < 0.002
+            vol[some & (vol == 0)] = rng.choice([1e-40, 1e-31, 1e-20, 1e-7, 1e-3, 0.3], size=int((some & (vol == 0)).sum()))
+    else:
+        vol = _volume(kind, shape, rng).astype(np.float32)
+    refs = _refs(shape, block, rng)
+    got = _match(cuda, native, vol, block, radius, max_m, min_m, thr, DEV, _abi.MATCH_FAST, refs)
+    patches, counts = _patch_table(vol, block)
+    want = gpu_match_patches(cuda, native, patches, counts, refs, radius, max_m, min_m, thr, DEV)
     for k in (1, 2, 0):
         np.testing.assert_array_equal(got[k], want[k])
