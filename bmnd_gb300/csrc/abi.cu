@@ -277,7 +277,8 @@ StageWorkspace carve(const BmndStageParams& sp, int64_t n_refs, void* base) {
     w.ssd_bytes = box.least ? 0 : ssd_tc_scratch_bytes(mp, sp.block, n_refs, sp.ssd_poisson_bias != 0);
     uint64_t o_ssd = take(w.ssd_bytes > 0 ? w.ssd_bytes : 16);
     w.bytes = off;
-    w.box_bytes = det && w.agg.bytes >= box.least ? 0 : box.full;
+    // (with less than half of what it asks for, its chunks of references get short)
+    w.box_bytes = det && w.agg.bytes >= box.full / 2 ? 0 : box.full;
     if (base) {
         char* b = static_cast<char*>(base);
         w.num = det ? nullptr : reinterpret_cast<double*>(b + o_num);

@@ -1844,9 +1844,7 @@ int32_t launch(MatchArgs& a, int code, int precision, cudaStream_t stream) {
                            precision == BMND_MATCH_REAL_VALUED) &&
                           a.max_m <= 32 && screened_smem_bytes(a.max_m, a.P, wmax) <= 200 * 1024;
     if (!screened) {
-        const bool counts = code == BMND_DIST_POISSON_DEVIANCE && a.use_table && !a.table && !a.fixup &&
-                            a.P <= 128 && a.max_m + a.required <= 48 && counts_smem_bytes(a) <= 96 * 1024;
-        return counts ? launch_counts(a, stream) : launch_exact(a, code, stream);
+        return counts_kernel_applies(a, code) ? launch_counts(a, stream) : launch_exact(a, code, stream);
     }
     size_t smem = screened_smem_bytes(a.max_m, a.P, wmax);
     // approximate mode on a volume: per-voxel c and per-origin box sums of
@@ -1949,6 +1947,11 @@ int32_t launch(MatchArgs& a, int code, int precision, cudaStream_t stream) {
 }
 
 }  // namespace
+
+bool counts_kernel_applies(const MatchArgs& a, int code) {
+    return code == BMND_DIST_POISSON_DEVIANCE && a.use_table && !a.table && !a.fixup && a.P <= 128 &&
+           a.max_m + a.required <= 48 && counts_smem_bytes(a) <= 96 * 1024;
+}
 
 int32_t launch_exact(MatchArgs& a, int code, cudaStream_t stream) {
     if (a.n_refs == 0) return BMND_OK;

@@ -1320,9 +1320,60 @@ struct BoxPlan {
     // scratch: origin map and column flags, the counts' box sums, the rows of a chunk of references
     uint64_t o_flag, o_fvox, o_fbox, o_rows, per_ref;
     uint64_t least, full;  // bytes: for a few references at a time, for chunks of up to kRowScratch
+    int64_t chunk(const MatchArgs& a, uint64_t bytes) const {
+        return std::min<int64_t>(static_cast<int64_t>((bytes - o_rows - 1024) / per_ref), a.n_refs);
+    }
 };
 
-BoxPlan plan_box_match(const MatchArgs& a, int code, int precision) {
+// Whether sharing row terms beats the kernel that would run instead.  The row
+// kernels work on all origins in the columns that hold references, the others on
+// the references alone, so it takes dense references.  Measured on one GB300, the
+// other kernel's ms against this file's (matching alone, no scratch allocated):
+//   * bounded screening, and exact terms of values that are no counts, lose at
+//     every density down to one reference per 64 origins, where the list ends
+//     (1024 x 1000, one per 63: 1.70 / 1.11; 128 x 120 x 132, 4x4x4, one per 60:
+//     5.78 / 4.06; terms of counts at a scale of 1.5: 2 to 4 times);
+//   * tabulated terms of counts: 1024 x 1000 one per 16 2.85 / 2.02, one per 25
+//     1.86 / 1.73, one per 36 1.30 / 1.59; 420 x 388 one per 16 0.45 / 0.41, one per
+//     24 0.29 / 0.36; 64 x 64 34 / 115 us; 128 x 120 x 132, 4x4x4, one per 33 6.23 /
+//     4.14, one per 44 4.69 / 3.96, one per 53 with every other column used 3.84 /
+//     5.90; 72 x 76 x 70, one per 31 1.10 / 0.93, one per 41 0.84 / 0.90, 5x5x5
+//     1.60 / 1.34.  Windows of 29^3 lose (5x5x5, 85.6 / 94.5; 23^3: 35.0 / 35.6);
+//   * exact SSD, a warp per reference: windows below a hundred offsets in 3-D lose
+//     (128 x 120 x 132, 3^3: 0.35 / 0.54 ms), small ones of few references (72 x 76
+//     x 70, 5x5x5, 5^3: 0.19 / 0.31; 420 x 388, 11^2: 0.147 / 0.149), and sparse ones
+//     in 2-D (one per 47 0.23 / 0.21, one per 61 0.16 / 0.21).  In 3-D sparse ones win
+//     where the last axis is among the sparse (72 x 76 x 70, 4x4x4, steps 4, 4, 4
+//     0.72 / 0.55, steps 6, 5, 2 0.74 / 0.86), which is not known here.  Where the
+//     scratch has to be allocated, which takes 0.1 ms and 0.9 ms per GB, 2-D needs
+//     more references (6.4 K: 0.34 / 0.37; 9.9 K: 0.51 / 0.39) and wider windows.
+// Real-valued stages come here whatever their size: few references gain 0.1 ms at
+// best in the screened kernel, and those it cannot settle cost 3.1 ms there
+// (24 x 24 x 40, peak 30; here 0.5 in all).
+bool pays_off(const MatchArgs& a, const BoxArgs& b, int code, int precision, bool allocates, int64_t n_lins) {
+    if (a.n_refs * 64 < n_lins) return false;
+    if (precision != BMND_MATCH_EXACT) return true;
+    const int64_t window = static_cast<int64_t>(b.nz) * b.ny * b.nx;
+    if (code == BMND_DIST_SSD) {
+        if (a.ndim == 2 && a.n_refs < std::max<int64_t>(allocates ? 8192 : 0, n_lins / 50)) return false;
+        return window >= 343 || ((a.ndim == 2 || window >= 100) && a.n_refs * window >= (allocates ? 10000000 : 2500000));
+    }
+    if (!counts_kernel_applies(a, code)) return true;
+    const int64_t least = a.ndim == 2 ? 4096 + n_lins / (allocates ? 25 : 28)
+                                      : std::max<int64_t>(8192, a.P == 64 ? 4096 + n_lins / 52 : n_lins / 48);
+    return a.n_refs >= least && b.rowlen <= 20000;
+}
+
+// First-axis extent of a chunk of references against the patch edge W: a tile's
+// halo of W - 1 origins is computed again for every chunk.  Exact SSD and tabulated
+// counts, which lose little to this file's kernels at wide windows, take over from
+// short chunks (5x5x5, SSD, 41^3 offsets, 16 origins a chunk: 43.5 ms, here 47.0).
+bool chunks_pay_off(const MatchArgs& a, const BoxArgs& b, int W, int code, int precision, int64_t chunk) {
+    if (precision != BMND_MATCH_EXACT || (code != BMND_DIST_SSD && !counts_kernel_applies(a, code))) return true;
+    return chunk >= a.n_refs || b.cnt[0] * chunk >= 4 * W * a.n_refs;
+}
+
+BoxPlan plan_box_match(const MatchArgs& a, int code, int precision, bool allocates) {
     BoxPlan p{};
     BoxArgs& b = p.b;
     const bool ssd = code == BMND_DIST_SSD;
@@ -1354,20 +1405,9 @@ BoxPlan plan_box_match(const MatchArgs& a, int code, int precision) {
     b.noise = a.noise_ssd;
     b.gamma = a.gamma;
     const int64_t n_lins = static_cast<int64_t>(b.cnt[0]) * b.cnt[1] * b.cnt[2];
-    // the shared terms pay off while references are dense: up to one per 64
-    // origins (the schedules have one per 4.5 to 27)
-    if (b.rowlen > (1 << 20) || a.n_refs * 64 < n_lins || a.n_refs > 0x7fffffffLL) return p;
-    // Few references of a stage on counts: the kernel of tabulated terms has no
-    // phases that wait on each other.  One GB300, that kernel against this file's:
-    // 64 x 64 34 against 115 us, 140 x 140 (3.9 K references) 164 against 169,
-    // 200 x 180 (7.5 K) 312 against 214; 40 x 49 x 66 (4.4 K) 454 against 590,
-    // 51 x 65 x 74 (9 K) 955 against 918, 72 x 80 x 60 1359 against 1086.
-    // Real-valued stages come here whatever their size: few references gain
-    // 0.1 ms at best in the screened kernel, and those it cannot settle cost
-    // 3.1 ms there (24 x 24 x 40, peak 30; here 0.5 in all).
     p.want_f = !ssd && precision != BMND_MATCH_REAL_VALUED && a.inv_scale == 1.0f;
-    const bool few = a.n_refs < (shape2 ? 4096 : 8192);
-    if (p.want_f && precision == BMND_MATCH_EXACT && a.use_table && few) return p;
+    if (b.rowlen > (1 << 20) || a.n_refs > 0x7fffffffLL || !pays_off(a, b, code, precision, allocates, n_lins))
+        return p;
 
     // tiles: the largest whose shared memory fits; first-axis offsets are split
     // over CTAs until every SM has several
@@ -1412,34 +1452,32 @@ BoxPlan plan_box_match(const MatchArgs& a, int code, int precision) {
     p.per_ref = 4ull * b.rowlen + 20;
     p.least = p.o_rows + 1024 + p.per_ref * std::min<int64_t>(a.n_refs, 512);
     p.full = std::max(p.least, p.o_rows + 1024 + std::min<uint64_t>(p.per_ref * a.n_refs, kRowScratch));
-    p.applies = true;
+    p.applies = chunks_pay_off(a, b, W, code, precision, p.chunk(a, p.full));
     return p;
 }
 
 }  // namespace
 
 BoxScratch box_match_scratch(const MatchArgs& a, int code, int precision) {
-    const BoxPlan p = plan_box_match(a, code, precision);
+    const BoxPlan p = plan_box_match(a, code, precision, false);
     return p.applies ? BoxScratch{p.least, p.full} : BoxScratch{0, 0};
 }
 
 int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t stream, bool* done) {
     *done = false;
-    const BoxPlan p = plan_box_match(a, code, precision);
+    const BoxPlan p = plan_box_match(a, code, precision, !a.box_ws);
     if (!p.applies) return BMND_OK;
     BoxArgs b = p.b;
     const bool ssd = code == BMND_DIST_SSD, want_f = p.want_f;
     const bool shape2 = a.ndim == 2, shape5 = a.ndim == 3 && a.block[0] == 5;
     const int64_t n_lins = static_cast<int64_t>(b.cnt[0]) * b.cnt[1] * b.cnt[2];
-    char* base = nullptr;
-    uint64_t bytes = 0;
+    const bool given = a.box_ws && a.box_ws_bytes >= p.least;
+    char* base = given ? a.box_ws : nullptr;
+    int64_t chunk = p.chunk(a, given ? a.box_ws_bytes : p.full);
+    if (!chunks_pay_off(a, b, shape2 ? 8 : (shape5 ? 5 : 4), code, precision, chunk)) return BMND_OK;
     bool owned = false;
-    if (a.box_ws && a.box_ws_bytes >= p.least) {
-        base = a.box_ws;
-        bytes = a.box_ws_bytes;
-    } else if (!a.no_alloc) {
-        bytes = p.full;
-        if (cudaMallocAsync(reinterpret_cast<void**>(&base), bytes, stream) == cudaSuccess) {
+    if (!given && !a.no_alloc) {
+        if (cudaMallocAsync(reinterpret_cast<void**>(&base), p.full, stream) == cudaSuccess) {
             owned = true;
             note_device_alloc();
         } else {
@@ -1448,8 +1486,6 @@ int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t str
         }
     }
     if (!base) return BMND_OK;
-    int64_t chunk = static_cast<int64_t>((bytes - p.o_rows - 1024) / p.per_ref);
-    if (chunk > a.n_refs) chunk = a.n_refs;
     const int64_t nchunks = (a.n_refs + chunk - 1) / chunk;
     chunk = (a.n_refs + nchunks - 1) / nchunks;
     b.map = reinterpret_cast<int32_t*>(base);

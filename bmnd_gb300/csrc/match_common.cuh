@@ -159,6 +159,9 @@ __device__ __forceinline__ float ratio_term(float r, float r2, float c, float& s
 // a.fixup set only the references whose count is negative are (re)done
 int32_t launch_exact(MatchArgs& a, int code, cudaStream_t stream);
 
+// whether exact requests take the kernel of tabulated count terms (blockmatch.cu)
+bool counts_kernel_applies(const MatchArgs& a, int code);
+
 // Box-sum matching (boxmatch.cu): *done is set when it ran; the references it
 // leaves to the exact kernel have count = -1
 int32_t launch_box_match(MatchArgs& a, int code, int precision, cudaStream_t stream, bool* done);

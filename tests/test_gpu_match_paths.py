@@ -115,3 +115,30 @@ def test_log_form_equals_patch_table(cuda, native, shape, block, radius, kind, m
     want = gpu_match_patches(cuda, native, patches, counts, refs, radius, max_m, min_m, thr, DEV)
     for k in (1, 2, 0):
         np.testing.assert_array_equal(got[k], want[k])
+
+
+@pytest.mark.parametrize("shape,block,radius,step,code,boxed", [
+    ((420, 388), (8, 8), (19, 19), (3, 3), DEV, True), ((420, 388), (8, 8), (19, 19), (6, 6), DEV, False),
+    ((72, 76, 70), (4, 4, 4), (7, 7, 7), (3, 3, 3), DEV, True), ((72, 76, 70), (4, 4, 4), (7, 7, 7), (3, 4, 4), DEV, False),
+    ((72, 76, 70), (4, 4, 4), (7, 14, 29), (3, 3, 3), DEV, False), ((72, 76, 70), (5, 5, 5), (7, 7, 7), (3, 3, 3), SSD, True),
+    ((72, 76, 70), (5, 5, 5), (1, 1, 1), (3, 3, 3), SSD, False), ((72, 76, 70), (4, 4, 4), (7, 7, 7), (4, 4, 4), SSD, True),
+    ((420, 388), (8, 8), (5, 5), (3, 3), SSD, False), ((140, 140), (8, 8), (19, 19), (3, 3), SSD, False),
+])
+def test_exact_requests_take_the_faster_kernel(cuda, native, shape, block, radius, step, code, boxed):
+    """Sparse counts, small windows and short chunks stay with the kernels of one
+    reference at a time; both routes give the same tables (precision fast takes
+    the box sums)."""
+    from bmnd_gb300 import _abi
+
+    rng = np.random.default_rng(zlib.crc32(repr((shape, radius, step)).encode()))
+    vol = _volume("counts", shape, rng).astype(np.float32)
+    axes = [np.unique(np.r_[0:s - b + 1:t, s - b]) for s, b, t in zip(shape, block, step)]
+    refs = np.stack(np.meshgrid(*axes, indexing="ij"), -1).reshape(-1, len(shape)).astype(np.int32)
+    args = (radius, 16, 2, 2.9527 if code == DEV else 30.0 * np.prod(block), code)
+    before = _abi.launch_count()
+    got = _match(cuda, native, vol, block, *args, _abi.MATCH_EXACT, refs)
+    # tabulated terms: 2 launches; exact: 1; box sums: 5 and more
+    assert (_abi.launch_count() - before >= 5) == boxed
+    want = _match(cuda, native, vol, block, *args, _abi.MATCH_FAST, refs)
+    for k in (1, 2, 0):
+        np.testing.assert_array_equal(got[k], want[k])
