@@ -37,8 +37,11 @@
 // 4.4 ms against 15.0, 768 x 640 2.2 ms against 15.2 (tensor-core products).
 // A low-count volume's smooth estimate leaves hundreds of candidates per
 // reference open: 90^3 at peak 5, both stages 15.3 ms against 19.4.
-// The row kernels are bound by FP32 issue and shared-memory loads (log form:
-// the SFU), the selection by the latency of its short dependent phases.
+// No pipe is full (72 x 76 x 70, ncu): the row kernels issue 0.62-0.65 instructions
+// per clock and scheduler with the 4 warps that 128 registers leave it (5x5x5 spills
+// 216 bytes), waiting for shared-memory loads and dependent results; load/store pipe
+// 44 %, FMA 30 %, log form's SFU 30 %.  The selection issues 0.80 (ALU 48 %, FMA
+// 40 %): instructions bound it, its heavy form (0.61) the latency of its row loads.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
