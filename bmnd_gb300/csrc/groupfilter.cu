@@ -118,7 +118,14 @@ __host__ inline int64_t padded_patch(const BmndStageParams& sp, int P) {
     return sp.ndim == 2 && specialised_shape(sp) ? padded<8>(P) : P;
 }
 
-__host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax, int64_t ucells, bool sigma) {
+// exact planes' G entries in pairs (g, g) for packed products
+__host__ inline int64_t pair_bytes(int nmax, int kmax) {
+    return kmax > 0 ? 8 * static_cast<int64_t>(nmax) * ((kmax + 3) / 4 * 4) : 16;
+}
+
+// `early`: the pairs have a place of their own; else one that the group buffers, or
+// hard thresholding's sigmas, take after the exact variance
+__host__ Layout layout_of(const BmndStageParams& sp, int P, int nmax, int kmax, int64_t ucells, bool sigma, bool early) {
     Layout L{};
     int64_t off = 0;
     auto round16 = [](int64_t b) { return (b + 15) & ~int64_t(15); };
@@ -132,14 +139,9 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     const bool wiener = sp.filter == BMND_FILTER_WIENER;
     const bool gauss = sp.noise_model == BMND_NOISE_GAUSSIAN;
     const bool keep = sp.exact_risk_weights != 0;
-    // exact planes' G entries in pairs (g, g) for packed products: the exact risk
-    // reads them after the shrinkage, the exact variance before (they may lie behind
-    // its lists, see below), stationary Gaussian noise without it never
-    const bool early = keep || specialised_shape(sp);  // the entries count from the start of shared memory
-    const int kpad = (kmax + 3) / 4 * 4;
-    const int64_t gt2_bytes = 8 * static_cast<int64_t>(nmax) * kpad;
+    const int64_t gt2_bytes = pair_bytes(nmax, kmax);
     L.g = take(4 * nmax * nmax);
-    if (early) L.gt2 = take(gt2_bytes > 0 ? gt2_bytes : 16);
+    if (early) L.gt2 = take(gt2_bytes);
     L.fw = take(4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE);
     L.fi = take(4 * BMND_MAX_DIMS * BMND_MAX_EDGE * BMND_MAX_EDGE);
     // group-mass conservation: transposed inverse spatial matrices, and the
@@ -157,7 +159,8 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.shf = take(4 * nmax * BMND_MAX_DIMS);
     L.shl = take(4 * nmax);
     // hard thresholding with a sigma map keeps each coefficient's sigma until the scatter
-    L.sg = take(sigma && !wiener ? 4 * npp : 16);
+    const int64_t sg_bytes = sigma && !wiener ? 4 * npp : 16;
+    L.sg = take(sg_bytes);
     L.ex = take(4 * static_cast<int64_t>(kmax) * P);
 
     L.scan = take(8 * (kThreads / 32 + 1));  // the warps' totals, then the block's
@@ -167,6 +170,11 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     L.risk = take(8 * (kThreads / 32 + 1));  // exact risk: per-warp partial sums, then the total
     // union region
     L.uni = off;
+    int64_t lists = L.uni;
+    if (!early) {
+        L.gt2 = sg_bytes >= gt2_bytes ? L.sg : lists;
+        if (L.gt2 == lists) lists += round16(gt2_bytes);
+    }
     const int64_t buf = round16(4 * npp);
     L.s = L.uni;
     L.x = L.s + buf;
@@ -195,24 +203,31 @@ __host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax
     // width: the default profiles) the lists are done with by then and give
     // theirs.  (Apart from the union region they made 8x8x8 patches at the default
     // stack of 32 need 233 728 bytes, above the limit of 232 448; so, 216 304.)
-    const int tile_w = 32 * kron_jr(P);
-    const int64_t part_bytes = !gauss && kmax > 0 ? 4 * (kThreads / 32) * 4 * static_cast<int64_t>(tile_w) : 0;
-    L.part_over = !keep && kmax <= 4 && P <= tile_w;
-    const int64_t ahead = keep ? (group_bytes > part_bytes ? group_bytes : part_bytes) : 0;
-    L.grid = L.uni + ahead;
+    if (keep) lists = L.uni + group_bytes;
+    L.grid = lists;
     L.lval = L.grid + round16(kl > 0 ? 4 * axis_masks : 0);
     L.lstart = L.lval + round16(4 * umax);
     L.lent = L.lstart + round16(4 * (umax + 1));
     int64_t end = L.lent + round16(kl > 0 ? 4 * (np + 2) : 0);
-    if (!early) {
-        L.gt2 = end;
-        if (kl > 0) end += gt2_bytes;
-    }
-    L.part = keep ? L.uni : (L.part_over ? L.grid : end);
-    if (!keep && end < L.part + part_bytes) end = L.part + part_bytes;
+    const int tile_w = 32 * kron_jr(P);
+    const int64_t part_bytes = !gauss && kmax > 0 ? 4 * (kThreads / 32) * 4 * static_cast<int64_t>(tile_w) : 0;
+    L.part_over = !keep && kmax <= 4 && P <= tile_w;
+    L.part = L.part_over ? L.grid : end;
+    if (end < L.part + part_bytes) end = L.part + part_bytes;
     off = end > L.uni + group_bytes ? end : L.uni + group_bytes;
     L.total = off;
     return L;
+}
+
+// The exact risk reads the pairs after the shrinkage, so there they keep a place of
+// their own, and in the specialised shapes, which are far from the limit; the
+// entries' 16-bit offsets must reach them.
+__host__ Layout make_layout(const BmndStageParams& sp, int P, int nmax, int kmax, int64_t ucells, bool sigma) {
+    if (!sp.exact_risk_weights && !specialised_shape(sp)) {
+        const Layout L = layout_of(sp, P, nmax, kmax, ucells, sigma, false);
+        if (L.gt2 + pair_bytes(nmax, kmax) <= 0x10000) return L;
+    }
+    return layout_of(sp, P, nmax, kmax, ucells, sigma, true);
 }
 
 template <bool V>
@@ -986,9 +1001,9 @@ struct PlaneVec {
 template <int RL, int NQ>
 __device__ __forceinline__ void exact_stream(const float* __restrict__ lval, const int* __restrict__ lstart,
                                              const uint32_t* __restrict__ lent, int u_lo, int u_hi,
-                                             const unsigned char* base, uint32_t plane_byte, uint32_t stride,
+                                             const unsigned char* smem, uint32_t plane_byte, uint32_t stride,
                                              const float* __restrict__ stl, float (&var)[RL][NQ]) {
-    const unsigned char* gb = base + plane_byte;
+    const unsigned char* gb = smem + plane_byte;
 #pragma unroll
     for (int r = 0; r < RL; ++r)
 #pragma unroll
@@ -1048,8 +1063,8 @@ __device__ __forceinline__ void exact_stream(const float* __restrict__ lval, con
 // multiply-adds per instruction, each rounded as its scalar form).  It is bound
 // by instruction issue, so addresses are kept in 32-bit shared-memory form (the
 // generic 64-bit pointers cost more integer instructions than the products):
-// an entry word holds the byte offset of the member's entries in the table of
-// paired G entries and the patch element; two words past the last one are readable.  A
+// an entry word holds the shared-memory byte offset of the member's paired G
+// entries and the patch element; two words past the last one are readable.  A
 // voxel's first entry starts its sums with a product.
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     uint32_t v;
@@ -1084,14 +1099,14 @@ __device__ __forceinline__ void load_row(float2 (&sv)[2], const char* row0, uint
 }
 
 template <int NQ>
-__device__ __forceinline__ void exact_pairs(const unsigned char* base, const float* lval, const int* lstart,
+__device__ __forceinline__ void exact_pairs(const unsigned char* smem, const float* lval, const int* lstart,
                                             const uint32_t* lent, int u_lo, int u_hi, uint32_t plane_byte,
                                             const float* __restrict__ st, uint32_t stride_b,
                                             float2 (&var)[2][NQ]) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) var[0][q] = var[1][q] = make_float2(0.0f, 0.0f);
     if (u_lo >= u_hi) return;
-    const uint32_t plane = static_cast<uint32_t>(__cvta_generic_to_shared(base)) + plane_byte;
+    const uint32_t plane = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + plane_byte;
     const uint32_t ents = static_cast<uint32_t>(__cvta_generic_to_shared(lent));
     uint32_t ls = static_cast<uint32_t>(__cvta_generic_to_shared(lstart + u_lo));
     const uint32_t lv = static_cast<uint32_t>(__cvta_generic_to_shared(lval)) -
@@ -1297,7 +1312,7 @@ __device__ __forceinline__ void exact_haar(const float* lval, const int* lstart,
 // halves' sums are added at the end.  (A whole warp per half, without the
 // divergence where only one half ends a voxel, took 14 % more instructions.)
 template <int JR, int NQ, bool HAAR>
-__device__ void exact_planes(const unsigned char* base, float a0, float b0, uint32_t kron_byte, const float* __restrict__ lval,
+__device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint32_t kron_byte, const float* __restrict__ lval,
                              const int* __restrict__ lstart, const uint32_t* __restrict__ lent, int U,
                              int kk, const float* __restrict__ st, int P,
                              float* __restrict__ EX, float* __restrict__ part, bool part_over) {
@@ -1328,7 +1343,7 @@ __device__ void exact_planes(const unsigned char* base, float a0, float b0, uint
                 // sums are added as in the generic form below)
                 constexpr int RP = JR / 2;
                 const int u_mid = JR == 2 ? first_voxel((lstart[u_lo] + lstart[u_hi]) >> 1, u_lo, u_hi) : u_hi;
-                const uint32_t kron_lane = static_cast<uint32_t>(__cvta_generic_to_shared(base)) + kron_byte + 8u * lane;
+                const uint32_t kron_lane = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + kron_byte + 8u * lane;
                 float2 var[RP][NQ];
                 exact_haar<RP, NQ>(lval, lstart, lent, u_lo, u_mid, a0, b0, st + JR * lane, kron_lane, var);
 #pragma unroll
@@ -1347,7 +1362,7 @@ __device__ void exact_planes(const unsigned char* base, float a0, float b0, uint
                     }
                 }
             } else if constexpr (JR == 1) {
-                exact_stream<1, NQ>(lval, lstart, lent, u_lo, u_hi, base, 8u * i0, stride, st + j0 + lane, out);
+                exact_stream<1, NQ>(lval, lstart, lent, u_lo, u_hi, smem, 8u * i0, stride, st + j0 + lane, out);
             } else {
                 float2 var[2][NQ];
                 int lo = u_lo, hi = u_hi;
@@ -1357,7 +1372,7 @@ __device__ void exact_planes(const unsigned char* base, float a0, float b0, uint
                     if (lane >> 4) lo = u_mid;
                     else hi = u_mid;
                 }
-                exact_pairs<NQ>(base, lval, lstart, lent, lo, hi, 8u * i0, st + j0 + jl, 4u * stride, var);
+                exact_pairs<NQ>(smem, lval, lstart, lent, lo, hi, 8u * i0, st + j0 + jl, 4u * stride, var);
 #pragma unroll
                 for (int q = 0; q < NQ; ++q)
 #pragma unroll
@@ -1396,15 +1411,15 @@ __device__ void exact_planes(const unsigned char* base, float a0, float b0, uint
 }
 
 template <int JR>
-__device__ void exact_planes_any(const unsigned char* base, bool haar, float a0, float b0, uint32_t kron_byte,
+__device__ void exact_planes_any(const unsigned char* smem, bool haar, float a0, float b0, uint32_t kron_byte,
                                  const float* __restrict__ lval, const int* __restrict__ lstart,
                                  const uint32_t* __restrict__ lent, int U, int kk, const float* __restrict__ st, int P,
                                  float* __restrict__ EX, float* __restrict__ part, bool part_over) {
     auto run = [&](auto h) {
         constexpr bool H = decltype(h)::value;
-        if (kk == 1) exact_planes<JR, 1, H>(base, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
-        else if (kk == 2) exact_planes<JR, 2, H>(base, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
-        else exact_planes<JR, 4, H>(base, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        if (kk == 1) exact_planes<JR, 1, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        else if (kk == 2) exact_planes<JR, 2, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        else exact_planes<JR, 4, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
     };
     if (JR > 1 && haar) run(BoolTag<JR != 1>{});
     else run(BoolTag<false>{});
@@ -1419,7 +1434,7 @@ __device__ void exact_planes_any(const unsigned char* base, bool haar, float a0,
 // one tile); (f SM)[j] = sum_p f[p] SM[p][j] takes f[p] from its lane by a
 // shuffle.  The voxel terms are float32, their sum over voxels float64.
 template <int JR, int NQ>
-__device__ double exact_risk_tile(const unsigned char* base, const float* __restrict__ lval, const int* __restrict__ lstart,
+__device__ double exact_risk_tile(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
                                   const uint32_t* __restrict__ lent, int u_lo, int u_hi,
                                   int i0, int kk,
                                   const float* __restrict__ st, const float* __restrict__ smt,
@@ -1443,7 +1458,7 @@ __device__ double exact_risk_tile(const unsigned char* base, const float* __rest
         {
             const uint32_t ent = lent[e];
             PlaneVec<NQ> gv;
-            gv.load_pairs(base + 8 * i0 + (ent & 0xffffu));
+            gv.load_pairs(smem + 8 * i0 + (ent & 0xffffu));
             KronVec<JR> sv;
             sv.load(stl + (ent >> 16) * static_cast<uint32_t>(stride));
 #pragma unroll
@@ -1454,7 +1469,7 @@ __device__ double exact_risk_tile(const unsigned char* base, const float* __rest
         for (++e; e < e1; ++e) {
             const uint32_t ent = lent[e];
             PlaneVec<NQ> gv;
-            gv.load_pairs(base + 8 * i0 + (ent & 0xffffu));
+            gv.load_pairs(smem + 8 * i0 + (ent & 0xffffu));
             KronVec<JR> sv;
             sv.load(stl + (ent >> 16) * static_cast<uint32_t>(stride));
 #pragma unroll
@@ -1501,7 +1516,7 @@ __device__ double exact_risk_tile(const unsigned char* base, const float* __rest
 // warp w takes the voxels whose entry lists start in its share of all entries
 // (the exact variance's split); lanes, then warps, add in a fixed order
 template <int JR, int NQ>
-__device__ void exact_risk(const unsigned char* base, const float* __restrict__ lval, const int* __restrict__ lstart,
+__device__ void exact_risk(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
                            const uint32_t* __restrict__ lent, int U, int kk, const float* __restrict__ st, const float* __restrict__ smt,
                            const float* __restrict__ att, int P, double* __restrict__ part) {
     const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
@@ -1520,7 +1535,7 @@ __device__ void exact_risk(const unsigned char* base, const float* __restrict__ 
     const int u_hi = warp == nw - 1 ? U : first_voxel(static_cast<int>(static_cast<int64_t>(E) * (warp + 1) / nw));
     double acc = 0.0;
     for (int i0 = 0; i0 < kk; i0 += NQ)
-        acc += exact_risk_tile<JR, NQ>(base, lval, lstart, lent, u_lo, u_hi, i0, kk, st, smt, att, P);
+        acc += exact_risk_tile<JR, NQ>(smem, lval, lstart, lent, u_lo, u_hi, i0, kk, st, smt, att, P);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) part[warp] = acc;
@@ -1533,14 +1548,17 @@ __device__ void exact_risk(const unsigned char* base, const float* __restrict__ 
     __syncthreads();
 }
 
+// (kept out of line: inlined, its registers and order followed unrelated changes of
+// the kernel, 20.1 to 21.3 ms for stage 1 of 220 x 260; so, 20.2, and stage 2 14.3
+// against 14.6)
 template <int JR>
-__device__ void exact_risk_any(const unsigned char* base, const float* __restrict__ lval, const int* __restrict__ lstart,
+__device__ __noinline__ void exact_risk_any(const unsigned char* smem, const float* __restrict__ lval, const int* __restrict__ lstart,
                                const uint32_t* __restrict__ lent, int U,
                                int kk, const float* __restrict__ st, const float* __restrict__ smt,
                                const float* __restrict__ att, int P, double* __restrict__ part) {
-    if (kk == 1) exact_risk<JR, 1>(base, lval, lstart, lent, U, kk, st, smt, att, P, part);
-    else if (kk == 2) exact_risk<JR, 2>(base, lval, lstart, lent, U, kk, st, smt, att, P, part);
-    else exact_risk<JR, 4>(base, lval, lstart, lent, U, kk, st, smt, att, P, part);
+    if (kk == 1) exact_risk<JR, 1>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
+    else if (kk == 2) exact_risk<JR, 2>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
+    else exact_risk<JR, 4>(smem, lval, lstart, lent, U, kk, st, smt, att, P, part);
 }
 
 // Exact Gaussian variances of planes 0 .. 3 of a Haar group (kk of them): with
@@ -1628,9 +1646,6 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
 
     float* G = sm<float>(smem, a.L.g);
     float2* GT2 = sm<float2>(smem, a.L.gt2);
-    // what the entries' 16-bit offsets into GT2 count from: it may lie above 64 KB
-    // in the runtime geometry
-    const int64_t ent_base = ND > 0 ? 0 : a.L.gt2;
     float* Fw = sm<float>(smem, a.L.fw);
     float* win = sm<float>(smem, a.L.win);
     double* mdiag = sm<double>(smem, a.L.mdiag);
@@ -1738,9 +1753,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         for (int e = tid; e < n * n; e += blockDim.x) G[e] = __ldg(gtab + e);
         // G^T restricted to the exact planes, padded to 4, each entry twice:
         // GT2[g * kpad + i] = (G[i, g], G[i, g])
-        // (the runtime geometry has no room for them where nothing reads them)
-        const bool pairs = !quarters && (ND > 0 || sp.noise_model == BMND_NOISE_POISSON || sp.exact_risk_weights);
-        for (int e = tid; pairs && e < n * kpad; e += blockDim.x) {
+        for (int e = tid; !quarters && e < n * kpad; e += blockDim.x) {
             const int g = e / kpad, i = e % kpad;
             const float v = i < kk ? __ldg(gtab + i * n + g) : 0.0f;
             GT2[e] = make_float2(v, v);
@@ -1961,7 +1974,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             base += incl - mine;
             int w = static_cast<int>(base >> 16), we = static_cast<int>(base & 0xffffu);
             const int* shl = sm<int>(smem, a.L.shl);
-            const uint32_t gt2_off = static_cast<uint32_t>(a.L.gt2 - ent_base), row_b = 4u * static_cast<uint32_t>(kron_stride(P));
+            const uint32_t gt2_off = static_cast<uint32_t>(a.L.gt2), row_b = 4u * static_cast<uint32_t>(kron_stride(P));
             const int lg = ilog2_floor(n);
             walk([&](uint32_t m, int vox, int lin) {
                 reinterpret_cast<int*>(lval)[w] = vox;
@@ -2002,9 +2015,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         } else {
             const int jr = kron_jr(P);
             float* part = sm<float>(smem, a.L.part);
-            if (jr == 1) exact_planes_any<1>(smem + ent_base, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
-            else if (jr == 2) exact_planes_any<2>(smem + ent_base, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
-            else exact_planes_any<4>(smem + ent_base, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            if (jr == 1) exact_planes_any<1>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            else if (jr == 2) exact_planes_any<2>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            else exact_planes_any<4>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
         }
     }
 
@@ -2195,9 +2208,9 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
         if (exact_risk) {
             const float* smt = a.st + static_cast<int64_t>(P) * kron_stride(P);
             const int jr = kron_jr(P);
-            if (jr == 1) exact_risk_any<1>(smem + ent_base, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
-            else if (jr == 2) exact_risk_any<2>(smem + ent_base, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
-            else exact_risk_any<4>(smem + ent_base, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
+            if (jr == 1) exact_risk_any<1>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
+            else if (jr == 2) exact_risk_any<2>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
+            else exact_risk_any<4>(smem, lval, lstart, lent, U, kk, a.st, smt, V, P, riskp);
         }
     }
 
