@@ -2426,7 +2426,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
     });
 }
 
-// One CTA per group.  (Persistent CTAs walking the groups, which would set up the
+// One CTA per group, CTAS resident.  (Persistent CTAs walking the groups, which would set up the
 // constants once, spill: the compiler then keeps 1.9 KB of local memory a thread.)
 // Resident CTAs per SM cover each other's barriers and serial phases: 64
 // registers and 38 KB (16 members) or 56 KB (32) allow four for patches of 64
@@ -2434,8 +2434,12 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
 // ms for 42 K groups of 4x4x4, 14.3 -> 12.6 ms for a Gaussian image); 5x5x5
 // patches hold three, and four where there are no exact planes (55 KB; 17.2 ->
 // 14.8 ms for 250 K groups).
-template <int ND, int B0, int B1, int B2, int NT, bool APPROX = false>
-__global__ void __launch_bounds__(NT, NT != kThreads ? 1 : ND == 2 || B0 == 4 || APPROX ? 4 : ND == 3 ? 3 : 2)
+// 8x8 stages whose exact planes take the general stream (more than four, or no Haar
+// group) hold three: at 64 registers its loop spills and four CTAs of 51 KB leave L1
+// 28 KB for S^T and the volumes (220 x 260, 32 members: 8 planes 3.12 -> 2.75 ms, 16
+// planes 6.69 -> 4.05, 32 planes 8.77 -> 6.61, DCT group 2.50 -> 2.40).
+template <int ND, int B0, int B1, int B2, int NT, int CTAS, bool APPROX = false>
+__global__ void __launch_bounds__(NT, CTAS)
     group_filter_kernel(FilterArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     filter_group<ND, B0, B1, B2, APPROX>(a, smem, blockIdx.x);
@@ -2628,11 +2632,15 @@ int32_t launch_group_filter(const BmndStageParams& sp, const float* noisy, const
         BMND_LAUNCH_CHECK("group_filter_kernel");
         return BMND_OK;
     };
-    if (!specialised_shape(sp)) return run(group_filter_kernel<0, 0, 0, 0, kThreads>, kThreads);
-    if (sp.ndim == 2) return run(group_filter_kernel<2, 8, 8, 1, kThreads>, kThreads);
-    if (sp.block[0] == 4) return run(group_filter_kernel<3, 4, 4, 4, kThreads>, kThreads);
-    return sp.variance_k > 0 ? run(group_filter_kernel<3, 5, 5, 5, kThreads>, kThreads)
-                             : run(group_filter_kernel<3, 5, 5, 5, kThreads, true>, kThreads);
+    if (!specialised_shape(sp)) return run(group_filter_kernel<0, 0, 0, 0, kThreads, 2>, kThreads);
+    if (sp.ndim == 2) {
+        const bool general = a.kmax > 0 && !a.L.kron_used && sp.noise_model == BMND_NOISE_POISSON;
+        return general ? run(group_filter_kernel<2, 8, 8, 1, kThreads, 3>, kThreads)
+                       : run(group_filter_kernel<2, 8, 8, 1, kThreads, 4>, kThreads);
+    }
+    if (sp.block[0] == 4) return run(group_filter_kernel<3, 4, 4, 4, kThreads, 4>, kThreads);
+    return a.kmax > 0 ? run(group_filter_kernel<3, 5, 5, 5, kThreads, 3>, kThreads)
+                      : run(group_filter_kernel<3, 5, 5, 5, kThreads, 4, true>, kThreads);
 }
 
 int32_t launch_finalize_sigma(const BmndStageParams& sp, const double* sig_num, const double* den,
