@@ -1098,7 +1098,12 @@ __device__ __forceinline__ void load_row(float2 (&sv)[2], const char* row0, uint
     sv[1] = make_float2(t.z, t.w);
 }
 
-template <int NQ>
+//
+// D entries' rows are in flight.  Two suffice where S^T lies in L1 or near it; the
+// runtime geometry's tables of more than 64 voxels (1 MB at 8x8x8, one CTA per SM)
+// come from L2, whose latency four cover (44 x 48 x 52, 8x8x8, 32 members: one plane
+// 51.2 -> 37.2 ms, four 57.9 -> 44.6; the scalar stream before the pairs 39.0, 52.7).
+template <int NQ, int D>
 __device__ __forceinline__ void exact_pairs(const unsigned char* smem, const float* lval, const int* lstart,
                                             const uint32_t* lent, int u_lo, int u_hi, uint32_t plane_byte,
                                             const float* __restrict__ st, uint32_t stride_b,
@@ -1119,11 +1124,6 @@ __device__ __forceinline__ void exact_pairs(const unsigned char* smem, const flo
     float2 c[2][NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) c[0][q] = c[1][q] = make_float2(0.0f, 0.0f);
-    float2 g0[NQ], s0[2], g1[NQ], s1[2];
-    uint32_t ent = lds32(ep);
-    load_pairs<NQ>(g0, plane, ent);
-    load_row(s0, row0, ent, stride_b);
-    ent = lds32(ep + 4);
     auto fold = [&]() {
         const float2 vv = make_float2(v, v);
 #pragma unroll
@@ -1132,6 +1132,47 @@ __device__ __forceinline__ void exact_pairs(const unsigned char* smem, const flo
             var[1][q] = __ffma2_rn(__fmul2_rn(vv, c[1][q]), c[1][q], var[1][q]);
         }
     };
+    if constexpr (D > 2) {
+        auto at = [&](int ahead) { return lds32(min(ep + 4u * ahead, end - 4u)); };  // (the last entry again at the end)
+        float2 g[NQ], sv[D][2];
+        uint32_t ent[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            ent[d] = at(d);
+            load_row(sv[d], row0, ent[d], stride_b);
+        }
+        while (true) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                load_pairs<NQ>(g, plane, ent[d]);
+                ent[d] = at(D);
+                if (ep == next) {
+                    fold();
+                    v = __uint_as_float(lds32(ls + lv));
+                    ls += 4;
+                    next = ents + 4u * lds32(ls);
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) c[0][q] = c[1][q] = make_float2(0.0f, 0.0f);
+                }
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {  // (fma(g, s, 0) is the rounded product)
+                    c[0][q] = __ffma2_rn(g[q], sv[d][0], c[0][q]);
+                    c[1][q] = __ffma2_rn(g[q], sv[d][1], c[1][q]);
+                }
+                load_row(sv[d], row0, ent[d], stride_b);
+                ep += 4;
+                if (ep == end) {
+                    fold();
+                    return;
+                }
+            }
+        }
+    }
+    float2 g0[NQ], s0[2], g1[NQ], s1[2];
+    uint32_t ent = lds32(ep);
+    load_pairs<NQ>(g0, plane, ent);
+    load_row(s0, row0, ent, stride_b);
+    ent = lds32(ep + 4);
     auto step = [&](const float2 (&g)[NQ], const float2 (&sv)[2]) {
         if (ep == next) {
             fold();
@@ -1311,7 +1352,7 @@ __device__ __forceinline__ void exact_haar(const float* lval, const int* lstart,
 // so an entry costs the same loads for 4 NQ multiply-adds instead of 2 NQ; the
 // halves' sums are added at the end.  (A whole warp per half, without the
 // divergence where only one half ends a voxel, took 14 % more instructions.)
-template <int JR, int NQ, bool HAAR>
+template <int JR, int NQ, bool HAAR, int D>
 __device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint32_t kron_byte, const float* __restrict__ lval,
                              const int* __restrict__ lstart, const uint32_t* __restrict__ lent, int U,
                              int kk, const float* __restrict__ st, int P,
@@ -1372,7 +1413,7 @@ __device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint
                     if (lane >> 4) lo = u_mid;
                     else hi = u_mid;
                 }
-                exact_pairs<NQ>(smem, lval, lstart, lent, lo, hi, 8u * i0, st + j0 + jl, 4u * stride, var);
+                exact_pairs<NQ, D>(smem, lval, lstart, lent, lo, hi, 8u * i0, st + j0 + jl, 4u * stride, var);
 #pragma unroll
                 for (int q = 0; q < NQ; ++q)
 #pragma unroll
@@ -1410,16 +1451,16 @@ __device__ void exact_planes(const unsigned char* smem, float a0, float b0, uint
     }
 }
 
-template <int JR>
+template <int JR, int D = 2>
 __device__ void exact_planes_any(const unsigned char* smem, bool haar, float a0, float b0, uint32_t kron_byte,
                                  const float* __restrict__ lval, const int* __restrict__ lstart,
                                  const uint32_t* __restrict__ lent, int U, int kk, const float* __restrict__ st, int P,
                                  float* __restrict__ EX, float* __restrict__ part, bool part_over) {
     auto run = [&](auto h) {
         constexpr bool H = decltype(h)::value;
-        if (kk == 1) exact_planes<JR, 1, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
-        else if (kk == 2) exact_planes<JR, 2, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
-        else exact_planes<JR, 4, H>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        if (kk == 1) exact_planes<JR, 1, H, D>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        else if (kk == 2) exact_planes<JR, 2, H, D>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
+        else exact_planes<JR, 4, H, D>(smem, a0, b0, kron_byte, lval, lstart, lent, U, kk, st, P, EX, part, part_over);
     };
     if (JR > 1 && haar) run(BoolTag<JR != 1>{});
     else run(BoolTag<false>{});
@@ -2017,7 +2058,7 @@ __device__ __forceinline__ void filter_group(const FilterArgs& a, unsigned char*
             float* part = sm<float>(smem, a.L.part);
             if (jr == 1) exact_planes_any<1>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
             else if (jr == 2) exact_planes_any<2>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
-            else exact_planes_any<4>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
+            else exact_planes_any<4, 4>(smem, false, 0.0f, 0.0f, 0u, lval, lstart, lent, U, kk, a.st, P, EX, part, a.L.part_over != 0);
         }
     }
 
